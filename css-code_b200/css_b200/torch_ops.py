@@ -34,6 +34,13 @@ def _vp(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+def _stream(t):
+    """PyTorch's current stream on t's device.  The default stream's handle is
+    0, which the library takes as the run's own (non-blocking) stream, where
+    nothing orders it with PyTorch's work: it is passed as cudaStreamLegacy."""
+    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream or 1)
+
+
 @torch.library.custom_op("css::deriv", mutates_args=(), device_types="cuda")
 def deriv(x: torch.Tensor, ctx: int, direction: int, order: int, bc_lo: Optional[torch.Tensor],
           bc_hi: Optional[torch.Tensor], bdry: int) -> torch.Tensor:
@@ -59,7 +66,7 @@ def deriv(x: torch.Tensor, ctx: int, direction: int, order: int, bc_lo: Optional
             faces.append(f.expand(nb, *fs))
         else:
             faces.append(f.reshape(nb, *fs))
-    stream = ctypes.c_void_p(torch.cuda.current_stream(xd.device).cuda_stream)
+    stream = _stream(xd)
     h = ctypes.c_void_p(ctx)
     for k in range(nb):
         lo = None if faces[0] is None else faces[0][k]
@@ -84,7 +91,7 @@ def deriv_adjoint(g: torch.Tensor, ctx: int, direction: int, order: int, bdry: i
     for d in gd.shape[:-3]:
         nb *= d
     gs, os_ = gd.reshape(nb, *gd.shape[-3:]), out.view(nb, *gd.shape[-3:])
-    stream = ctypes.c_void_p(torch.cuda.current_stream(gd.device).cuda_stream)
+    stream = _stream(gd)
     h = ctypes.c_void_p(ctx)
     for k in range(nb):
         check(_lib.lib().css_deriv_adjoint_dev(h, int(direction), int(order), _vp(gs[k]), _vp(os_[k]), int(bdry),

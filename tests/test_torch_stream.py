@@ -1,0 +1,32 @@
+"""The torch derivative operators' stream ordering."""
+import pytest
+
+from css_b200 import problem
+from css_b200.context import Simulation
+
+pytestmark = pytest.mark.gpu
+
+
+def test_default_stream_orders_with_torch(gpu_available):
+    """On PyTorch's default stream (handle 0) the operator waits for the work
+    that makes its input and its readers wait for it: the same values as with
+    a synchronisation on both sides."""
+    import torch
+    from css_b200 import torch_ops
+    p, prof, _, _, _ = problem.build((64, 64, 96), decomp=(2, 2, 3))
+    sim = Simulation(p, prof)
+    x0 = torch.randn(p.nr, p.nphi, p.nth, generator=torch.Generator().manual_seed(3), dtype=torch.float64).cuda()
+    a = torch.randn(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    want = torch_ops.dbydt(x0 * 3.0, sim)
+    torch.cuda.synchronize()
+    want = want + 1.0
+    for _ in range(10):
+        for _ in range(4):
+            b = a @ a  # keeps the default stream busy before the input is made
+        x = x0 * 3.0
+        got = torch_ops.dbydt(x, sim) + 1.0
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    del b
+    sim.close()
