@@ -20,6 +20,7 @@
 
 #include "../../include/css_b200.h"
 #include "css_kernels.cuh"
+#include "css_deriv.cuh"
 #include "css_stats.cuh"
 #include "css_closure.cuh"
 #include "css_lap.cuh"
@@ -71,10 +72,9 @@ struct css_ctx {
   double *rtw = nullptr;            // two-pass stage: zero-datum d(rho)/dtheta on the theta-wall blocks
   double *cyc = nullptr;            // cyclic phi derivative tables, per order: w, piv, z (nphi each), v.z
   double *bg2 = nullptr;            // mixed precision: rho and s backgrounds, [2][nr][nth]
-  // adjoints of css_deriv (torch backward): dense block operators per
-  // (direction, order, bdry), built on first use, and their block offsets
-  double *adjM[3][2][5] = {};
-  int *adjOff[3][2][5] = {};
+  // adjoints of css_deriv (torch backward): edge-row tables of the blocks per
+  // (direction, order, bdry), built on first use
+  double *adjE[3][2][5] = {};
   PlaneMaps pmaps[5];               // two-pass stage: TMA maps of v0, vA, vB, bf (plane kernel) and vs (curl)
   int vs_map = 0;                   // pmaps[4] and vs_slab hold vs's maps
   SlabMaps vs_slab;
@@ -271,7 +271,7 @@ extern "C" void css_destroy(css_ctx *c) {
   cudaFree(c->v0); cudaFree(c->vA); cudaFree(c->vB); cudaFree(c->dv); cudaFree(c->vs);
   for (int d = 0; d < 3; d++)
     for (int o = 0; o < 2; o++)
-      for (int b = 0; b < 5; b++) { cudaFree(c->adjM[d][o][b]); cudaFree(c->adjOff[d][o][b]); }
+      for (int b = 0; b < 5; b++) cudaFree(c->adjE[d][o][b]);
   cudaFree(c->bf); cudaFree(c->vcc); cudaFree(c->cda); cudaFree(c->flag); cudaFree(c->tbuf); cudaFree(c->rtw); cudaFree(c->cyc); cudaFree(c->bg2);
   cudaFree(c->lapbuf); cudaFree(c->lapface); cudaFree(c->radbuf); cudaFree(c->radface);
   cudaFree(c->io); cudaFree(c->io_part); cudaFree(c->rain); cudaFree(c->ash_slices); cudaFree(c->ashv);
@@ -352,12 +352,18 @@ static int setup_kernels() {
   CSS_FUSED_ATTR((k_rstage<1, 3>), RstageCfg<1>);
   CSS_FUSED_ATTR((k_rstage<1, 4>), RstageCfg<1>);
 #undef CSS_FUSED_ATTR
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_theta<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_theta<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_phi<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_phi<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_r<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  CUDA_TRY(cudaFuncSetAttribute(k_deriv_r<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  // run-time block lengths: up to 256 points a line
+#define CSS_LINE_ATTR(...) CUDA_TRY(cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
+  CSS_LINE_ATTR(k_deriv_s<0, 0>);
+  CSS_LINE_ATTR(k_deriv_s<2, 0>);
+  CSS_LINE_ATTR(k_deriv_t<0>);
+  CSS_LINE_ATTR(k_adj_s<0, 1, 0>);
+  CSS_LINE_ATTR(k_adj_s<0, 2, 0>);
+  CSS_LINE_ATTR(k_adj_s<2, 1, 0>);
+  CSS_LINE_ATTR(k_adj_s<2, 2, 0>);
+  CSS_LINE_ATTR(k_adj_t<1, 0>);
+  CSS_LINE_ATTR(k_adj_t<2, 0>);
+#undef CSS_LINE_ATTR
   done = true;
   return CSS_OK;
 }
@@ -999,6 +1005,41 @@ static void launch_phi_p(css_ctx *c, const double *cur) {
   k_phi_terms_p<MT, TLC><<<grid, 128, smem, c->stream>>>(g, cur, c->bf, c->dv, c->tbuf);
 }
 
+// threads of a CTA whose lanes keep a line of m doubles in shared memory:
+// 128 while that is at most 48 KB, fewer for longer lines
+static int line_threads(int m) { return m <= 48 ? 128 : (m <= 96 ? 64 : 32); }
+
+// n <= DERIV_MAX derivatives along one direction in one launch
+static int launch_derivs(css_ctx *c, int dir, const DerivItem *it, int n, cudaStream_t st) {
+  const CssGeo &g = c->g;
+  DerivBatch B;
+  for (int k = 0; k < n; k++) B.it[k] = it[k];
+  const int nb = g.d[dir].nb, m = g.d[dir].maxm, mt = c->mt[dir];
+  if (dir == 1) {
+    const int warps = 2 * 8 * dv_theta_warp(m) <= 200 * 1024 ? 2 : 1, nl = g.nphi * g.nr;
+    const size_t smem = (size_t)warps * dv_theta_warp(m) * 8;
+    const dim3 grid((nl + 32 * warps - 1) / (32 * warps), nb, n);
+    if (mt == 32) k_deriv_t<32><<<grid, 32 * warps, smem, st>>>(g, B);
+    else if (mt == 16) k_deriv_t<16><<<grid, 32 * warps, smem, st>>>(g, B);
+    else k_deriv_t<0><<<grid, 32 * warps, smem, st>>>(g, B);
+    return check_launch(c);
+  }
+  const int nl = dir == 0 ? g.nth * g.nphi : g.nth * g.nr;
+  const int nt = mt ? DV_NT : line_threads(m);
+  const size_t smem = mt ? 0 : (size_t)nt * m * 8;
+  const dim3 grid((nl + nt - 1) / nt, nb, n);
+  if (dir == 0) {
+    if (mt == 32) k_deriv_s<0, 32><<<grid, nt, smem, st>>>(g, B);
+    else if (mt == 16) k_deriv_s<0, 16><<<grid, nt, smem, st>>>(g, B);
+    else k_deriv_s<0, 0><<<grid, nt, smem, st>>>(g, B);
+  } else {
+    if (mt == 32) k_deriv_s<2, 32><<<grid, nt, smem, st>>>(g, B);
+    else if (mt == 16) k_deriv_s<2, 16><<<grid, nt, smem, st>>>(g, B);
+    else k_deriv_s<2, 0><<<grid, nt, smem, st>>>(g, B);
+  }
+  return check_launch(c);
+}
+
 // stage input of storage type TS, next stage state of storage type TO
 // explicit viscosity (Laplacian): the viscous terms of the three sweeps and
 // the cross terms, added into c->dv after the phi sweep; FP64 states only
@@ -1011,49 +1052,53 @@ static int launch_lap(css_ctx *c, const double *cur) {
   const int nbp = (int)std::min<size_t>((n + 255) / 256, (size_t)c->nsm * 8);
   const int nbf = (int)std::min<size_t>((nf + 255) / 256, (size_t)c->nsm * 8);
   cudaStream_t st = c->stream;
-#define LAP_D(dir, ord, x, out, lo, hi, bdry) \
-  if (int rc = css_deriv_dev(c, dir, ord, x, out, lo, hi, bdry, nullptr)) return rc
+  // the derivatives of one direction are independent: one launch
+#define LAP_D(dir, ...)                                                                     \
+  do {                                                                                      \
+    const DerivItem it_[] = {__VA_ARGS__};                                                  \
+    if (int rc = launch_derivs(c, dir, it_, (int)(sizeof it_ / sizeof *it_), st)) return rc; \
+  } while (0)
   // theta sweep: d/dth and d2/dth2 of w, v (wall datum cot v), u
   k_lap_bc_theta<<<nbf, 256, 0, st>>>(g, cur, F, F + nf);
   if (int rc = check_launch(c)) return rc;
-  LAP_D(1, 1, w, S, nullptr, nullptr, g.ibct[2]);
-  LAP_D(1, 1, v, S + n, F, F + nf, g.ibct[3]);
-  LAP_D(1, 1, u, S + 2 * n, nullptr, nullptr, g.ibct[4]);
-  LAP_D(1, 2, w, S + 3 * n, nullptr, nullptr, g.ibct[2]);
-  LAP_D(1, 2, v, S + 4 * n, F, F + nf, g.ibct[3]);
-  LAP_D(1, 2, u, S + 5 * n, nullptr, nullptr, g.ibct[4]);
+  LAP_D(1, DerivItem{w, S, nullptr, nullptr, g.ibct[2], 1},
+           DerivItem{v, S + n, F, F + nf, g.ibct[3], 1},
+           DerivItem{u, S + 2 * n, nullptr, nullptr, g.ibct[4], 1},
+           DerivItem{w, S + 3 * n, nullptr, nullptr, g.ibct[2], 2},
+           DerivItem{v, S + 4 * n, F, F + nf, g.ibct[3], 2},
+           DerivItem{u, S + 5 * n, nullptr, nullptr, g.ibct[4], 2});
   k_lap_theta<<<nbp, 256, 0, st>>>(g, cur, S, L, c->dv);
   if (int rc = check_launch(c)) return rc;
   // phi sweep: v, w, u
-  LAP_D(2, 1, v, S, nullptr, nullptr, 0);
-  LAP_D(2, 1, w, S + n, nullptr, nullptr, 0);
-  LAP_D(2, 1, u, S + 2 * n, nullptr, nullptr, 0);
-  LAP_D(2, 2, v, S + 3 * n, nullptr, nullptr, 0);
-  LAP_D(2, 2, w, S + 4 * n, nullptr, nullptr, 0);
-  LAP_D(2, 2, u, S + 5 * n, nullptr, nullptr, 0);
+  LAP_D(2, DerivItem{v, S, nullptr, nullptr, 0, 1},
+           DerivItem{w, S + n, nullptr, nullptr, 0, 1},
+           DerivItem{u, S + 2 * n, nullptr, nullptr, 0, 1},
+           DerivItem{v, S + 3 * n, nullptr, nullptr, 0, 2},
+           DerivItem{w, S + 4 * n, nullptr, nullptr, 0, 2},
+           DerivItem{u, S + 5 * n, nullptr, nullptr, 0, 2});
   k_lap_phi<<<nbp, 256, 0, st>>>(g, cur, c->tbuf, S, L, c->dv);
   if (int rc = check_launch(c)) return rc;
   // radial sweep: w, v with the stress-free data, u
   k_lap_bc_r<<<nbf, 256, 0, st>>>(g, cur, F, F + nf, F + 2 * nf, F + 3 * nf);
   if (int rc = check_launch(c)) return rc;
-  LAP_D(0, 1, w, S, F, F + nf, g.ibcr[2]);
-  LAP_D(0, 1, v, S + n, F + 2 * nf, F + 3 * nf, g.ibcr[3]);
-  LAP_D(0, 1, u, S + 2 * n, nullptr, nullptr, g.ibcr[4]);
-  LAP_D(0, 2, w, S + 3 * n, F, F + nf, g.ibcr[2]);
-  LAP_D(0, 2, v, S + 4 * n, F + 2 * nf, F + 3 * nf, g.ibcr[3]);
-  LAP_D(0, 2, u, S + 5 * n, nullptr, nullptr, g.ibcr[4]);
+  LAP_D(0, DerivItem{w, S, F, F + nf, g.ibcr[2], 1},
+           DerivItem{v, S + n, F + 2 * nf, F + 3 * nf, g.ibcr[3], 1},
+           DerivItem{u, S + 2 * n, nullptr, nullptr, g.ibcr[4], 1},
+           DerivItem{w, S + 3 * n, F, F + nf, g.ibcr[2], 2},
+           DerivItem{v, S + 4 * n, F + 2 * nf, F + 3 * nf, g.ibcr[3], 2},
+           DerivItem{u, S + 5 * n, nullptr, nullptr, g.ibcr[4], 2});
   k_lap_r<<<nbp, 256, 0, st>>>(g, cur, c->tbuf, S, L, c->dv);
   if (int rc = check_launch(c)) return rc;
   // cross terms: r derivatives of r L0 (var 2), r L5 (var 4), r L2 (var 4),
   // r L3 (var 3); theta derivatives of sin L3 (var 3), sin L4 (var 2)
   k_lap_bc_cross<<<nbf, 256, 0, st>>>(g, L, F, F + nf, F + 2 * nf, F + 3 * nf);
   if (int rc = check_launch(c)) return rc;
-  LAP_D(0, 1, S, L, F, nullptr, g.ibcr[2]);
-  LAP_D(0, 1, S + n, L + n, nullptr, nullptr, g.ibcr[4]);
-  LAP_D(0, 1, S + 2 * n, L + 2 * n, nullptr, nullptr, g.ibcr[4]);
-  LAP_D(0, 1, S + 3 * n, L + 3 * n, nullptr, F + nf, g.ibcr[3]);
-  LAP_D(1, 1, S + 4 * n, L + 4 * n, F + 2 * nf, F + 3 * nf, g.ibct[3]);
-  LAP_D(1, 1, S + 5 * n, L + 5 * n, nullptr, nullptr, g.ibct[2]);
+  LAP_D(0, DerivItem{S, L, F, nullptr, g.ibcr[2], 1},
+           DerivItem{S + n, L + n, nullptr, nullptr, g.ibcr[4], 1},
+           DerivItem{S + 2 * n, L + 2 * n, nullptr, nullptr, g.ibcr[4], 1},
+           DerivItem{S + 3 * n, L + 3 * n, nullptr, F + nf, g.ibcr[3], 1});
+  LAP_D(1, DerivItem{S + 4 * n, L + 4 * n, F + 2 * nf, F + 3 * nf, g.ibct[3], 1},
+           DerivItem{S + 5 * n, L + 5 * n, nullptr, nullptr, g.ibct[2], 1});
   k_lap_cross<<<nbp, 256, 0, st>>>(g, cur, L, c->dv);
   if (int rc = check_launch(c)) return rc;
   if (g.magnetic) {
@@ -1062,12 +1107,12 @@ static int launch_lap(css_ctx *c, const double *cur) {
     const double *bf = c->bf;
     k_mhd_curl_in<<<nbp, 256, 0, st>>>(g, bf, S);
     if (int rc = check_launch(c)) return rc;
-    LAP_D(1, 1, S, L, nullptr, nullptr, bdry_t);
-    LAP_D(1, 1, bf + 2 * n, L + n, nullptr, nullptr, bdry_t);
-    LAP_D(2, 1, bf + 2 * n, L + 2 * n, nullptr, nullptr, 0);
-    LAP_D(2, 1, bf, L + 3 * n, nullptr, nullptr, 0);
-    LAP_D(0, 1, S + n, L + 4 * n, nullptr, nullptr, g.ibcr[7]);
-    LAP_D(0, 1, S + 2 * n, L + 5 * n, nullptr, nullptr, g.ibcr[8]);
+    LAP_D(1, DerivItem{S, L, nullptr, nullptr, bdry_t, 1},
+             DerivItem{bf + 2 * n, L + n, nullptr, nullptr, bdry_t, 1});
+    LAP_D(2, DerivItem{bf + 2 * n, L + 2 * n, nullptr, nullptr, 0, 1},
+             DerivItem{bf, L + 3 * n, nullptr, nullptr, 0, 1});
+    LAP_D(0, DerivItem{S + n, L + 4 * n, nullptr, nullptr, g.ibcr[7], 1},
+             DerivItem{S + 2 * n, L + 5 * n, nullptr, nullptr, g.ibcr[8], 1});
     k_mhd_resist<<<nbp, 256, 0, st>>>(g, cur, c->tbuf, L, L + 3 * n, c->dv);
     if (int rc = check_launch(c)) return rc;
   }
@@ -1088,17 +1133,17 @@ static int launch_rad(css_ctx *c, const double *cur) {
   cudaStream_t st = c->stream;
   k_rad_bc<<<nbf, 256, 0, st>>>(g, cur, c->dv, T, F, F + nf, F + 2 * nf, F + 3 * nf, F + 4 * nf, F + 5 * nf);
   if (int rc = check_launch(c)) return rc;
-#define RAD_D(dir, ord, x, out, lo, hi, bdry) \
-  if (int rc = css_deriv_dev(c, dir, ord, x, out, lo, hi, bdry, nullptr)) return rc
-  RAD_D(1, 1, rho, S, F, F + nf, g.ibct[1]);
-  RAD_D(1, 1, T, S + n, F + 2 * nf, F + 3 * nf, g.ibct[6]);
-  RAD_D(1, 2, T, S + 2 * n, F + 2 * nf, F + 3 * nf, g.ibct[6]);
-  RAD_D(2, 1, rho, S + 3 * n, nullptr, nullptr, 0);
-  RAD_D(2, 1, T, S + 4 * n, nullptr, nullptr, 0);
-  RAD_D(2, 2, T, S + 5 * n, nullptr, nullptr, 0);
-  RAD_D(0, 1, T, S + 6 * n, F + 4 * nf, F + 5 * nf, g.ibcr[6]);
-  RAD_D(0, 2, T, S + 7 * n, F + 4 * nf, F + 5 * nf, g.ibcr[6]);
-#undef RAD_D
+  const DerivItem th[] = {{rho, S, F, F + nf, g.ibct[1], 1},
+                          {T, S + n, F + 2 * nf, F + 3 * nf, g.ibct[6], 1},
+                          {T, S + 2 * n, F + 2 * nf, F + 3 * nf, g.ibct[6], 2}};
+  const DerivItem ph[] = {{rho, S + 3 * n, nullptr, nullptr, 0, 1},
+                          {T, S + 4 * n, nullptr, nullptr, 0, 1},
+                          {T, S + 5 * n, nullptr, nullptr, 0, 2}};
+  const DerivItem rr[] = {{T, S + 6 * n, F + 4 * nf, F + 5 * nf, g.ibcr[6], 1},
+                          {T, S + 7 * n, F + 4 * nf, F + 5 * nf, g.ibcr[6], 2}};
+  if (int rc = launch_derivs(c, 1, th, 3, st)) return rc;
+  if (int rc = launch_derivs(c, 2, ph, 3, st)) return rc;
+  if (int rc = launch_derivs(c, 0, rr, 2, st)) return rc;
   k_rad_point<<<nbp, 256, 0, st>>>(g, cur, T, S, c->dv);
   return check_launch(c);
 }
@@ -1549,28 +1594,8 @@ extern "C" int css_deriv_dev(css_ctx *c, int dir, int order, const double *x, do
     set_err("css_deriv: bad argument");
     return CSS_ERR_ARG;
   }
-  cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-  const CssGeo &g = c->g;
-  if (dir == 1) {
-    int TL = c->tl_theta;
-    dim3 gr(g.d[1].nb * ((g.nphi + TL - 1) / TL), g.nr);
-    size_t sm = smem_theta(1, 1, g.d[1].maxm, TL);
-    if (order == 1) k_deriv_theta<1, 0><<<gr, 128, sm, st>>>(g, x, dx, bc_lo, bc_hi, bdry, TL);
-    else k_deriv_theta<2, 0><<<gr, 128, sm, st>>>(g, x, dx, bc_lo, bc_hi, bdry, TL);
-  } else if (dir == 2) {
-    int TL = c->tl_phi;
-    dim3 gr(g.d[2].nb * ((g.nth + TL - 1) / TL), g.nr);
-    size_t sm = smem_line(1, 1, 0, g.d[2].maxm, TL);
-    if (order == 1) k_deriv_phi<1, 0><<<gr, 128, sm, st>>>(g, x, dx, TL);
-    else k_deriv_phi<2, 0><<<gr, 128, sm, st>>>(g, x, dx, TL);
-  } else {
-    int TL = c->tl_r;
-    dim3 gr(g.d[0].nb * ((g.nth + TL - 1) / TL), g.nphi);
-    size_t sm = smem_line(1, 1, 0, g.d[0].maxm, TL);
-    if (order == 1) k_deriv_r<1, 0><<<gr, 128, sm, st>>>(g, x, dx, bc_lo, bc_hi, bdry, TL);
-    else k_deriv_r<2, 0><<<gr, 128, sm, st>>>(g, x, dx, bc_lo, bc_hi, bdry, TL);
-  }
-  return check_launch(c);
+  const DerivItem I{x, dx, bc_lo, bc_hi, bdry, order};
+  return launch_derivs(c, dir, &I, 1, stream ? (cudaStream_t)stream : c->stream);
 }
 
 extern "C" int css_dbydp_cyclic_dev(css_ctx *c, const double *x, double *dx, int order, void *stream) {
@@ -1595,50 +1620,75 @@ extern "C" int css_dbydp_cyclic(css_ctx *c, const double *x, double *dx, int ord
   return CSS_OK;
 }
 
-// dense block operators of css_deriv along dir (zero boundary data): block
-// b's m x (m + 8) matrix is the solver applied, on the host, to each unit
-// input of the block and its halos, with the run's tables and closures
-static int adjoint_mats(css_ctx *c, int dir, int order, int bdry) {
+// edge-row tables of css_deriv's adjoint along dir (css_deriv.cuh): the rows
+// 1, 2, m-1 and m of every block, the row functions applied on the host to
+// unit inputs (zero boundary data)
+static int adjoint_tables(css_ctx *c, int dir, int order, int bdry) {
   const int ob = dir == 2 ? 0 : bdry;
-  if (c->adjM[dir][order - 1][ob]) return CSS_OK;
+  if (c->adjE[dir][order - 1][ob]) return CSS_OK;
   const CssDir &D = c->g.d[dir];
-  std::vector<double> M;
-  std::vector<int> off(D.nb);
+  std::vector<double> E((size_t)D.nb * ADJ_TAB, 0.0);
   for (int b = 0; b < D.nb; b++) {
-    const int m = D.size[b], ts = m + 2, w = m + 8;
-    off[b] = (int)M.size();
-    M.resize(M.size() + (size_t)m * w);
-    std::vector<double> T(3 * (size_t)ts, 0.0), x(w), o(m);
-    double *g1 = T.data(), *g2 = g1 + ts, *g3 = g2 + ts;
-    if (dir == 2) tab_p(m, order == 1 ? 1.0 / 3.0 : 2.0 / 11.0, g1, g2, g3);
-    else if (order == 1) tab_d1(m, D.lphys[b], D.rphys[b], bdry, g1, g2, g3);
-    else tab_d2(m, D.lphys[b], D.rphys[b], bdry, g1, g2, g3);
+    const int m = D.size[b];
     const int dtype = dir == 2 ? 3 : (D.lphys[b] ? (D.rphys[b] ? 0 : 2) : (D.rphys[b] ? 1 : 3));
-    const double dn = D.dnum[b], sc = order == 1 ? dn : dn * dn;
-    for (int col = 0; col < w; col++) {
-      std::fill(x.begin(), x.end(), 0.0);
-      x[col] = 1.0;
-      if (order == 1)
-        line_solve_a<1>(x.data() + 4, StridedIn{1}, m, dtype, ob, 0.0, 0.0, T.data(), ts, dn, sc, dir == 2,
-                        o.data(), StridedOut{1});
-      else
-        line_solve_a<2>(x.data() + 4, StridedIn{1}, m, dtype, ob, 0.0, 0.0, T.data(), ts, dn, sc, dir == 2,
-                        o.data(), StridedOut{1});
-      for (int q = 0; q < m; q++) M[(size_t)off[b] + (size_t)q * w + col] = o[q];
+    std::vector<double> xv(m + 8, 0.0);
+    const double *x = xv.data() + 4;
+    const StridedIn xi{1};
+    double *e = &E[(size_t)b * ADJ_TAB];
+    for (int k = 0; k < ADJ_W; k++) {
+      xv[k] = 1.0;  // column k - 3
+      if (order == 1) {
+        e[ADJ_W + k] = d1_row_lo2(x, xi, dtype);
+        e[k] = d1_row_lo1(x, xi, dtype, ob, 0.0, 1.0, e[ADJ_W + k]);
+      } else {
+        e[ADJ_W + k] = d2_row_lo2(x, xi, dtype);
+        e[k] = d2_row_lo1(x, xi, dtype, ob, 0.0, 1.0);
+      }
+      xv[k] = 0.0;
+      xv[m - 4 + k] = 1.0;  // column m - 7 + k
+      if (order == 1) {
+        e[2 * ADJ_W + k] = d1_row_hi1(x, xi, m, dtype);
+        e[3 * ADJ_W + k] = d1_row_hi2(x, xi, m, dtype, ob, 0.0, 1.0, e[2 * ADJ_W + k]);
+      } else {
+        e[2 * ADJ_W + k] = d2_row_hi1(x, xi, m, dtype);
+        e[3 * ADJ_W + k] = d2_row_hi2(x, xi, m, dtype, ob, 0.0, 1.0);
+      }
+      xv[m - 4 + k] = 0.0;
     }
   }
-  double *dM = nullptr;
-  int *dO = nullptr;
-  if (cudaMalloc(&dM, M.size() * 8) != cudaSuccess || cudaMalloc(&dO, off.size() * sizeof(int)) != cudaSuccess) {
-    cudaFree(dM);
+  double *dE = nullptr;
+  if (cudaMalloc(&dE, E.size() * 8) != cudaSuccess) {
     set_err("css_deriv_adjoint: device allocation failed");
     return CSS_ERR_NOMEM;
   }
-  CUDA_TRY(cudaMemcpy(dM, M.data(), M.size() * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dO, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
-  c->adjM[dir][order - 1][ob] = dM;
-  c->adjOff[dir][order - 1][ob] = dO;
+  if (cudaMemcpy(dE, E.data(), E.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(dE);
+    set_err("css_deriv_adjoint: table copy failed");
+    return CSS_ERR_CUDA;
+  }
+  c->adjE[dir][order - 1][ob] = dE;
   return CSS_OK;
+}
+
+template <int DIR, int ORDER>
+static void launch_adj_s(css_ctx *c, const double *E, const double *gin, double *gout, int bdry, cudaStream_t st) {
+  const CssGeo &g = c->g;
+  const int nl = DIR == 0 ? g.nth * g.nphi : g.nth * g.nr, m = g.d[DIR].maxm, mt = c->mt[DIR];
+  const int nt = mt ? DV_NT : line_threads(m);
+  const unsigned grid = (unsigned)((nl + nt - 1) / nt);
+  if (mt == 32) k_adj_s<DIR, ORDER, 32><<<grid, nt, 0, st>>>(g, E, gin, gout, bdry);
+  else if (mt == 16) k_adj_s<DIR, ORDER, 16><<<grid, nt, 0, st>>>(g, E, gin, gout, bdry);
+  else k_adj_s<DIR, ORDER, 0><<<grid, nt, (size_t)nt * m * 8, st>>>(g, E, gin, gout, bdry);
+}
+template <int ORDER>
+static void launch_adj_t(css_ctx *c, const double *E, const double *gin, double *gout, int bdry, cudaStream_t st) {
+  const CssGeo &g = c->g;
+  const int m = g.d[1].maxm, mt = c->mt[1];
+  const size_t smem = 2 * (size_t)32 * adj_theta_stride(m) * 8;
+  const unsigned grid = (unsigned)((g.nphi * g.nr + 63) / 64);
+  if (mt == 32) k_adj_t<ORDER, 32><<<grid, 64, smem, st>>>(g, E, gin, gout, bdry);
+  else if (mt == 16) k_adj_t<ORDER, 16><<<grid, 64, smem, st>>>(g, E, gin, gout, bdry);
+  else k_adj_t<ORDER, 0><<<grid, 64, smem, st>>>(g, E, gin, gout, bdry);
 }
 
 extern "C" int css_deriv_adjoint_dev(css_ctx *c, int dir, int order, const double *g, double *gx, int bdry,
@@ -1647,11 +1697,20 @@ extern "C" int css_deriv_adjoint_dev(css_ctx *c, int dir, int order, const doubl
     set_err("css_deriv_adjoint: bad argument");
     return CSS_ERR_ARG;
   }
-  if (int rc = adjoint_mats(c, dir, order, bdry)) return rc;
+  if (int rc = adjoint_tables(c, dir, order, bdry)) return rc;
   const int ob = dir == 2 ? 0 : bdry;
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-  k_deriv_adjoint<<<(unsigned)((c->ncell + 255) / 256), 256, 0, st>>>(c->g, dir, c->adjM[dir][order - 1][ob],
-                                                                       c->adjOff[dir][order - 1][ob], g, gx);
+  const double *E = c->adjE[dir][order - 1][ob];
+  if (dir == 1) {
+    if (order == 1) launch_adj_t<1>(c, E, g, gx, ob, st);
+    else launch_adj_t<2>(c, E, g, gx, ob, st);
+  } else if (dir == 0) {
+    if (order == 1) launch_adj_s<0, 1>(c, E, g, gx, ob, st);
+    else launch_adj_s<0, 2>(c, E, g, gx, ob, st);
+  } else {
+    if (order == 1) launch_adj_s<2, 1>(c, E, g, gx, ob, st);
+    else launch_adj_s<2, 2>(c, E, g, gx, ob, st);
+  }
   return check_launch(c);
 }
 

@@ -1902,99 +1902,6 @@ __global__ void k_sld_ohmic(CssGeo g, const double *__restrict__ v, const double
   }
 }
 
-// ---------------------------------------------------------------------------
-// generic single-field derivative (css_deriv): one kernel per direction
-// ---------------------------------------------------------------------------
-template <int ORDER, int MT>
-__global__ void __launch_bounds__(128) k_deriv_theta(CssGeo g, const double *__restrict__ f, double *__restrict__ out,
-                                                     const double *__restrict__ bclo, const double *__restrict__ bchi,
-                                                     int bdry, int TL) {
-  extern __shared__ double sm[];
-  const int nchunk = (g.nphi + TL - 1) / TL;
-  const int bt = blockIdx.x / nchunk, pb = (blockIdx.x - bt * nchunk) * TL;
-  const int ir = blockIdx.y;
-  const CssDir &D = g.d[1];
-  const int t0 = D.start[bt], m = D.size[bt];
-  const int SR = m + 9, SO = m + 1;
-  double *H = sm, *O = H + (size_t)TL * SR;
-  load_theta_tile(g, f, H, SR, t0, m, pb, TL, ir, true);
-  __syncthreads();
-  for (int l = threadIdx.x; l < TL; l += blockDim.x) {
-    int ip = pb + l;
-    if (ip >= g.nphi) continue;
-    double lo = (D.lphys[bt] && bclo) ? bclo[ip + (size_t)g.nphi * ir] : 0.0;
-    double hi = (D.rphys[bt] && bchi) ? bchi[ip + (size_t)g.nphi * ir] : 0.0;
-    double dn = (ORDER == 1) ? D.dnum[bt] : dnum_d2_theta(g, ir);
-    double sc = (ORDER == 1) ? D.dnum[bt] : D.dnum[bt] * D.dnum[bt];
-    solve<ORDER, MT>(H + (size_t)l * SR + 4, 1, m, dtype_of(D, bt), bdry, lo, hi, tabp(g, 1, bt, ORDER, bdry),
-                      g.tstride, dn, sc, 0, O + (size_t)l * SO, 1);
-  }
-  __syncthreads();
-  for (int pt = threadIdx.x; pt < TL * m; pt += blockDim.x) {
-    int l = pt / m, j = pt - l * m;
-    if (pb + l >= g.nphi) continue;
-    out[css_idx(g, t0 + j, pb + l, ir)] = O[(size_t)l * SO + j];
-  }
-}
-
-template <int ORDER, int MT>
-__global__ void __launch_bounds__(128) k_deriv_phi(CssGeo g, const double *__restrict__ f, double *__restrict__ out,
-                                                   int TL) {
-  extern __shared__ double sm[];
-  const int nchunk = (g.nth + TL - 1) / TL;
-  const int bp = blockIdx.x / nchunk, tb = (blockIdx.x - bp * nchunk) * TL;
-  const int ir = blockIdx.y;
-  const CssDir &D = g.d[2];
-  const int p0 = D.start[bp], m = D.size[bp];
-  const int SR = TL + 1;
-  double *H = sm, *O = H + (size_t)(m + 8) * SR;
-  load_phi_tile(g, f, H, SR, p0, m, tb, TL, ir, true);
-  __syncthreads();
-  for (int l = threadIdx.x; l < TL; l += blockDim.x) {
-    if (tb + l >= g.nth) continue;
-    double sc = (ORDER == 1) ? D.dnum[bp] : D.dnum[bp] * D.dnum[bp];
-    solve<ORDER, MT>(H + 4 * SR + l, SR, m, 3, 0, 0.0, 0.0, tabp(g, 2, bp, ORDER, 0), g.tstride, D.dnum[bp], sc, 1,
-                      O + l, SR);
-  }
-  __syncthreads();
-  for (int pt = threadIdx.x; pt < TL * m; pt += blockDim.x) {
-    int j = pt / TL, l = pt - j * TL;
-    if (tb + l >= g.nth) continue;
-    out[css_idx(g, tb + l, p0 + j, ir)] = O[(size_t)j * SR + l];
-  }
-}
-
-template <int ORDER, int MT>
-__global__ void __launch_bounds__(128) k_deriv_r(CssGeo g, const double *__restrict__ f, double *__restrict__ out,
-                                                 const double *__restrict__ bclo, const double *__restrict__ bchi,
-                                                 int bdry, int TL) {
-  extern __shared__ double sm[];
-  const int nchunk = (g.nth + TL - 1) / TL;
-  const int br = blockIdx.x / nchunk, tb = (blockIdx.x - br * nchunk) * TL;
-  const int ip = blockIdx.y;
-  const CssDir &D = g.d[0];
-  const int r0 = D.start[br], m = D.size[br];
-  const int SR = TL + 1;
-  double *H = sm, *O = H + (size_t)(m + 8) * SR;
-  load_r_tile(g, f, H, SR, r0, m, tb, TL, ip, true);
-  __syncthreads();
-  for (int l = threadIdx.x; l < TL; l += blockDim.x) {
-    int it = tb + l;
-    if (it >= g.nth) continue;
-    double lo = (D.lphys[br] && bclo) ? bclo[it + (size_t)g.nth * ip] : 0.0;
-    double hi = (D.rphys[br] && bchi) ? bchi[it + (size_t)g.nth * ip] : 0.0;
-    double sc = (ORDER == 1) ? D.dnum[br] : D.dnum[br] * D.dnum[br];
-    solve<ORDER, MT>(H + 4 * SR + l, SR, m, dtype_of(D, br), bdry, lo, hi, tabp(g, 0, br, ORDER, bdry), g.tstride,
-                      D.dnum[br], sc, 0, O + l, SR);
-  }
-  __syncthreads();
-  for (int pt = threadIdx.x; pt < TL * m; pt += blockDim.x) {
-    int j = pt / TL, l = pt - j * TL;
-    if (tb + l >= g.nth) continue;
-    out[css_idx(g, tb + l, ip, r0 + j)] = O[(size_t)j * SR + l];
-  }
-}
-
 // Cyclic phi derivative of one field (css_dbydp_cyclic; an extension with
 // no counterpart in the reference, whose Dbydp closes each block with halo
 // rows, derivatives.f90:1480-1591): every whole phi line is periodic and
@@ -2040,49 +1947,6 @@ __global__ void k_dbydp_cyclic(CssGeo g, const double *__restrict__ x, double *_
     const size_t q = base + (size_t)j * nth;
     out[q] = scale * (out[q] - fact * __ldg(z + j));
   }
-}
-
-// Adjoint of the whole-field compact derivative along direction dir (the
-// backward of torch.ops.css.deriv): gx = D^T g with zero boundary data.
-// M holds every block's dense operator, rows = the block's m outputs,
-// columns = its m + 8 inputs (4 halo points below, the block, 4 above),
-// at M + off[b].  A point is an input of its own block and, within four
-// points of a block face, a halo input of the neighbouring block (phi
-// periodic), so gx at that point gathers one column of each: a fixed-order
-// sum, deterministic.  One thread per point.
-__global__ void k_deriv_adjoint(CssGeo g, int dir, const double *__restrict__ M, const int *__restrict__ off,
-                                const double *__restrict__ gin, double *__restrict__ gout) {
-  const size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (id >= (size_t)g.ncell) return;
-  const int it = (int)(id % g.nth), ip = (int)((id / g.nth) % g.nphi), ir = (int)(id / ((size_t)g.nth * g.nphi));
-  const CssDir &D = g.d[dir];
-  const int a = dir == 0 ? ir : (dir == 1 ? it : ip);
-  int b = 0;
-  while (b + 1 < D.nb && D.start[b + 1] <= a) b++;
-  const int i = a - D.start[b], m = D.size[b];
-  auto gat = [&](int aa) -> double {
-    return __ldg(gin + (dir == 0 ? css_idx(g, it, ip, aa) : (dir == 1 ? css_idx(g, aa, ip, ir) : css_idx(g, it, aa, ir))));
-  };
-  auto col = [&](int bb, int c) -> double {
-    const int mb = D.size[bb], s0 = D.start[bb];
-    const double *Mb = M + off[bb];
-    double acc = 0.0;
-    for (int q = 0; q < mb; q++) acc += __ldg(Mb + (size_t)q * (mb + 8) + c) * gat(s0 + q);
-    return acc;
-  };
-  double acc = col(b, i + 4);
-  const bool periodic = dir == 2;
-  if (i < 4) {
-    int bb = b - 1;
-    if (bb < 0 && periodic) bb = D.nb - 1;
-    if (bb >= 0) acc += col(bb, D.size[bb] + 4 + i);
-  }
-  if (i >= m - 4) {
-    int bb = b + 1;
-    if (bb >= D.nb && periodic) bb = 0;
-    if (bb < D.nb) acc += col(bb, i - (m - 4));
-  }
-  gout[id] = acc;
 }
 
 // independent lines with explicit closures, staged through shared memory:
