@@ -2469,7 +2469,14 @@ extern "C" int css_closure_scales(int nct, int ncp, int ncr, const double *field
 
 extern "C" int css_closure_features(int nct, int ncp, int ncr, const double *fields, const float *scale, void *x) {
   if (!fields || !scale || !x || nct < 1 || ncp < 1 || ncr < 1) { set_err("css_closure_features: bad argument"); return CSS_ERR_ARG; }
-  k_closure_features<<<148 * 8, 128>>>(fields, nct, ncp, ncr, scale, (__nv_bfloat16 *)x);
+  // segments of phi: long ones recompute fewer columns at their ends (two a
+  // segment), but every SM should hold its four CTAs
+  const int ntc = (nct + CF_T - 1) / CF_T;
+  int seg = 32;
+  while (seg > 4 && (long long)ntc * ncr * ((ncp + seg - 1) / seg) < 4 * 148) seg /= 2;
+  const dim3 grid(ntc, (ncp + seg - 1) / seg, ncr);
+  k_closure_features<<<grid, CF_NT>>>(fields, nct, ncp, ncr, scale, seg,
+                                         (uintptr_t)x % 16 == 0, (__nv_bfloat16 *)x);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaDeviceSynchronize());
   return CSS_OK;

@@ -399,3 +399,31 @@ def test_study_reports_what_the_closure_gains(gpu_available):
     assert r["errors"]["variance"]["E_K"] < 0.5 * r["errors"]["prescribed"]["E_K"]
     assert r["loss_last"] < 0.5 * r["loss_first"]
     assert r["fine_window_s"] > r["coarse_window_s"]["variance"]
+
+
+@pytest.mark.parametrize("dims", [(65, 3, 2), (64, 33, 1), (5, 70, 3), (130, 1, 2)])
+def test_features_at_tile_edges(dims, gpu_available):
+    """Cell counts around the feature kernel's tiles (64 theta, segments of
+    phi) and an output that is not 16-byte aligned, bit for bit against numpy."""
+    import torch
+    from css_b200 import _lib
+    nct, ncp, ncr = dims
+    rng = np.random.default_rng(nct)
+    F = rng.standard_normal((7, ncr, ncp, nct))
+    if ncr == 1:  # one radius: ds'/dr is 0 / 0 in the reference statement too
+        F[3] = 0.0
+    qs = np.array([1.0, 2.0, 0.5, 3.0, 0.7], np.float32)
+    fd, qd = torch.from_numpy(F.reshape(-1)).cuda(), torch.from_numpy(qs).cuda()
+    n = nct * ncp * ncr * 144
+    out = []
+    for off in (0, 3):
+        x = torch.empty(n + 16, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        _lib.check(_lib.lib().css_closure_features(nct, ncp, ncr, fd.data_ptr(), qd.data_ptr(),
+                                                   x.data_ptr() + 2 * off))
+        out.append(x[off:off + n].float().cpu().numpy().reshape(-1, 144))
+    with np.errstate(invalid="ignore"):
+        want = numpy_features(F, qs)
+    for x in out:
+        assert np.array_equal(np.isnan(x), np.isnan(want))
+        assert np.array_equal(np.nan_to_num(x), np.nan_to_num(want))
