@@ -2555,17 +2555,18 @@ struct css_mlp {
   int dims[5];          // padded widths: input, hidden x3, output
   int nreal_in, nreal_out;
   size_t cap;           // rows per pass
+  unsigned char *arena = nullptr;  // the allocation every buffer below lies in
   float *W[4] = {}, *B[4] = {}, *gW[4] = {}, *gB[4] = {}, *mW[4] = {}, *vW[4] = {}, *mB[4] = {}, *vB[4] = {};
   __nv_bfloat16 *Wb[4] = {};
   __nv_bfloat16 *WbT[4] = {};   // Wb transposed (out x in), for the forward products
   bool wt_ok = false;
   float *Z[4] = {};             // pre-activations; Z[3] is the output
   __nv_bfloat16 *H[4] = {};     // H[1..3] activations; H[0] is the caller's input
-  float *dH = nullptr;          // FP32 gradient scratch
-  __nv_bfloat16 *dZb = nullptr; // BF16 gradient
+  __nv_bfloat16 *dZb[2] = {};   // BF16 gradients of two layers in turn
   double *part = nullptr;
   int adam_t = 0;
-  float *gpart = nullptr;       // row-chunk partials of the weight gradients
+  float *wpart[4] = {};         // row-chunk partials of the weight gradients
+  double *bpart[4] = {};        // row-tile partials of the bias gradients
   cudaStream_t st = nullptr, own_st = nullptr;
   unsigned char *packed = nullptr;  // weights for the fused forward kernel
   bool packed_ok = false;
@@ -2575,28 +2576,35 @@ struct css_mlp {
 
 // the products of a pass, on k_gemm_bf16 (row-major; see css_closure.cuh)
 #define GM_NSPLIT 64
-// Z = X W with W read as its transpose WT (out x in): the same access
-// pattern as dH = dZ W^T, so both run the row-contiguous form of the kernel
-static int gemm_fwd(css_mlp *m, const __nv_bfloat16 *X, const __nv_bfloat16 *WT, float *Z, size_t rows, int K, int M) {
+#define MSE_BLOCKS 256
+// Z = X W + b and H = bf16(GELU(Z)) with W read as its transpose WT (out x
+// in): both operands run along the reduction
+static int gemm_fwd(css_mlp *m, const __nv_bfloat16 *X, int l, __nv_bfloat16 *H, size_t rows) {
+  const int K = m->dims[l], M = m->dims[l + 1];
   dim3 grid((unsigned)((rows + GM_TP - 1) / GM_TP), (M + GM_TQ - 1) / GM_TQ);
-  k_gemm_bf16<GM_DIN><<<grid, 128, 0, m->st>>>(X, WT, Z, (int)rows, M, K, K, K, 0);
+  const GmEpi E{m->B[l], m->Z[l], H, nullptr, nullptr};
+  k_gemm_bf16<GM_ACT><<<grid, 128, 0, m->st>>>(X, m->WbT[l], E, (int)rows, M, K, K, K, 0);
   CUDA_TRY(cudaGetLastError());
   return CSS_OK;
 }
-static int gemm_din(css_mlp *m, const __nv_bfloat16 *D, const __nv_bfloat16 *W, float *dH, size_t rows, int K, int M) {
+// dZ of layer l - 1 (bf16, into D2) and its column sums per row tile
+static int gemm_back(css_mlp *m, const __nv_bfloat16 *D, int l, __nv_bfloat16 *D2, size_t rows) {
+  const int K = m->dims[l], M = m->dims[l + 1];
   dim3 grid((unsigned)((rows + GM_TP - 1) / GM_TP), (K + GM_TQ - 1) / GM_TQ);
-  k_gemm_bf16<GM_DIN><<<grid, 128, 0, m->st>>>(D, W, dH, (int)rows, K, M, M, M, 0);
+  const GmEpi E{nullptr, m->Z[l - 1], D2, m->bpart[l - 1], nullptr};
+  k_gemm_bf16<GM_BACK><<<grid, 128, 0, m->st>>>(D, m->Wb[l], E, (int)rows, K, M, M, M, 0);
   CUDA_TRY(cudaGetLastError());
   return CSS_OK;
 }
-static int gemm_dw(css_mlp *m, const __nv_bfloat16 *X, const __nv_bfloat16 *D, float *gW, size_t rows, int K, int M) {
+// row-chunk partials of dW of layer l; the number of chunks in *nsplit
+static int gemm_dw(css_mlp *m, const __nv_bfloat16 *X, const __nv_bfloat16 *D, int l, size_t rows, int *nsplit) {
+  const int K = m->dims[l], M = m->dims[l + 1];
   long long chunk = ((long long)rows + GM_NSPLIT - 1) / GM_NSPLIT;
   chunk = std::max(256LL, (chunk + 15) / 16 * 16);
-  const int nsplit = (int)(((long long)rows + chunk - 1) / chunk);
-  dim3 grid((K + GM_TP - 1) / GM_TP, (M + GM_TQ - 1) / GM_TQ, nsplit);
-  k_gemm_bf16<GM_DW><<<grid, 128, 0, m->st>>>(X, D, m->gpart, K, M, (long long)rows, K, M, chunk);
-  CUDA_TRY(cudaGetLastError());
-  k_sum_partials<<<64, 256, 0, m->st>>>(m->gpart, nsplit, K * M, gW);
+  *nsplit = (int)(((long long)rows + chunk - 1) / chunk);
+  dim3 grid((K + GM_TP - 1) / GM_TP, (M + GM_TQ - 1) / GM_TQ, *nsplit);
+  const GmEpi E{nullptr, nullptr, nullptr, nullptr, m->wpart[l]};
+  k_gemm_bf16<GM_DW><<<grid, 128, 0, m->st>>>(X, D, E, K, M, (long long)rows, K, M, chunk);
   CUDA_TRY(cudaGetLastError());
   return CSS_OK;
 }
@@ -2608,12 +2616,7 @@ __global__ void k_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__restrict
 
 extern "C" void css_mlp_destroy(css_mlp *m) {
   if (!m) return;
-  for (int l = 0; l < 4; l++) {
-    cudaFree(m->W[l]); cudaFree(m->B[l]); cudaFree(m->gW[l]); cudaFree(m->gB[l]);
-    cudaFree(m->mW[l]); cudaFree(m->vW[l]); cudaFree(m->mB[l]); cudaFree(m->vB[l]); cudaFree(m->Wb[l]); cudaFree(m->WbT[l]);
-    cudaFree(m->Z[l]); cudaFree(m->H[l]);
-  }
-  cudaFree(m->dH); cudaFree(m->dZb); cudaFree(m->part); cudaFree(m->gpart); cudaFree(m->packed);
+  cudaFree(m->arena);
   cudaFree(m->flag);
   if (m->own_st) cudaStreamDestroy(m->own_st);
   else if (m->st) cudaStreamDestroy(m->st);
@@ -2636,24 +2639,33 @@ extern "C" int css_mlp_create(int n_in, int width, int n_out, int max_rows, unsi
   m->cap = (size_t)max_rows;
   cudaError_t e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   const int wmax = std::max(std::max(m->dims[0], width), m->dims[4]);
-  if (!e) e = cudaMalloc(&m->gpart, (size_t)GM_NSPLIT * wmax * wmax * 4);
-  for (int l = 0; l < 4 && !e; l++) {
+  // every buffer in one allocation (256-byte aligned pieces)
+  std::vector<std::pair<void **, size_t>> bufs;
+  auto add = [&](auto &p, size_t bytes) { bufs.push_back({reinterpret_cast<void **>(&p), (bytes + 255) / 256 * 256}); };
+  for (int l = 0; l < 4; l++) {
     const size_t K = m->dims[l], M = m->dims[l + 1];
-    float **f4[] = {&m->W[l], &m->gW[l], &m->mW[l], &m->vW[l]};
-    for (auto pp : f4)
-      if (!e) e = cudaMalloc(pp, K * M * 4);
-    float **b4[] = {&m->B[l], &m->gB[l], &m->mB[l], &m->vB[l]};
-    for (auto pp : b4)
-      if (!e) e = cudaMalloc(pp, M * 4);
-    if (!e) e = cudaMalloc(&m->Wb[l], K * M * 2);
-    if (!e) e = cudaMalloc(&m->WbT[l], K * M * 2);
-    if (!e) e = cudaMalloc(&m->Z[l], m->cap * M * 4);
-    if (!e && l > 0) e = cudaMalloc(&m->H[l], m->cap * K * 2);
+    for (auto pp : {&m->W[l], &m->gW[l], &m->mW[l], &m->vW[l]}) add(*pp, K * M * 4);
+    for (auto pp : {&m->B[l], &m->gB[l], &m->mB[l], &m->vB[l]}) add(*pp, M * 4);
+    add(m->Wb[l], K * M * 2);
+    add(m->WbT[l], K * M * 2);
+    add(m->Z[l], m->cap * M * 4);
+    if (l > 0) add(m->H[l], m->cap * K * 2);
+    add(m->wpart[l], (size_t)GM_NSPLIT * K * M * 4);
+    add(m->bpart[l], std::max((m->cap + GM_TP - 1) / GM_TP, (size_t)MSE_BLOCKS) * M * 8);
   }
-  if (!e) e = cudaMalloc(&m->dH, m->cap * wmax * 4);
-  if (!e) e = cudaMalloc(&m->dZb, m->cap * wmax * 2);
-  if (!e) e = cudaMalloc(&m->part, 1024 * 8);
-  if (!e) e = cudaMalloc(&m->packed, FM_PARAM_BYTES);
+  for (auto &d : m->dZb) add(d, m->cap * wmax * 2);
+  add(m->part, MSE_BLOCKS * 8);
+  add(m->packed, FM_PARAM_BYTES);
+  size_t total = 0;
+  for (auto &b : bufs) total += b.second;
+  if (!e) e = cudaMalloc(&m->arena, total);
+  if (!e) {
+    size_t o = 0;
+    for (auto &b : bufs) {
+      *b.first = m->arena + o;
+      o += b.second;
+    }
+  }
   if (e) {
     set_err("css_mlp_create: %s", cudaGetErrorString(e));
     css_mlp_destroy(m);
@@ -2716,11 +2728,8 @@ static int mlp_forward_rows(css_mlp *m, const __nv_bfloat16 *x, size_t n) {
   }
   const __nv_bfloat16 *in = x;
   for (int l = 0; l < 4; l++) {
-    const int K = m->dims[l], M = m->dims[l + 1];
-    if (int rc = gemm_fwd(m, in, m->WbT[l], m->Z[l], n, K, M)) return rc;
     __nv_bfloat16 *next = l < 3 ? m->H[l + 1] : nullptr;
-    k_bias_gelu<<<148 * 4, 256, 0, m->st>>>(m->Z[l], m->B[l], next, M, n);
-    CUDA_TRY(cudaGetLastError());
+    if (int rc = gemm_fwd(m, in, l, next, n)) return rc;
     in = next;
   }
   return CSS_OK;
@@ -2813,35 +2822,32 @@ extern "C" int css_mlp_train_step(css_mlp *m, const void *x, const float *t, lon
   const size_t rows = (size_t)n;
   const __nv_bfloat16 *xb = (const __nv_bfloat16 *)x;
   if (int rc = mlp_forward_rows(m, xb, rows)) return rc;
-  const int nb = 256;
-  k_mse<<<nb, 256, 0, m->st>>>(m->Z[3], t, rows, m->nreal_out, m->dH, m->dZb, m->part);
+  k_mse<<<MSE_BLOCKS, 256, 0, m->st>>>(m->Z[3], t, rows, m->nreal_out, m->dZb[1], m->part, m->bpart[3]);
   CUDA_TRY(cudaGetLastError());
-  for (int l = 3; l >= 0; l--) {
-    const int K = m->dims[l], M = m->dims[l + 1];
-    const __nv_bfloat16 *in = l == 0 ? xb : m->H[l];
-    // dW = dZ^T-contracted input, db = column sums of dZ
-    if (int rc = gemm_dw(m, in, m->dZb, m->gW[l], rows, K, M)) return rc;
-    k_colsum<<<M, 256, 0, m->st>>>(m->dH, M, rows, m->gB[l]);
-    CUDA_TRY(cudaGetLastError());
-    if (l > 0) {
-      if (int rc = gemm_din(m, m->dZb, m->Wb[l], m->dH, rows, K, M)) return rc;
-      k_gelu_back<<<148 * 4, 256, 0, m->st>>>(m->dH, m->Z[l - 1], m->dZb, (size_t)K * rows);
-      CUDA_TRY(cudaGetLastError());
-    }
-  }
   m->adam_t++;
   m->packed_ok = false;
-  m->wt_ok = false;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float c1 = 1.0f - powf(b1, (float)m->adam_t), c2 = 1.0f - powf(b2, (float)m->adam_t);
-  for (int l = 0; l < 4; l++) {
-    const size_t K = m->dims[l], M = m->dims[l + 1];
-    k_adam<<<148, 256, 0, m->st>>>(m->W[l], m->gW[l], m->mW[l], m->vW[l], m->Wb[l], K * M, lr, b1, b2, eps, c1, c2);
-    k_adam<<<4, 256, 0, m->st>>>(m->B[l], m->gB[l], m->mB[l], m->vB[l], nullptr, M, lr, b1, b2, eps, c1, c2);
+  MlpUpdate U;
+  U.lr = lr; U.b1 = 0.9f; U.b2 = 0.999f; U.eps = 1e-8f;
+  U.c1 = 1.0f - powf(U.b1, (float)m->adam_t);
+  U.c2 = 1.0f - powf(U.b2, (float)m->adam_t);
+  int nbw = 0, ncb = 0;
+  for (int l = 3; l >= 0; l--) {
+    const __nv_bfloat16 *in = l == 0 ? xb : m->H[l], *dz = m->dZb[l & 1];
+    int nsplit;
+    if (int rc = gemm_dw(m, in, dz, l, rows, &nsplit)) return rc;
+    if (l > 0)
+      if (int rc = gemm_back(m, dz, l, m->dZb[(l - 1) & 1], rows)) return rc;
+    const int nbp = l == 3 ? MSE_BLOCKS : (int)((rows + GM_TP - 1) / GM_TP);
+    U.l[l] = {m->W[l], m->gW[l], m->mW[l], m->vW[l], m->B[l], m->gB[l], m->mB[l], m->vB[l], m->Wb[l], m->WbT[l],
+              m->wpart[l], m->bpart[l], m->dims[l], m->dims[l + 1], nsplit, nbp};
+    nbw += m->dims[l] * m->dims[l + 1] / 32;
+    ncb += (m->dims[l + 1] + 31) / 32;
   }
+  U.nbw = nbw;
+  k_mlp_update<<<U.nbw + ncb, 256, 0, m->st>>>(U);
   CUDA_TRY(cudaGetLastError());
-  std::vector<double> h(nb);
-  CUDA_TRY(cudaMemcpyAsync(h.data(), m->part, nb * 8, cudaMemcpyDeviceToHost, m->st));
+  std::vector<double> h(MSE_BLOCKS);
+  CUDA_TRY(cudaMemcpyAsync(h.data(), m->part, MSE_BLOCKS * 8, cudaMemcpyDeviceToHost, m->st));
   CUDA_TRY(cudaStreamSynchronize(m->st));
   double s = 0.0;
   for (double v : h) s += v;

@@ -1,7 +1,7 @@
 // css_closure.cuh -- the learned subgrid closure: box filtering of a fine
 // state into coarse fields and subgrid targets, the 3x3x3 stencil features,
-// and the elementwise parts of the MLP (bias + GELU and its derivative,
-// loss, bias gradients, Adam), and k_gemm_bf16: the MLP's matrix products
+// and the elementwise parts of the MLP (loss,
+// gradient sums and Adam), and k_gemm_bf16: the MLP's matrix products
 // for training and the per-layer forward pass, BF16 operands with FP32
 // accumulation on the tensor cores (mma.sync m16n8k16), issued from
 // css_api.cu.
@@ -282,84 +282,121 @@ __device__ __forceinline__ float gelu_df(float x) {
   return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * du;
 }
 
-// Z (col-major M x n: Z[r*M + j]) += b[j]; H = bf16(GELU(Z)) when H != NULL
-__global__ void k_bias_gelu(float *__restrict__ Z, const float *__restrict__ b, __nv_bfloat16 *__restrict__ H,
-                            int M, size_t n) {
-  const size_t tot = (size_t)M * n;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
-    const float z = Z[i] + b[i % M];
-    Z[i] = z;
-    if (H) H[i] = __float2bfloat16_rn(gelu_f(z));
-  }
-}
-
 // loss and output gradient: D = Y - T over the first nreal of CL_YPAD
-// columns; dY = 2 D / (n nreal) (FP32 and BF16), pad columns zero;
-// part[block] = partial sum of D^2
-__global__ void k_mse(const float *__restrict__ Y, const float *__restrict__ T, size_t n, int nreal,
-                      float *__restrict__ dY, __nv_bfloat16 *__restrict__ dYb, double *__restrict__ part) {
-  __shared__ double red[256];
+// columns; dY = 2 D / (n nreal) in BF16, pad columns zero; part[block] =
+// partial sum of D^2, cpart[block * CL_YPAD + k] the block's column sums of
+// the FP32 dY (the output bias gradient).  The stride is a multiple of
+// CL_YPAD, so a thread stays in its column.
+__global__ void __launch_bounds__(256) k_mse(const float *__restrict__ Y, const float *__restrict__ T, size_t n,
+                                             int nreal, __nv_bfloat16 *__restrict__ dYb, double *__restrict__ part,
+                                             double *__restrict__ cpart) {
+  __shared__ double red[256], col[256];
   const size_t tot = n * CL_YPAD;
   const float sc = 2.0f / ((float)n * (float)nreal);
-  double acc = 0.0;
+  const int k = threadIdx.x % CL_YPAD;
+  double acc = 0.0, cs = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(i % CL_YPAD);
     float d = 0.0f;
     if (k < nreal) {
       d = Y[i] - T[i];
       acc += (double)d * d;
     }
-    dY[i] = sc * d;
+    cs += (double)(sc * d);
     dYb[i] = __float2bfloat16_rn(sc * d);
   }
   red[threadIdx.x] = acc;
+  col[threadIdx.x] = cs;
   __syncthreads();
   for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    if ((int)threadIdx.x < s) {
+      red[threadIdx.x] += red[threadIdx.x + s];
+      if (s >= CL_YPAD) col[threadIdx.x] += col[threadIdx.x + s];
+    }
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  if (threadIdx.x < CL_YPAD) cpart[(size_t)blockIdx.x * CL_YPAD + threadIdx.x] = col[threadIdx.x];
 }
 
-// back through GELU: dZ = dH * GELU'(Z) (FP32 in place of dH, and BF16)
-__global__ void k_gelu_back(float *__restrict__ dH, const float *__restrict__ Z, __nv_bfloat16 *__restrict__ dZb,
-                            size_t tot) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
-    const float d = dH[i] * gelu_df(Z[i]);
-    dH[i] = d;
-    dZb[i] = __float2bfloat16_rn(d);
-  }
+// The update of a training step: every layer's weight and bias gradients
+// summed from their partials (weights over the row chunks of k_gemm_bf16,
+// biases over the row tiles), then bias-corrected Adam on the FP32 master
+// parameters, with the BF16 copy and its transpose refreshed.  One launch for
+// all eight tensors: each is a few microseconds of work on its own.  A block
+// takes 32 weights (blocks below nbw) or 32 biases, the partials of each
+// spread over eight threads so that their loads overlap, summed in a fixed
+// order.  26 us after 16384 rows, against 121 us with a thread per weight
+// walking its 64 partials, and 230 us for the column sums, partial sums, Adam
+// and transposes as launches of their own.
+struct MlpUpdate {
+  struct Layer {
+    float *W, *gW, *mW, *vW, *B, *gB, *mB, *vB;
+    __nv_bfloat16 *Wb, *WbT;
+    const float *wpart;   // [nsplit][K * M]
+    const double *bpart;  // [nbp][M]
+    int K, M, nsplit, nbp;
+  } l[4];
+  int nbw;
+  float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adam_one(const MlpUpdate &U, float w, float gi, float &m, float &v) {
+  m = U.b1 * m + (1.0f - U.b1) * gi;
+  v = U.b2 * v + (1.0f - U.b2) * gi * gi;
+  return w - U.lr * (m / U.c1) / (sqrtf(v / U.c2) + U.eps);
 }
-
-// bias gradient: db[j] = sum over the n rows of dZ[r*M + j]; grid = M
-// blocks, each sums its column in a fixed order (deterministic)
-__global__ void k_colsum(const float *__restrict__ dZ, int M, size_t n, float *__restrict__ db) {
-  __shared__ double red[256];
-  const int j = blockIdx.x;
-  double acc = 0.0;
-  for (size_t r = threadIdx.x; r < n; r += blockDim.x) acc += dZ[r * M + j];
-  red[threadIdx.x] = acc;
+// sum of this column's nz partials (stride doubles apart), eight threads
+// taking every eighth; the total on the threads of the first eighth
+template <typename T>
+__device__ __forceinline__ T mlp_sum8(const T *__restrict__ p, int nz, size_t stride, int c, int h, T (*red)[33]) {
+  T s = (T)0;
+#pragma unroll 8
+  for (int z = h; z < nz; z += 8) s += __ldg(p + (size_t)z * stride);
+  red[h][c] = s;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) db[j] = (float)red[0];
+  T t = (T)0;
+  if (h == 0)
+#pragma unroll
+    for (int k = 0; k < 8; k++) t += red[k][c];
+  return t;
 }
-
-// Adam (bias-corrected) on FP32 master parameters, refreshing the BF16 copy
-__global__ void k_adam(float *__restrict__ w, const float *__restrict__ gr, float *__restrict__ m,
-                       float *__restrict__ v2, __nv_bfloat16 *__restrict__ wb, size_t cnt, float lr, float b1,
-                       float b2, float eps, float c1, float c2) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cnt; i += (size_t)gridDim.x * blockDim.x) {
-    const float gi = gr[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v2[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v2[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16_rn(wi);
+__global__ void __launch_bounds__(256) k_mlp_update(const __grid_constant__ MlpUpdate U) {
+  __shared__ union {
+    float w[8][33];
+    double b[8][33];
+  } red;
+  const int c = threadIdx.x & 31, h = threadIdx.x >> 5;
+  int blk = blockIdx.x, l = 0;
+  if (blk < U.nbw) {
+    while (blk * 32 >= U.l[l].K * U.l[l].M) blk -= U.l[l].K * U.l[l].M / 32, l++;
+    const MlpUpdate::Layer &L = U.l[l];
+    const int cnt = L.K * L.M, i = blk * 32 + c;  // K and M are multiples of 16
+    const float gs = mlp_sum8<float>(L.wpart + i, L.nsplit, (size_t)cnt, c, h, red.w);
+    if (h == 0) {
+      L.gW[i] = gs;
+      float m = L.mW[i], v = L.vW[i];
+      const float w = adam_one(U, L.W[i], gs, m, v);
+      L.mW[i] = m;
+      L.vW[i] = v;
+      L.W[i] = w;
+      const __nv_bfloat16 wb = __float2bfloat16_rn(w);
+      L.Wb[i] = wb;
+      const int k = i / L.M, q = i - k * L.M;
+      L.WbT[(size_t)q * L.K + k] = wb;
+    }
+    return;
+  }
+  blk -= U.nbw;
+  while (blk >= (U.l[l].M + 31) / 32) blk -= (U.l[l].M + 31) / 32, l++;
+  const MlpUpdate::Layer &L = U.l[l];
+  const int q = blk * 32 + c;
+  const bool in = q < L.M;
+  const float gi = (float)mlp_sum8<double>(L.bpart + (in ? q : 0), L.nbp, (size_t)L.M, c, h, red.b);
+  if (h == 0 && in) {
+    L.gB[q] = gi;
+    float m = L.mB[q], v = L.vB[q];
+    L.B[q] = adam_one(U, L.B[q], gi, m, v);
+    L.mB[q] = m;
+    L.vB[q] = v;
   }
 }
 
@@ -899,19 +936,28 @@ __global__ void __launch_bounds__(TC_NT, 1) k_mlp_tc(const __nv_bfloat16 *__rest
 
 // ---------------------------------------------------------------------------
 // The products of a training step on the tensor cores: BF16 mma.sync
-// m16n8k16 with FP32 accumulation, row-major operands.
-//   GM_FWD: C[n][i] = sum_k X[n][k] W[k][i]             (Z = X W)
-//   GM_DIN: C[n][j] = sum_i D[n][i] W[j][i]             (dH = dZ W^T)
-//   GM_DW:  C[z][j][i] = sum_{n in chunk z} X[n][j] D[n][i]   (dW = X^T dZ,
-//           split over row chunks; k_sum_partials adds the chunks in order)
+// m16n8k16 with FP32 accumulation, row-major operands, each with what follows
+// it folded into its epilogue.
+//   GM_ACT:  Z = X W + b (W read as its transpose), H = bf16(GELU(Z))
+//   GM_BACK: dZ = (D W^T) GELU'(Z) in BF16, and its FP32 column sums per row
+//            tile (the bias gradient)
+//   GM_DW:   part[z] = sum_{n in chunk z} X[n][j] D[n][i]  (dW = X^T dZ,
+//            split over row chunks; k_mlp_update adds the chunks in order)
 // A CTA of 4 warps computes a 32 (p) x 64 (q) tile of C; the reduction runs
-// in 16-wide steps through shared memory, zero-filled outside the operands.
+// in 64-wide stages through shared memory, zero-filled outside the operands,
+// the next stage's vectors in registers while this one multiplies.  GM_DW's
+// operands arrive with the reduction index outermost: they are stored as
+// they come and ldmatrix transposes them: 34 us for the four products of
+// 16384 rows, against 85 us stored column by column, two bytes at a time.  The
+// folded epilogues replace the separate bias + GELU, GELU-backward and column
+// sums (154 + 71 us for the seven products and those passes, now 70).
 // ---------------------------------------------------------------------------
-enum { GM_FWD = 0, GM_DIN = 1, GM_DW = 2 };
+enum { GM_ACT = 0, GM_BACK = 1, GM_DW = 2 };
 #define GM_TP 32
 #define GM_TQ 64
 #define GM_KS 64              // reduction width of one shared-memory stage
 #define GM_RS (GM_KS + 8)     // shared row stride in BF16: 144 B, rows stay 16-byte aligned
+#define GM_PS (GM_TP + 8)     // GM_DW: stride of A's rows (80 B: ldmatrix meets no bank conflict)
 
 // 8 consecutive BF16 from p (n of them valid, the rest zero): one 16-byte
 // load when all 8 are valid (p is then 16-byte aligned: every leading
@@ -923,27 +969,33 @@ __device__ __forceinline__ uint4 gm_ld8(const __nv_bfloat16 *__restrict__ p, int
   for (int e = 0; e < 8; e++) v[e] = e < n ? p[e] : __float2bfloat16_rn(0.0f);
   return *reinterpret_cast<uint4 *>(v);
 }
-
-// scatter 8 BF16 down a column of a [row][GM_RS] shared tile
-__device__ __forceinline__ void gm_st8_col(__nv_bfloat16 (*T)[GM_RS], int row0, int col, uint4 v) {
-  const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
-#pragma unroll
-  for (int k = 0; k < 8; k++) T[row0 + k][col] = e[k];
+__device__ __forceinline__ void gm_ldsm_t(unsigned (&r)[4], const __nv_bfloat16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
 }
+
+struct GmEpi {
+  const float *bias;     // GM_ACT
+  float *Z;              // GM_ACT: written; GM_BACK: the layer's pre-activations, read
+  __nv_bfloat16 *H;      // GM_ACT: activations (may be NULL); GM_BACK: dZ
+  double *cpart;         // GM_BACK: [row tile][Q]
+  float *part;           // GM_DW: [chunk][P * Q]
+};
 
 template <int MODE>
 __global__ void __launch_bounds__(128) k_gemm_bf16(const __nv_bfloat16 *__restrict__ X,
-                                                   const __nv_bfloat16 *__restrict__ Y, float *__restrict__ C,
-                                                   int P, int Q, long long R, int ldx, int ldy, long long chunk) {
-  __shared__ __align__(16) __nv_bfloat16 As[GM_TP][GM_RS];
-  __shared__ __align__(16) __nv_bfloat16 Bs[GM_TQ][GM_RS];
+                                                   const __nv_bfloat16 *__restrict__ Y, GmEpi E, int P, int Q,
+                                                   long long R, int ldx, int ldy, long long chunk) {
+  constexpr int AS = MODE == GM_DW ? GM_KS * GM_PS : GM_TP * GM_RS;
+  __shared__ __align__(16) __nv_bfloat16 As[AS];
+  __shared__ __align__(16) __nv_bfloat16 Bs[GM_TQ * GM_RS];  // GM_DW: [r][q], else [q][r]; both 64 x 64
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const int p0 = blockIdx.x * GM_TP, q0 = blockIdx.y * GM_TQ;
   long long r0 = 0, r1 = R;
   if (MODE == GM_DW) {
     r0 = (long long)blockIdx.z * chunk;
     r1 = r0 + chunk < R ? r0 + chunk : R;
-    C += (size_t)blockIdx.z * P * Q;
   }
   const int wp = (w & 1) * 16, wq = (w >> 1) * 32;
   float acc[4][4];
@@ -951,66 +1003,130 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const __nv_bfloat16 *__restri
   for (int nt = 0; nt < 4; nt++)
 #pragma unroll
     for (int c = 0; c < 4; c++) acc[nt][c] = 0.0f;
-  for (long long rb = r0; rb < r1; rb += GM_KS) {
+  // one stage's vectors of 8: A 32 x 64 (two a thread), B 64 x 64 (four)
+  uint4 va[2], vb[4];
+  auto fetch = [&](long long rb) {
     const long long rleft = r1 - rb;
-    // A tile (32 p x 64 r): 256 vectors of 8, two per thread
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int v = tid + h * 128;
       if (MODE == GM_DW) {  // A(p, r) = X[r * ldx + p]: vectors along p
-        const int rr = v >> 2, p8 = (v & 3) * 8;
-        const int p = p0 + p8;
-        const int n = (rr < rleft) ? (P - p < 8 ? P - p : 8) : 0;
-        gm_st8_col(As, p8, rr, gm_ld8(X + (rb + rr) * ldx + p, n));
+        const int rr = v >> 2, p = p0 + (v & 3) * 8;
+        const int n = (rr < rleft) ? (P - p < 8 ? (P - p > 0 ? P - p : 0) : 8) : 0;
+        va[h] = gm_ld8(X + (rb + rr) * ldx + (n > 0 ? p : 0), n);
       } else {  // A(p, r) = X[p * ldx + r]: vectors along r
-        const int pp = v >> 3, r8 = (v & 7) * 8;
-        const int p = p0 + pp;
+        const int p = p0 + (v >> 3), r8 = (v & 7) * 8;
         const long long rl = rleft - r8;
         const int n = (p < P) ? (int)(rl < 8 ? (rl > 0 ? rl : 0) : 8) : 0;
-        *reinterpret_cast<uint4 *>(&As[pp][r8]) = gm_ld8(X + (long long)p * ldx + rb + r8, n);
+        va[h] = gm_ld8(X + (long long)(n > 0 ? p : 0) * ldx + rb + r8, n);
       }
     }
-    // B tile (64 q x 64 r), stored [q][r]: 512 vectors of 8, four per thread
 #pragma unroll
     for (int h = 0; h < 4; h++) {
       const int v = tid + h * 128;
-      if (MODE == GM_DIN) {  // B(r, q) = Y[q * ldy + r]: vectors along r
-        const int qq = v >> 3, r8 = (v & 7) * 8;
-        const int q = q0 + qq;
+      if (MODE == GM_DW) {  // B(r, q) = Y[r * ldy + q]: vectors along q
+        const int rr = v >> 3, q = q0 + (v & 7) * 8;
+        const int n = (rr < rleft) ? (Q - q < 8 ? (Q - q > 0 ? Q - q : 0) : 8) : 0;
+        vb[h] = gm_ld8(Y + (rb + rr) * ldy + (n > 0 ? q : 0), n);
+      } else {  // B(r, q) = Y[q * ldy + r]: vectors along r
+        const int q = q0 + (v >> 3), r8 = (v & 7) * 8;
         const long long rl = rleft - r8;
         const int n = (q < Q) ? (int)(rl < 8 ? (rl > 0 ? rl : 0) : 8) : 0;
-        *reinterpret_cast<uint4 *>(&Bs[qq][r8]) = gm_ld8(Y + (long long)q * ldy + rb + r8, n);
-      } else {  // B(r, q) = Y[r * ldy + q]: vectors along q
-        const int rr = v >> 3, q8 = (v & 7) * 8;
-        const int q = q0 + q8;
-        const int n = (rr < rleft) ? (Q - q < 8 ? (Q - q > 0 ? Q - q : 0) : 8) : 0;
-        gm_st8_col(Bs, q8, rr, gm_ld8(Y + (rb + rr) * ldy + (n > 0 ? q : 0), n));
+        vb[h] = gm_ld8(Y + (long long)(n > 0 ? q : 0) * ldy + rb + r8, n);
       }
     }
+  };
+  fetch(r0);
+  for (long long rb = r0; rb < r1; rb += GM_KS) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int v = tid + h * 128;
+      *reinterpret_cast<uint4 *>(As + (MODE == GM_DW ? (v >> 2) * GM_PS + (v & 3) * 8 : (v >> 3) * GM_RS + (v & 7) * 8)) =
+          va[h];
+    }
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      const int v = tid + h * 128;
+      *reinterpret_cast<uint4 *>(Bs + (v >> 3) * GM_RS + (v & 7) * 8) = vb[h];
+    }
     __syncthreads();
+    if (rb + GM_KS < r1) fetch(rb + GM_KS);
 #pragma unroll
     for (int ks = 0; ks < GM_KS; ks += 16) {
       unsigned a[4];
-      a[0] = *reinterpret_cast<const unsigned *>(&As[wp + g][ks + 2 * t]);
-      a[1] = *reinterpret_cast<const unsigned *>(&As[wp + g + 8][ks + 2 * t]);
-      a[2] = *reinterpret_cast<const unsigned *>(&As[wp + g][ks + 2 * t + 8]);
-      a[3] = *reinterpret_cast<const unsigned *>(&As[wp + g + 8][ks + 2 * t + 8]);
+      if (MODE == GM_DW) {
+        const int i = lane >> 3, j = lane & 7;
+        gm_ldsm_t(a, As + (ks + (i >> 1) * 8 + j) * GM_PS + wp + (i & 1) * 8);
 #pragma unroll
-      for (int nt = 0; nt < 4; nt++) {
-        const __nv_bfloat16 *br = &Bs[wq + nt * 8 + g][ks + 2 * t];
-        mma_bf16_16816(acc[nt], a, *reinterpret_cast<const unsigned *>(br),
-                       *reinterpret_cast<const unsigned *>(br + 8));
+        for (int nt = 0; nt < 4; nt += 2) {
+          unsigned b[4];
+          gm_ldsm_t(b, Bs + (ks + (i & 1) * 8 + j) * GM_RS + wq + nt * 8 + (i >> 1) * 8);
+          mma_bf16_16816(acc[nt], a, b[0], b[1]);
+          mma_bf16_16816(acc[nt + 1], a, b[2], b[3]);
+        }
+      } else {
+        const __nv_bfloat16 *ar = As + (wp + g) * GM_RS + ks + 2 * t;
+        a[0] = *reinterpret_cast<const unsigned *>(ar);
+        a[1] = *reinterpret_cast<const unsigned *>(ar + 8 * GM_RS);
+        a[2] = *reinterpret_cast<const unsigned *>(ar + 8);
+        a[3] = *reinterpret_cast<const unsigned *>(ar + 8 * GM_RS + 8);
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++) {
+          const __nv_bfloat16 *br = Bs + (wq + nt * 8 + g) * GM_RS + ks + 2 * t;
+          mma_bf16_16816(acc[nt], a, *reinterpret_cast<const unsigned *>(br),
+                         *reinterpret_cast<const unsigned *>(br + 8));
+        }
       }
     }
     __syncthreads();
   }
+  // epilogue: a thread holds the pairs (p, q), (p, q + 1) of rows p and p + 8;
+  // Q is a multiple of 16, so a pair is inside or outside as one
 #pragma unroll
-  for (int nt = 0; nt < 4; nt++)
+  for (int nt = 0; nt < 4; nt++) {
+    const int q = q0 + wq + nt * 8 + 2 * t;
+    double cs0 = 0.0, cs1 = 0.0;
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int p = p0 + wp + g + (c >= 2 ? 8 : 0), q = q0 + wq + nt * 8 + 2 * t + (c & 1);
-      if (p < P && q < Q) C[(size_t)p * Q + q] = acc[nt][c];
+    for (int c = 0; c < 2; c++) {
+      const int p = p0 + wp + g + c * 8;
+      if (p < P && q < Q) {
+        const size_t o = (size_t)p * Q + q;
+        float x0 = acc[nt][2 * c], x1 = acc[nt][2 * c + 1];
+        if (MODE == GM_DW) {
+          *reinterpret_cast<float2 *>(E.part + (size_t)blockIdx.z * P * Q + o) = make_float2(x0, x1);
+        } else if (MODE == GM_ACT) {
+          x0 += __ldg(E.bias + q);
+          x1 += __ldg(E.bias + q + 1);
+          *reinterpret_cast<float2 *>(E.Z + o) = make_float2(x0, x1);
+          if (E.H) *reinterpret_cast<__nv_bfloat162 *>(E.H + o) = __floats2bfloat162_rn(gelu_f(x0), gelu_f(x1));
+        } else {
+          const float2 z = *reinterpret_cast<const float2 *>(E.Z + o);
+          x0 *= gelu_df(z.x);
+          x1 *= gelu_df(z.y);
+          *reinterpret_cast<__nv_bfloat162 *>(E.H + o) = __floats2bfloat162_rn(x0, x1);
+          cs0 += (double)x0;
+          cs1 += (double)x1;
+        }
+      }
     }
+    if (MODE == GM_BACK) {  // columns over the warp's 16 rows, then both warps' (the stages are done with Bs)
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        cs0 += __shfl_xor_sync(0xffffffffu, cs0, o);
+        cs1 += __shfl_xor_sync(0xffffffffu, cs1, o);
+      }
+      double *cr = reinterpret_cast<double *>(Bs) + (w & 1) * GM_TQ + wq + nt * 8 + 2 * t;
+      if (g == 0) {
+        cr[0] = cs0;
+        cr[1] = cs1;
+      }
+    }
+  }
+  if (MODE == GM_BACK) {
+    __syncthreads();
+    const double *cr = reinterpret_cast<const double *>(Bs);
+    if (tid < GM_TQ && q0 + tid < Q) E.cpart[(size_t)blockIdx.x * Q + q0 + tid] = cr[tid] + cr[GM_TQ + tid];
+  }
 }
 
 // dst (M x K) = src (K x M) transposed, BF16
@@ -1019,15 +1135,6 @@ __global__ void k_transpose_bf16(const __nv_bfloat16 *__restrict__ src, int K, i
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int q = i / K, k = i - q * K;
     dst[i] = src[(size_t)k * M + q];
-  }
-}
-
-// out[i] = sum over z in order of part[z * count + i]
-__global__ void k_sum_partials(const float *__restrict__ part, int nsplit, int count, float *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int z = 0; z < nsplit; z++) s += part[(size_t)z * count + i];
-    out[i] = s;
   }
 }
 

@@ -427,3 +427,25 @@ def test_features_at_tile_edges(dims, gpu_available):
     for x in out:
         assert np.array_equal(np.isnan(x), np.isnan(want))
         assert np.array_equal(np.nan_to_num(x), np.nan_to_num(want))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 300, 16400])
+def test_gradients_at_row_counts(n, gpu_available):
+    """Row counts around the product tiles (32 rows, 64-wide stages, chunks
+    of 256): weight and bias gradients against the numpy statement with the
+    device's roundings (the bar of the test above, normwise)."""
+    import torch
+    from css_b200 import closure as C
+    rng = np.random.default_rng(n)
+    net = C.Mlp(135, 128, 12, max_rows=16400, seed=7)
+    x = np.zeros((n, 144), np.float32)
+    x[:, :135] = to_bf16(rng.standard_normal((n, 135)).astype(np.float32))
+    t = np.zeros((n, 16), np.float32)
+    t[:, :12] = rng.standard_normal((n, 12))
+    loss = net.train_step(torch.from_numpy(x).to(torch.bfloat16).cuda(), torch.from_numpy(t).cuda(), n, 0.0)
+    _, grads, want = numpy_net(net, x, t, 12)
+    assert abs(loss - want) <= 2e-2 * want
+    for l in range(4):
+        gw, gb = net.grads(l)
+        assert np.linalg.norm(gw - grads[l][0]) <= 2e-2 * np.linalg.norm(grads[l][0]), l
+        assert np.linalg.norm(gb - grads[l][1]) <= 2e-2 * np.linalg.norm(grads[l][1]), l
