@@ -712,7 +712,7 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   const double *rhor = &P[CSS_PROF_RHO * nr];
   double tv[8] = {1e-8 * rhor[nr - 1], 1e-8, 1e-8, 1e-8, 1e-8 * 1e5, 1e-8 * 1e8, 1e-8 * 1e8, 1e-8 * 1e8};
   memcpy(g.tinyvar, tv, sizeof tv);
-  for (int k = 0; k < 8; k++) g.inv_tinyvar[k] = 1.0 / tv[k];  // correctly rounded, as a device division
+  for (int k = 0; k < 8; k++) g.inv_tinyvar2[k] = (1.0 / tv[k]) * (1.0 / tv[k]);
   g.nsld = 0;
   if (p.mass_diffusion) g.varlist[g.nsld++] = 0;
   for (int i = 1; i <= 4; i++) g.varlist[g.nsld++] = i;
@@ -1289,7 +1289,18 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
   prof_end(c);
   if (int rc = check_launch(c)) return rc;
   prof_begin(c, KI_SLD);
-  dim3 gs((g.nth + SLD_TT - 1) / SLD_TT, (g.nphi + SLD_TP - 1) / SLD_TP, (g.nr + SLD_RC - 1) / SLD_RC);
+  // radii a CTA marches over: the chunk that takes the fewest radii in a row
+  // over the waves of two CTAs an SM, where a chunk's start (its windows, the
+  // first planes) counts as one and a half.  On large shells that is 32 or
+  // 16; on 64x64x128, 32 left 84 of 148 SMs idle (279 us a launch, 99 with 8).
+  const long long ntile = (long long)((g.nth + SLD_TT - 1) / SLD_TT) * ((g.nphi + SLD_TP - 1) / SLD_TP);
+  int rc = 32;
+  double best = 1e30;
+  for (int k = 32; k >= 4; k /= 2) {
+    const long long waves = (ntile * ((g.nr + k - 1) / k) + 2 * c->nsm - 1) / (2 * c->nsm);
+    if (waves * (k + 1.5) < best) { best = waves * (k + 1.5); rc = k; }
+  }
+  dim3 gs((g.nth + SLD_TT - 1) / SLD_TT, (g.nphi + SLD_TP - 1) / SLD_TP, (g.nr + rc - 1) / rc);
   // the diffused fields are contiguous from varlist[0]; MHD runs them in two
   // launches (the hydro fields, then A) so each carries a register window
   // of at most five fields
@@ -1302,17 +1313,17 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
   const unsigned all = (1u << g.nv) - 1u;
   const int th = SLD_TT * SLD_TP;
   switch (g.nsld) {
-    case 4: k_sld<4, 1><<<gs, th, sizeof(SldSmem<4>), c->stream>>>(g, v, av, c->vcc, dout, all, tb); break;
-    case 5: k_sld<5, 0><<<gs, th, sizeof(SldSmem<5>), c->stream>>>(g, v, av, c->vcc, dout, all, tb); break;
+    case 4: k_sld<4, 1><<<gs, th, sizeof(SldSmem<4>), c->stream>>>(g, v, av, c->vcc, dout, all, tb, rc); break;
+    case 5: k_sld<5, 0><<<gs, th, sizeof(SldSmem<5>), c->stream>>>(g, v, av, c->vcc, dout, all, tb, rc); break;
     case 7:  // fields 1..7: rho is not diffused (its tendency is zero)
-      k_sld<4, 1><<<gs, th, sizeof(SldSmem<4>), c->stream>>>(g, v, av, c->vcc, dout, 0x1Fu, tb);
+      k_sld<4, 1><<<gs, th, sizeof(SldSmem<4>), c->stream>>>(g, v, av, c->vcc, dout, 0x1Fu, tb, rc);
       if (int rc = check_launch(c)) return rc;
-      k_sld<3, 5><<<gs, th, sizeof(SldSmem<3>), c->stream>>>(g, v, av, c->vcc, dout, 0xE0u, tb);
+      k_sld<3, 5><<<gs, th, sizeof(SldSmem<3>), c->stream>>>(g, v, av, c->vcc, dout, 0xE0u, tb, rc);
       break;
     default:  // fields 0..7
-      k_sld<5, 0><<<gs, th, sizeof(SldSmem<5>), c->stream>>>(g, v, av, c->vcc, dout, 0x1Fu, tb);
+      k_sld<5, 0><<<gs, th, sizeof(SldSmem<5>), c->stream>>>(g, v, av, c->vcc, dout, 0x1Fu, tb, rc);
       if (int rc = check_launch(c)) return rc;
-      k_sld<3, 5><<<gs, th, sizeof(SldSmem<3>), c->stream>>>(g, v, av, c->vcc, dout, 0xE0u, tb);
+      k_sld<3, 5><<<gs, th, sizeof(SldSmem<3>), c->stream>>>(g, v, av, c->vcc, dout, 0xE0u, tb, rc);
       break;
   }
   prof_end(c);

@@ -63,7 +63,7 @@ struct CssGeo {
   double s_flux_lo, s_flux_hi;  // entropy-gradient datum at constant-flux faces
   // slope-limited diffusion
   double sld_coef, sld_pr, sld_prm;
-  double tinyvar[8], inv_tinyvar[8];  // floors of the SLD limiter and their reciprocals
+  double tinyvar[8], inv_tinyvar2[8];  // floors of the SLD limiter and their squared reciprocals
   int nsld, varlist[8];
   int dstype, mass_diffusion, do_viscous_heating, do_ohmic_heating;
   // open radial boundaries (Top_/Bottom_Inflow_Outflow, rhs_mpi.f90:1857-2067)

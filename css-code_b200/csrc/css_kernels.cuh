@@ -1503,29 +1503,30 @@ __global__ void k_sld_vcc(CssGeo g, const double *__restrict__ v, const double *
   }
 }
 
-// q * max(0, min(1, q*qph / max(|q|,tiny)^2)).  For |q| >= tiny the ratio is
-// qph/q, so the limited value is 0 (opposite signs), q (|qph| >= |q|) or qph:
-// a minmod, evaluated without the division (equal to the reference's
-// product to within its roundings); below tiny the formula as written.
-__device__ __forceinline__ double sld_limiter(double q, double qph, double tiny, double inv_tiny) {
-  const double a = fabs(q);
-  if (a >= tiny) {
-    if (!(q * qph > 0.0)) return q * 0.0;
-    return fabs(qph) >= a ? q : qph;
-  }
-  double rtmp = inv_tiny;  // 1/tiny, the same correctly rounded quotient
-  rtmp = q * (rtmp * rtmp);
-  rtmp = rtmp * qph;
-  rtmp = fmin(1.0, rtmp);
-  return q * fmax(0.0, rtmp);
+// Limited difference of two neighbouring differences: q * max(0, min(1,
+// q*qph / max(|q|,tiny)^2)).  For |q| >= tiny the ratio is qph/q, so the
+// limited value is 0 (opposite signs), q (|qph| >= |q|) or qph: a minmod,
+// evaluated without the division (equal to the reference's product to within
+// its roundings); below tiny the formula as written, k = qph / tiny^2 in
+// hand.  Selections only: lanes on either side of tiny do not diverge (with
+// the branch, 2.10 -> 1.74 ms a launch on 128x256x512; FP64 work did not
+// change, the branch's re-convergence and the second product did).
+__device__ __forceinline__ double sld_limiter(double q, double qph, double k, double tiny) {
+  const double kq = q * k;
+  const bool big = fabs(q) >= tiny;
+  const bool whole = big ? fabs(qph) >= fabs(q) : __double2hiint(kq) >= 0x3FF00000;  // kq >= 1
+  const double part = big ? qph : q * kq;
+  const double r = whole ? q : part;
+  return (__double2hiint(q) ^ __double2hiint(qph)) < 0 ? 0.0 : r;
 }
 
 // limited face difference delta at the face whose neighbours are
 // x(-2..+1) around it: qmh = x_{-1}-x_{-2}, qph = x_0-x_{-1}, qp3h = x_1-x_0
 __device__ __forceinline__ double sld_face(double xm2, double xm1, double x0, double x1, double tiny,
-                                         double inv_tiny) {
+                                         double inv_tiny2) {
   double qmh = xm1 - xm2, qph = x0 - xm1, qp3h = x1 - x0;
-  double pl = sld_limiter(qmh, qph, tiny, inv_tiny), pr = sld_limiter(qp3h, qph, tiny, inv_tiny);
+  const double k = inv_tiny2 * qph;
+  double pl = sld_limiter(qmh, qph, k, tiny), pr = sld_limiter(qp3h, qph, k, tiny);
   return qph - 0.5 * (pr + pl);
 }
 
@@ -1599,8 +1600,8 @@ __device__ __forceinline__ double sld_ghost_t(const CssGeo &g, int iv, double q0
 }
 
 // Slope-limited diffusion, all three directions and all nsld fields in one
-// pass.  CTA = a 32 (theta) x 8 (phi) plane tile marching over an r chunk of
-// SLD_RC radii.  Per radius: the plane values of every field (2-point halo)
+// pass.  CTA = a 32 (theta) x 8 (phi) plane tile marching over a chunk of rc
+// radii.  Per radius: the plane values of every field (2-point halo)
 // and the speed plane (1-point halo) go to shared memory, every theta and
 // phi face flux is computed once, the r faces come from a 4-point window
 // per field carried in registers (one new global load per field and
@@ -1615,7 +1616,6 @@ __device__ __forceinline__ double sld_ghost_t(const CssGeo &g, int iv, double q0
 // mean of each radius (sld_val).
 #define SLD_TT 32
 #define SLD_TP 8
-#define SLD_RC 32
 #define SLD_XW (SLD_TT + 4)  // plane row: 36 doubles = 288 B, so 16-byte copies stay aligned
 #define SLD_VW (SLD_TT + 3)
 template <int NF>
@@ -1691,7 +1691,7 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
                                                             const double *__restrict__ av,
                                                             const double *__restrict__ vcc,
                                                             double *__restrict__ dout, unsigned wmask,
-                                                            const double *__restrict__ tb) {
+                                                            const double *__restrict__ tb, int rc) {
   constexpr int off = OFF;  // first diffused field: every field index below is a constant
   extern __shared__ double sm_raw[];
   SldSmem<NF> &S = *reinterpret_cast<SldSmem<NF> *>(sm_raw);
@@ -1701,7 +1701,7 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
   const int nth = g.nth, nphi = g.nphi, nr = g.nr;
   const int tx = threadIdx.x % SLD_TT, ty = threadIdx.x / SLD_TT;
   const int t0 = blockIdx.x * SLD_TT, p0 = blockIdx.y * SLD_TP;
-  const int r0 = blockIdx.z * SLD_RC, r1 = min(r0 + SLD_RC, nr);
+  const int r0 = blockIdx.z * rc, r1 = min(r0 + rc, nr);
   const int it = t0 + tx, ip = p0 + ty;
   const bool live = it < nth && ip < nphi;
   const int itc = min(it, nth - 1), ipc = min(ip, nphi - 1);
@@ -1736,7 +1736,7 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
     if (r0 > 0) {
       const double vc = __ldg(vcc + css_idx(g, itc, ipc, r0)), vcm = __ldg(vcc + css_idx(g, itc, ipc, r0 - 1));
       carry[f] = (g.sld_coef * sqrt(0.5 * (vc + vcm))) *
-                 (sld_face(xr(r0 - 2), win[f][0], win[f][1], win[f][2], g.tinyvar[iv], g.inv_tinyvar[iv]) * g.sld_r[2 * nr + r0]);
+                 (sld_face(xr(r0 - 2), win[f][0], win[f][1], win[f][2], g.tinyvar[iv], g.inv_tinyvar2[iv]) * g.sld_r[2 * nr + r0]);
     }
   }
   sld_issue_plane<NF>(g, v, av, vcc, S, cp, 0, r0, off);
@@ -1805,7 +1805,7 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
     // on 128x256x512)
 #pragma unroll
     for (int f = 0; f < NF; f++) {
-      const double tiny = g.tinyvar[f + off], itiny = g.inv_tinyvar[f + off];
+      const double tiny = g.tinyvar[f + off], itiny = g.inv_tinyvar2[f + off];
       const double *xr = &X[f][ty + 2][tx + 1];
       FT[f][ty][tx + 1] = th_hi_in ? st_hi * sld_face(xr[0], xr[1], xr[2], xr[3], tiny, itiny) : 0.0;
       FP[f][ty + 1][tx] = sp_hi * sld_face(X[f][ty + 1][tx + 2], X[f][ty + 2][tx + 2], X[f][ty + 3][tx + 2],
@@ -1839,7 +1839,7 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
       }
       double dup = (ir == nr - 1) ? 0.0
                                   : vr_hi * (sld_face(win[f][0], win[f][1], win[f][2], win[f][3], g.tinyvar[iv],
-                                                      g.inv_tinyvar[iv]) * rhi2);
+                                                      g.inv_tinyvar2[iv]) * rhi2);
       double flux = t3 * (dup - carry[f]);
       if (prR != 1.0) flux = prR * flux;
       double acc = flux;
