@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(DV_NT, M == 32 ? 3 : 4) k_deriv_s(CssGeo g, co
   auto go = [&](auto ord, const auto &xi) {
     constexpr int ORD = decltype(ord)::value;
     if constexpr (M > 0)
-      line_solve_r<ORD, M>(I.x + base, xi, dtype, bdry, lo, hi, G, g.tstride, dn, sc, DIR == 2, I.out + base,
+      line_solve_c<ORD, M>(I.x + base, xi, dtype, bdry, lo, hi, G, g.tstride, dn, sc, DIR == 2, I.out + base,
                            GlobOut{s});
     else
       line_solve_g<ORD>(I.x + base, xi, m, dtype, bdry, lo, hi, G, g.tstride, dn, sc, DIR == 2, sm + threadIdx.x,
@@ -221,14 +221,14 @@ __global__ void __launch_bounds__(64) k_deriv_t(CssGeo g, const __grid_constant_
     // D2bydt2's Neumann datum takes the radial spacing
     if (I.order == 1) {
       if constexpr (M > 0)
-        line_solve_r<1, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, O + lane * SO,
+        line_solve_c<1, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, O + lane * SO,
                            StridedOut{1});
       else
         line_solve<1>(x, 1, m, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, O + lane * SO, 1);
     } else {
       const double d2 = dnum_d2_theta(g, ir);
       if constexpr (M > 0)
-        line_solve_r<2, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, O + lane * SO,
+        line_solve_c<2, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, O + lane * SO,
                            StridedOut{1});
       else
         line_solve<2>(x, 1, m, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, O + lane * SO, 1);

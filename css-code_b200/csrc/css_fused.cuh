@@ -244,10 +244,10 @@ __device__ __forceinline__ void thph_theta_solve(const CssGeo &g, const double *
   const double dn = DT.dnum[bt];
   if (order == 2) {
     if (g.slaplacian)
-      line_solve_r<2, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 2, bdry), g.tstride, dnum_d2_theta(g, T.ir),
+      line_solve_c<2, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 2, bdry), g.tstride, dnum_d2_theta(g, T.ir),
                           dn * dn, 0, O + k * FA_OUT, SwzRow{p});
   } else {
-    line_solve_r<1, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 1, bdry), g.tstride, dn, dn, 0,
+    line_solve_c<1, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 1, bdry), g.tstride, dn, dn, 0,
                         O + k * FA_OUT, SwzRow{p});
   }
 }
@@ -262,10 +262,10 @@ __device__ __forceinline__ void thph_phi_solve(const CssGeo &g, const double *F,
   const double *x = F + thph_foff(MAG, f);
   if (k == 5) {
     if (g.slaplacian)
-      line_solve_r<2, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 2, 0), g.tstride, dn, dn * dn, 1,
+      line_solve_c<2, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 2, 0), g.tstride, dn, dn * dn, 1,
                           O + (k0 + k) * FA_OUT, SwzCol{t});
   } else {
-    line_solve_r<1, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1,
+    line_solve_c<1, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1,
                         O + (k0 + k) * FA_OUT, SwzCol{t});
   }
 }
@@ -278,7 +278,7 @@ __device__ __forceinline__ void thph_wall_rho(const CssGeo &g, const double *F, 
   const int bdry = g.ibct[1], side = DT.lphys[T.bt] ? 0 : 1;
   const double dn = DT.dnum[T.bt];
   double *o = rtw + (((size_t)T.ir * g.nphi + T.p0 + p) * 2 + side) * FM;
-  line_solve_r<1, FM>(F + p * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0, 0.0, tabp(g, 1, T.bt, 1, bdry),
+  line_solve_c<1, FM>(F + p * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0, 0.0, tabp(g, 1, T.bt, 1, bdry),
                       g.tstride, dn, dn, 0, o, StridedOut{1});
 }
 
@@ -605,11 +605,11 @@ __global__ void __launch_bounds__(NTH, NBUF == 2 ? 2 : 3) k_curl_pl(CssGeo g, do
       if (wrp < 2) {  // theta lines (line = phi row p = lane): sin A_phi (ibct 11), A_r (ibct 12)
         const int bdry = g.ibct[wrp == 0 ? 11 : 12];
         const double dn = DT.dnum[T.bt];
-        line_solve_r<1, FM>(F + (size_t)(1 + wrp) * FA_FIELD + lane * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0,
+        line_solve_c<1, FM>(F + (size_t)(1 + wrp) * FA_FIELD + lane * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0,
                             0.0, tabp(g, 1, T.bt, 1, bdry), g.tstride, dn, dn, 0, O + wrp * FA_OUT, SwzRow{lane});
       } else {  // phi lines (line = theta column t = lane): A_r, A_theta
         const double dn = g.d[2].dnum[T.bp];
-        line_solve_r<1, FM>(F + (size_t)(wrp == 2 ? 2 : 0) * FA_FIELD, PhIdx{lane}, 3, 0, 0.0, 0.0,
+        line_solve_c<1, FM>(F + (size_t)(wrp == 2 ? 2 : 0) * FA_FIELD, PhIdx{lane}, 3, 0, 0.0, 0.0,
                             tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1, O + wrp * FA_OUT, SwzCol{lane});
       }
     }
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(CR_NT, 4) k_curl_rs(CssGeo g, double *__restri
   if (wrp < 2) {
     const int bdry = g.ibcr[wrp == 0 ? 10 : 11];
     const double dn = D.dnum[T.br];
-    line_solve_r<1, FM>(H + (size_t)wrp * FB_FIELD + 4 * FM + lane, StridedIn{FM}, dtype_of(D, T.br), bdry, 0.0, 0.0,
+    line_solve_c<1, FM>(H + (size_t)wrp * FB_FIELD + 4 * FM + lane, StridedIn{FM}, dtype_of(D, T.br), bdry, 0.0, 0.0,
                         tabp(g, 0, T.br, 1, bdry), g.tstride, dn, dn, 0, O + wrp * FB_OUT + lane, StridedOut{FM});
   }
   __syncthreads();

@@ -45,7 +45,8 @@ struct HaloD1 {
 // base pointers are __restrict__ parameters of the solvers, so the compiler
 // may move the line's loads ahead of the stores of its results; xi and oi
 // only map indices (a stride, or the fused kernels' halo-apart and swizzled
-// tiles).
+// tiles).  The row functions take any pointer-like P whose xb[k] is the
+// value (a line of FP32 values about a background, for instance).
 struct StridedIn {
   int s;
   __host__ __device__ __forceinline__ int operator()(int j) const { return (j - 1) * s; }
@@ -60,8 +61,8 @@ struct StridedOut {
 // Right-hand side of the first-derivative system, rows written to d[] (a
 // per-thread scratch that aliases the output buffer).  Returns nothing; the
 // caller runs the sweeps.
-template <class X>
-__host__ __device__ __forceinline__ double d1_row_lo1(const double *__restrict__ xb, const X &xi, int dtype, int bdry, double bclo,
+template <class P, class X>
+__host__ __device__ __forceinline__ double d1_row_lo1(P xb, const X &xi, int dtype, int bdry, double bclo,
                                              double dnum, double row2) {
   if (dtype == 1 || dtype == 3) {
     return (-HaloD1::c1) * CSS_X(-3) + HaloD1::c2 * CSS_X(-2) + HaloD1::cnst * CSS_X(-1) +
@@ -78,24 +79,24 @@ __host__ __device__ __forceinline__ double d1_row_lo1(const double *__restrict__
   return r;
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d1_row_lo2(const double *__restrict__ xb, const X &xi, int dtype) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d1_row_lo2(P xb, const X &xi, int dtype) {
   if (dtype == 1 || dtype == 3)
     return (7.0 / 9.0) * (CSS_X(3) - CSS_X(1)) + (1.0 / 36.0) * (CSS_X(4) - CSS_X(0));
   return (-43.0 / 96.0) * CSS_X(1) + (-5.0 / 6.0) * CSS_X(2) + (9.0 / 8.0) * CSS_X(3) + (1.0 / 6.0) * CSS_X(4) +
          (-1.0 / 96.0) * CSS_X(5);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d1_row_hi1(const double *__restrict__ xb, const X &xi, int m, int dtype) {  // row m-1
+template <class P, class X>
+__host__ __device__ __forceinline__ double d1_row_hi1(P xb, const X &xi, int m, int dtype) {  // row m-1
   if (dtype == 2 || dtype == 3)
     return HaloD1::r_c1 * (CSS_X(m) - CSS_X(m - 2)) + HaloD1::r_c2 * (CSS_X(m + 1) - CSS_X(m - 3));
   return (43.0 / 96.0) * CSS_X(m) + (5.0 / 6.0) * CSS_X(m - 1) + (-9.0 / 8.0) * CSS_X(m - 2) +
          (-1.0 / 6.0) * CSS_X(m - 3) + (1.0 / 96.0) * CSS_X(m - 4);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d1_row_hi2(const double *__restrict__ xb, const X &xi, int m, int dtype, int bdry, double bchi,
+template <class P, class X>
+__host__ __device__ __forceinline__ double d1_row_hi2(P xb, const X &xi, int m, int dtype, int bdry, double bchi,
                                              double dnum, double rowm1) {  // row m
   if (dtype == 2 || dtype == 3)
     return HaloD1::r_c1 * CSS_X(m + 1) + HaloD1::r_cnst * CSS_X(m + 2) + HaloD1::r_c4 * CSS_X(m + 3) +
@@ -111,8 +112,8 @@ __host__ __device__ __forceinline__ double d1_row_hi2(const double *__restrict__
   return r;
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d1_row_int(const double *__restrict__ xb, const X &xi, int j) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d1_row_int(P xb, const X &xi, int j) {
   return (7.0 / 9.0) * (CSS_X(j + 1) - CSS_X(j - 1)) + (1.0 / 36.0) * (CSS_X(j + 2) - CSS_X(j - 2));
 }
 
@@ -121,8 +122,8 @@ struct HaloD2 {
   static constexpr double c1 = 12.0 / 11.0, c2 = 3.0 / 44.0, c3 = -1.0 / 990.0;
 };
 
-template <class X>
-__host__ __device__ __forceinline__ double d2_row_lo1(const double *__restrict__ xb, const X &xi, int dtype, int bdry, double bclo, double dnum) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d2_row_lo1(P xb, const X &xi, int dtype, int bdry, double bclo, double dnum) {
   if (dtype == 1 || dtype == 3) {
     double r = HaloD2::c3 * (2.0 * (CSS_X(-3) + CSS_X(3)) + (-27.0) * (CSS_X(-2) + CSS_X(2)) +
                              270.0 * (CSS_X(-1) + CSS_X(1)) + (-490.0) * CSS_X(0));
@@ -138,23 +139,23 @@ __host__ __device__ __forceinline__ double d2_row_lo1(const double *__restrict__
          (-55.0 / 78.0) * CSS_X(4) + (-29.0 / 156.0) * CSS_X(5) + (7.0 / 156.0) * CSS_X(6);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d2_row_lo2(const double *__restrict__ xb, const X &xi, int dtype) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d2_row_lo2(P xb, const X &xi, int dtype) {
   if (dtype == 1 || dtype == 3)
     return HaloD2::c1 * (CSS_X(3) - 2.0 * CSS_X(2) + CSS_X(1)) + HaloD2::c2 * (CSS_X(0) - 2.0 * CSS_X(2) + CSS_X(4));
   return 1.2375 * CSS_X(1) + (-3.0) * CSS_X(2) + 2.325 * CSS_X(3) + (-0.6) * CSS_X(4) + 0.0375 * CSS_X(5);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d2_row_hi1(const double *__restrict__ xb, const X &xi, int m, int dtype) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d2_row_hi1(P xb, const X &xi, int m, int dtype) {
   if (dtype == 2 || dtype == 3)
     return HaloD2::c1 * (CSS_X(m) - 2.0 * CSS_X(m - 1) + CSS_X(m - 2)) +
            HaloD2::c2 * (CSS_X(m - 3) - 2.0 * CSS_X(m - 1) + CSS_X(m + 1));
   return 1.2375 * CSS_X(m) + (-3.0) * CSS_X(m - 1) + 2.325 * CSS_X(m - 2) + (-0.6) * CSS_X(m - 3) + 0.0375 * CSS_X(m - 4);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d2_row_hi2(const double *__restrict__ xb, const X &xi, int m, int dtype, int bdry, double bchi,
+template <class P, class X>
+__host__ __device__ __forceinline__ double d2_row_hi2(P xb, const X &xi, int m, int dtype, int bdry, double bchi,
                                              double dnum) {
   if (dtype == 2 || dtype == 3) {
     double r = HaloD2::c1 * (CSS_X(m + 1) - 2.0 * CSS_X(m) + CSS_X(m - 1)) +
@@ -171,8 +172,8 @@ __host__ __device__ __forceinline__ double d2_row_hi2(const double *__restrict__
          (465.0 / 386.0) * CSS_X(m - 3) + (-547.0 / 1158.0) * CSS_X(m - 4) + (157.0 / 2316.0) * CSS_X(m - 5);
 }
 
-template <class X>
-__host__ __device__ __forceinline__ double d2_row_int(const double *__restrict__ xb, const X &xi, int j) {
+template <class P, class X>
+__host__ __device__ __forceinline__ double d2_row_int(P xb, const X &xi, int j) {
   return HaloD2::c1 * (CSS_X(j + 1) - 2.0 * CSS_X(j) + CSS_X(j - 1)) +
          HaloD2::c2 * (CSS_X(j - 2) - 2.0 * CSS_X(j) + CSS_X(j + 2));
 }
@@ -233,6 +234,78 @@ __host__ __device__ __forceinline__ void line_solve_a(const double *__restrict__
   }
 }
 
+// Tables of a block with halos on both ends, of length M: the sweeps'
+// coefficients do not depend on the run, so they live in constant memory at
+// addresses known at compile time, where an FP64 instruction reads them as an
+// operand (no load).  a, b: the interior row's coefficients times g2.  With
+// them the plane pass of the hydro stage went from 811 to 640 us a launch on
+// 128x256x512, the curl's plane pass from 55 to 49 us and its slab pass from
+// 78 to 68 us on 128x128x256.  The slab pass of the stage keeps the loaded
+// tables: its solves are not what bounds it, and on a shell of two radial
+// blocks, which has no such line, the second form of the code cost 47 -> 51 us.
+template <int ORDER, int M>
+struct HaloTab {
+  double g1[M + 1], g2[M + 1], g3[M + 1], a[M + 1], b[M + 1];
+  constexpr HaloTab() : g1{}, g2{}, g3{}, a{}, b{} {
+    const double alpha = ORDER == 1 ? 1.0 / 3.0 : 2.0 / 11.0;
+    const double ca = ORDER == 1 ? 7.0 / 9.0 : 12.0 / 11.0, cb = ORDER == 1 ? 1.0 / 36.0 : 3.0 / 44.0;
+    g2[1] = 1.0;
+    for (int j = 2; j <= M; j++) {  // tab_p's recurrence
+      const double c3 = alpha * g2[j - 1];
+      g1[j] = -c3;
+      g2[j] = 1.0 / (1.0 - alpha * c3);
+      g3[j] = -alpha * g2[j];
+    }
+    for (int j = 1; j <= M; j++) {
+      a[j] = g2[j] * ca;
+      b[j] = g2[j] * cb;
+    }
+  }
+};
+#ifdef __CUDACC__
+__constant__ const HaloTab<1, 16> kHalo1_16;
+__constant__ const HaloTab<2, 16> kHalo2_16;
+__constant__ const HaloTab<1, 32> kHalo1_32;
+__constant__ const HaloTab<2, 32> kHalo2_32;
+template <int ORDER, int M>
+__device__ __forceinline__ const HaloTab<ORDER, M> &halo_tab() {
+  if constexpr (ORDER == 1 && M == 16) return kHalo1_16;
+  else if constexpr (ORDER == 2 && M == 16) return kHalo2_16;
+  else if constexpr (ORDER == 1) return kHalo1_32;
+  else return kHalo2_32;
+}
+// forward rows first .. last-but-two of such a line: a row is g2 (rhs) + g3 t,
+// one multiply-add on the chain from row to row.  Written with explicit
+// roundings, so that every kernel gives the same bits.
+template <int ORDER, int M, class P, class X>
+__device__ __forceinline__ double halo_row(const HaloTab<ORDER, M> &T, P xb, const X &xi, int j, double t) {
+  double d;
+  if (ORDER == 1) {
+    d = __fma_rn(T.b[j], CSS_X(j + 2) - CSS_X(j - 2), __dmul_rn(T.a[j], CSS_X(j + 1) - CSS_X(j - 1)));
+  } else {
+    const double x0 = CSS_X(j);
+    d = __fma_rn(T.b[j], __fma_rn(-2.0, x0, CSS_X(j - 2)) + CSS_X(j + 2),
+                 __dmul_rn(T.a[j], __fma_rn(-2.0, x0, CSS_X(j + 1)) + CSS_X(j - 1)));
+  }
+  return __fma_rn(T.g3[j], t, d);
+}
+// its first two and last two right-hand sides
+template <int ORDER, int M, class P, class X>
+__device__ __forceinline__ void halo_ends(P xb, const X &xi, double &r1, double &r2, double &rm1, double &rm) {
+  if (ORDER == 1) {
+    r2 = d1_row_lo2(xb, xi, 3);
+    r1 = d1_row_lo1(xb, xi, 3, 0, 0.0, 1.0, r2);
+    rm1 = d1_row_hi1(xb, xi, M, 3);
+    rm = d1_row_hi2(xb, xi, M, 3, 0, 0.0, 1.0, rm1);
+  } else {
+    r1 = d2_row_lo1(xb, xi, 3, 0, 0.0, 1.0);
+    r2 = d2_row_lo2(xb, xi, 3);
+    rm1 = d2_row_hi1(xb, xi, M, 3);
+    rm = d2_row_hi2(xb, xi, M, 3, 0, 0.0, 1.0);
+  }
+}
+#endif
+
 // Same operator with the block length M known at compile time: the sweeps
 // are fully unrolled (the forward values go through the output buffer, so
 // register use stays low); identical arithmetic to line_solve_a.
@@ -240,9 +313,34 @@ template <int ORDER, int M, class X, class O>
 __device__ __forceinline__ void line_solve_ua(const double *__restrict__ xb, const X &xi, int dtype, int bdry, double bclo, double bchi,
                                               const double *__restrict__ G, int ts, double dnum, double scale,
                                               int phi, double *__restrict__ ob, const O &oi) {
+  double r1, r2, rm1, rm;
+  if constexpr (M == 16 || M == 32) {
+    if (dtype == 3) {  // no physical end: the tables are constants (line_solve_h's arithmetic)
+      const HaloTab<ORDER, M> &T = halo_tab<ORDER, M>();
+      halo_ends<ORDER, M>(xb, xi, r1, r2, rm1, rm);
+      double t = __dmul_rn(T.g2[1], r1);
+      ob[oi(0)] = t;
+      t = __fma_rn(T.g3[2], t, __dmul_rn(T.g2[2], r2));
+      ob[oi(1)] = t;
+#pragma unroll
+      for (int j = 3; j <= M - 2; j++) {
+        t = halo_row<ORDER, M>(T, xb, xi, j, t);
+        ob[oi(j - 1)] = t;
+      }
+      t = __fma_rn(T.g3[M - 1], t, __dmul_rn(T.g2[M - 1], rm1));
+      ob[oi(M - 2)] = t;
+      double sol = __fma_rn(T.g3[M], t, __dmul_rn(T.g2[M], rm));
+      ob[oi(M - 1)] = scale * sol;
+#pragma unroll
+      for (int j = M - 1; j >= 1; j--) {
+        sol = __fma_rn(T.g1[j + 1], sol, ob[oi(j - 1)]);
+        ob[oi(j - 1)] = scale * sol;
+      }
+      return;
+    }
+  }
   const double *g1 = G, *g2 = G + ts, *g3 = G + 2 * ts;
   const double a1 = (ORDER == 1) ? -1.0 / 3.0 : -2.0 / 11.0;
-  double r1, r2, rm1, rm;
   if (ORDER == 1) {
     r2 = d1_row_lo2(xb, xi, dtype);
     r1 = d1_row_lo1(xb, xi, dtype, bdry, bclo, dnum, r2);
@@ -282,6 +380,30 @@ __device__ __forceinline__ void line_solve_ua(const double *__restrict__ xb, con
     ob[oi(j - 1)] = scale * sol;
   }
 }
+
+#ifdef __CUDACC__
+// A line with halos on both ends (dtype 3), the forward values in registers.
+template <int ORDER, int M, class X, class O>
+__device__ __forceinline__ void line_solve_h(const double *__restrict__ xb, const X &xi, double scale,
+                                             double *__restrict__ ob, const O &oi) {
+  const HaloTab<ORDER, M> &T = halo_tab<ORDER, M>();
+  double t[M], r1, r2, rm1, rm;
+  halo_ends<ORDER, M>(xb, xi, r1, r2, rm1, rm);
+  t[0] = __dmul_rn(T.g2[1], r1);
+  t[1] = __fma_rn(T.g3[2], t[0], __dmul_rn(T.g2[2], r2));
+#pragma unroll
+  for (int j = 3; j <= M - 2; j++) t[j - 1] = halo_row<ORDER, M>(T, xb, xi, j, t[j - 2]);
+  t[M - 2] = __fma_rn(T.g3[M - 1], t[M - 3], __dmul_rn(T.g2[M - 1], rm1));
+  t[M - 1] = __fma_rn(T.g3[M], t[M - 2], __dmul_rn(T.g2[M], rm));
+  double sol = t[M - 1];
+  ob[oi(M - 1)] = scale * sol;
+#pragma unroll
+  for (int j = M - 1; j >= 1; j--) {
+    sol = __fma_rn(T.g1[j + 1], sol, t[j - 1]);
+    ob[oi(j - 1)] = scale * sol;
+  }
+}
+#endif
 
 // Same arithmetic as line_solve_ua with the forward values held in
 // registers instead of the output buffer: the forward sweep then only
@@ -331,6 +453,18 @@ __device__ __forceinline__ void line_solve_r(const double *__restrict__ xb, cons
     ob[oi(j - 1)] = scale * sol;
   }
 }
+
+#ifdef __CUDACC__
+// line_solve_r with the constant tables where both ends are halos
+template <int ORDER, int M, class X, class O>
+__device__ __forceinline__ void line_solve_c(const double *__restrict__ xb, const X &xi, int dtype, int bdry,
+                                             double bclo, double bchi, const double *__restrict__ G, int ts,
+                                             double dnum, double scale, int phi, double *__restrict__ ob,
+                                             const O &oi) {
+  if (dtype == 3) line_solve_h<ORDER, M>(xb, xi, scale, ob, oi);
+  else line_solve_r<ORDER, M>(xb, xi, dtype, bdry, bclo, bchi, G, ts, dnum, scale, phi, ob, oi);
+}
+#endif
 
 // pointer-and-stride forms: x[(j-1)*sx], out[(j-1)*so]
 template <int ORDER>
