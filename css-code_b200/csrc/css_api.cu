@@ -26,6 +26,7 @@
 #include "css_lap.cuh"
 #include "css_inout.cuh"
 #include "css_fused.cuh"
+#include "css_stage.cuh"
 #include "css_voronoi.h"
 
 using namespace css;
@@ -103,8 +104,12 @@ struct css_ctx {
   long long launches;
   int tl_theta, tl_phi, tl_r;
   int phi_pers = 0;                 // 1: persistent double-buffered phi kernel (autotuned)
-  int fused_ok = 0;                 // the run qualifies for the two-pass RK4 stage (css_fused.cuh)
+  int fused_ok = 0;                 // the run qualifies for the two-pass RK4 stage of 32-point blocks (css_fused.cuh)
   int fused = 0;                    // 1: FP64 RK4 stages run k_thph + k_rstage
+  int two = 0;                      // 1: the other stages run k_thph + k_rstage_g (css_stage.cuh)
+  int maps = 0;                     // the TMA maps of the FP64 state buffers exist
+  PlaneMaps fmaps[2];               // vA, vB as FP32 stage states (mixed precision)
+  SlabMaps fslab[2];
   int curl_tp = 2;                  // B = curl A's theta and phi parts: 0 two passes, 1 one pass (k_curl_tp),
                                     // 2 one pass from TMA-staged planes (k_curl_pl) where the maps exist
   int nsm = 148;                    // SMs of the device
@@ -323,6 +328,24 @@ static int setup_mt() {
   return CSS_OK;
 }
 
+template <int MAG, typename TS>
+static int setup_thph() {
+  const int mx = (int)ThphCfg<MAG, TS>::SMEM;
+  CUDA_TRY(cudaFuncSetAttribute(k_thph<MAG, TS, 32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  CUDA_TRY(cudaFuncSetAttribute(k_thph<MAG, TS, 32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  CUDA_TRY(cudaFuncSetAttribute(k_thph<MAG, TS, 16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  CUDA_TRY(cudaFuncSetAttribute(k_thph<MAG, TS, 16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  return CSS_OK;
+}
+template <typename TS, typename TO, int KIND, int... STG>
+static int setup_stage() {
+  const int mx = (int)SG_SMEM;
+  for (cudaError_t e : {cudaFuncSetAttribute(k_rstage_g<TS, TO, KIND, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             mx)...})
+    CUDA_TRY(e);
+  return CSS_OK;
+}
+
 static int setup_kernels() {
   static bool done = false;
   if (done) return CSS_OK;
@@ -341,8 +364,19 @@ static int setup_kernels() {
   int mx = 200 * 1024;
 #define CSS_FUSED_ATTR(K, CFG) \
   CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CFG::SMEM))
-  CSS_FUSED_ATTR(k_thph<0>, ThphCfg<0>);
-  CSS_FUSED_ATTR(k_thph<1>, ThphCfg<1>);
+  if (int rc2 = setup_thph<0, double>()) return rc2;
+  if (int rc2 = setup_thph<0, float>()) return rc2;
+  if (int rc2 = setup_thph<1, double>()) return rc2;
+  if (int rc2 = setup_thph<1, float>()) return rc2;
+  if (int rc2 = setup_stage<double, double, 0, 1, 2, 3, 4, -1>()) return rc2;
+  if (int rc2 = setup_stage<double, double, 1, 1, 2, 3, 4, -1>()) return rc2;
+  if (int rc2 = setup_stage<double, double, 2, 1, 2, 3, 4, -1>()) return rc2;
+  if (int rc2 = setup_stage<double, float, 0, 1, -1>()) return rc2;
+  if (int rc2 = setup_stage<double, float, 2, 1, -1>()) return rc2;
+  if (int rc2 = setup_stage<float, float, 0, 2, 3, -1>()) return rc2;
+  if (int rc2 = setup_stage<float, float, 2, 2, 3, -1>()) return rc2;
+  if (int rc2 = setup_stage<float, double, 0, 4, -1>()) return rc2;
+  if (int rc2 = setup_stage<float, double, 2, 4, -1>()) return rc2;
   CSS_FUSED_ATTR((k_rstage<0, 1>), RstageCfg<0>);
   CSS_FUSED_ATTR((k_rstage<0, 2>), RstageCfg<0>);
   CSS_FUSED_ATTR((k_rstage<0, 3>), RstageCfg<0>);
@@ -440,8 +474,8 @@ static bool plane_maps(css_ctx *c) {
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return false;
-    // the stage kernel's slab box: 32 theta x 1 phi x 40 r
-    const cuuint32_t bslab[4] = {FM, 1, FM + 8, 1};
+    // the stage kernels' slab box: 32 theta x 1 phi x the radial block with its halos
+    const cuuint32_t bslab[4] = {FM, 1, (cuuint32_t)(g.d[0].maxm + 8), 1};
     if (encode(&c->smaps[k].slab, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, bufs[k], dims, strides, bslab, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -462,11 +496,31 @@ static bool plane_maps(css_ctx *c) {
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       memset(&c->pmaps[4], 0, sizeof(PlaneMaps));  // the ohmic curl keeps its tile kernels
     else {
-      const cuuint32_t bslab[4] = {FM, 1, FM + 8, 1};
+      const cuuint32_t bslab[4] = {FM, 1, (cuuint32_t)(g.d[0].maxm + 8), 1};
       if (encode(&c->vs_slab.slab, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, c->vs, dims, strides, bslab, estr,
                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
         c->vs_map = 1;
+    }
+  }
+  if (c->p.precision == 1) {  // the FP32 stage states in vA and vB
+    for (int k = 0; k < 2; k++) {
+      void *buf = k == 0 ? c->vA : c->vB;
+      const cuuint64_t dims[4] = {(cuuint64_t)g.nth, (cuuint64_t)g.nphi, (cuuint64_t)g.nr, (cuuint64_t)c->nv};
+      const cuuint64_t strides[3] = {(cuuint64_t)g.nth * 4, (cuuint64_t)g.nth * g.nphi * 4, (cuuint64_t)c->ncell * 4};
+      const cuuint32_t estr[4] = {1, 1, 1, 1};
+      const cuuint32_t bmain[4] = {FA_FRW, FM, 1, 1}, bhalo[4] = {FM, 4, 1, 1},
+                       bslab[4] = {FM, 1, (cuuint32_t)(g.d[0].maxm + 8), 1};
+      if (encode(&c->fmaps[k].main, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, buf, dims, strides, bmain, estr,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+          encode(&c->fmaps[k].halo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, buf, dims, strides, bhalo, estr,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+          encode(&c->fslab[k].slab, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, buf, dims, strides, bslab, estr,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
     }
   }
   {  // rtw: (theta 32, side 2, phi, r), box 32 x 1 x 1 x 32
@@ -900,7 +954,12 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   c->fused_ok = c->mt[0] == 32 && c->mt[1] == 32 && c->mt[2] == 32 && p.precision == 0 &&
                 (p.time_stepper == 4 || p.time_stepper == 0) && !p.laplacian && !p.do_radheat && !p.top_inout &&
                 !p.bot_inout && !p.bottom_specified;
-  if (c->fused_ok) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
+  // its general form (css_stage.cuh): 16- or 32-point blocks in theta and phi,
+  // any radial block whose slab fits shared memory, either storage of the
+  // stage states, any stepper, open radial faces and explicit viscosity; radiative
+  // diffusion alone sits between the radial terms and the update
+  c->two = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, 8) <= SG_SMEM && !p.do_radheat;
+  if (c->two) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
   if (p.precision == 1) {  // backgrounds of the FP32 stage states, refreshed at every upload
     ALLOC(c->bg2, 2 * (size_t)nr * nth * sizeof(double));
     cudaMemset(c->bg2, 0, 2 * (size_t)nr * nth * sizeof(double));
@@ -913,7 +972,8 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
     ALLOC(c->cyc, CY.size() * sizeof(double));
     cudaMemcpy(c->cyc, CY.data(), CY.size() * sizeof(double), cudaMemcpyHostToDevice);
   }
-  if (c->fused_ok && !plane_maps(c)) c->fused_ok = 0;
+  c->maps = c->two && plane_maps(c);
+  if (!c->maps) c->two = c->fused_ok = 0;
   c->fused = c->fused_ok;
   *out = c;
   return CSS_OK;
@@ -943,7 +1003,7 @@ static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
     mi = ad == c->v0 + 5 * c->ncell ? 0 : (ad == c->vA + 5 * c->ncell ? 1 : (ad == c->vB + 5 * c->ncell ? 2 : -1));
     if (mi < 0 && c->vs_map && ad == c->vs + 5 * c->ncell) mi = 4;  // the SLD tendency
   }
-  if (c->curl_tp == 2 && c->fused_ok && mi >= 0 && c->mt[1] == 32 && c->mt[2] == 32) {
+  if (c->curl_tp == 2 && c->maps && mi >= 0 && c->mt[1] == 32 && c->mt[2] == 32) {
     prof_begin(c, KI_CURL_THETA);
     // one plane buffer per CTA and three CTAs of 128 threads per SM: 1.51 ms
     // per curl on MHD 256x512x1024, against 2.13 ms for two buffers per CTA
@@ -975,7 +1035,7 @@ static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
     prof_end(c);
     if (int rc = check_launch(c)) return rc;
   }
-  if (c->curl_tp == 2 && c->fused_ok && mi >= 0 && c->mt[0] == 32 && c->mt[1] == 32) {  // radial part from TMA slabs
+  if (c->curl_tp == 2 && c->maps && mi >= 0 && c->mt[0] == 32 && c->mt[1] == 32) {  // radial part from TMA slabs
     prof_begin(c, KI_CURL_R);
     k_curl_rs<<<g.d[0].nb * g.d[1].nb * g.nphi, CR_NT, CR_SMEM, c->stream>>>(
         g, out, mi < 3 ? c->smaps[mi] : c->vs_slab, apply_bc, c->flag);
@@ -1168,12 +1228,17 @@ static int launch_inout(css_ctx *c, const double *cur) {
   return check_launch(c);
 }
 
+template <typename TS, typename TO>
+static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, double ca, double cb,
+                            double dsld, bool with_sld);
+
 // with_sld: the step's slope-limited diffusion tendency of `cur` into c->vs,
 // launched after the radial kernel (the theta kernel has left T(cur) in
 // tbuf) and before the update that reads vs
 template <typename TS, typename TO>
 static int launch_rhs(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, double ca = 0.0, double cb = 0.0,
                       double dsld = 0.0, bool with_sld = false) {
+  if (stage > 0 && c->two) return launch_stage_two(c, cur, nx, stage, dtcur, ca, cb, dsld, with_sld);
   const CssGeo &g = c->g;
   const int mag = g.magnetic;
   if (mag) {
@@ -1292,7 +1357,7 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
   // radii a CTA marches over: the chunk that takes the fewest radii in a row
   // over the waves of two CTAs an SM, where a chunk's start (its windows, the
   // first planes) counts as one and a half.  On large shells that is 32 or
-  // 16; on 64x64x128, 32 left 84 of 148 SMs idle (279 us a launch, 99 with 8).
+  // 16; on 64x64x128, 32 left 84 of 148 SMs idle (279 us against 97 with 8).
   const long long ntile = (long long)((g.nth + SLD_TT - 1) / SLD_TT) * ((g.nphi + SLD_TP - 1) / SLD_TP);
   int rc = 32;
   double best = 1e30;
@@ -1338,25 +1403,41 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
   return CSS_OK;
 }
 
-// One RK4 stage in two passes (css_fused.cuh): [curl] -> k_thph -> [SLD
-// of the step's start in stage 1] -> k_rstage<stage>
-static int launch_stage_fused(css_ctx *c, const double *cur, double *nx, int stage, double dtcur, bool with_sld) {
-  const CssGeo &g = c->g;
-  const int mag = g.magnetic;
-  if (mag)
-    if (int rc = launch_curl(c, cur + 5 * c->ncell, c->bf, 1)) return rc;
-  // persistent kernels: one CTA per SM
+// the plane pass of a stage (k_thph: the theta and phi sweeps of `cur`),
+// persistent, one CTA per SM
+template <typename TS>
+static int launch_plane(css_ctx *c, const TS *cur, int *map) {
+  const void *bufs[3] = {c->v0, c->vA, c->vB};
+  int mi = 0;
+  while (mi < 3 && bufs[mi] != (const void *)cur) mi++;
+  if (mi == 3 || (sizeof(TS) == 4 && mi == 0)) { set_err("launch_plane: stage input is not a state buffer"); return CSS_ERR_ARG; }
+  *map = mi;
+  const PlaneMaps &mc = sizeof(TS) == 4 ? c->fmaps[mi - 1] : c->pmaps[mi], &mb = c->pmaps[3];
   const dim3 ga(c->nsm);
   prof_begin(c, KI_THPH);
-  const int mi = cur == c->v0 ? 0 : (cur == c->vA ? 1 : (cur == c->vB ? 2 : -1));
-  if (mi < 0) { set_err("launch_stage_fused: stage input is not a state buffer"); return CSS_ERR_ARG; }
-  const PlaneMaps &mc = c->pmaps[mi], &mb = c->pmaps[3];
-  if (mag) k_thph<1><<<ga, FNT, ThphCfg<1>::SMEM, c->stream>>>(g, cur, c->bf, c->dv, c->tbuf, c->rtw, mc, mb, c->flag);
-  else k_thph<0><<<ga, FNT, ThphCfg<0>::SMEM, c->stream>>>(g, cur, c->bf, c->dv, c->tbuf, c->rtw, mc, mb, c->flag);
+#define CSS_THPH(M, BT, BP)                                                                                       \
+  k_thph<M, TS, BT, BP><<<ga, FNT, ThphCfg<M, TS>::SMEM, c->stream>>>(c->g, c->dv, c->tbuf, c->rtw, mc, mb, c->flag)
+  switch ((c->g.magnetic ? 10000 : 0) + c->mt[1] * 100 + c->mt[2]) {
+    case 3232: CSS_THPH(0, 32, 32); break;
+    case 3216: CSS_THPH(0, 32, 16); break;
+    case 1632: CSS_THPH(0, 16, 32); break;
+    case 1616: CSS_THPH(0, 16, 16); break;
+    case 13232: CSS_THPH(1, 32, 32); break;
+    case 13216: CSS_THPH(1, 32, 16); break;
+    case 11632: CSS_THPH(1, 16, 32); break;
+    case 11616: CSS_THPH(1, 16, 16); break;
+    default: set_err("launch_plane: blocks of %d and %d points", c->mt[1], c->mt[2]); return CSS_ERR_ARG;
+  }
+#undef CSS_THPH
   prof_end(c);
-  if (int rc = check_launch(c)) return rc;
-  if (with_sld)
-    if (int rc = launch_sld(c, cur, cur + 5 * c->ncell, c->vs, c->tbuf)) return rc;
+  return check_launch(c);
+}
+
+// the stage pass of an FP64 RK4 run with closed radial faces and 32-point
+// blocks in r and theta (k_rstage); mi: the state buffer `cur` is
+static int launch_rstage32(css_ctx *c, const double *cur, double *nx, int stage, double dtcur, int mi) {
+  const CssGeo &g = c->g;
+  const int mag = g.magnetic;
   // hydro: one tile per CTA; MHD: persistent, one CTA per SM
   const int nrtile = g.d[0].nb * g.d[1].nb * g.nphi;
   const dim3 gb(mag ? std::min(c->nsm, nrtile) : nrtile);
@@ -1374,9 +1455,63 @@ static int launch_stage_fused(css_ctx *c, const double *cur, double *nx, int sta
     case 12: CSS_RSTAGE(1, 2); break;
     case 13: CSS_RSTAGE(1, 3); break;
     case 14: CSS_RSTAGE(1, 4); break;
-    default: set_err("launch_stage_fused: stage %d", stage); return CSS_ERR_ARG;
+    default: set_err("launch_rstage32: stage %d", stage); return CSS_ERR_ARG;
   }
 #undef CSS_RSTAGE
+  prof_end(c);
+  return check_launch(c);
+}
+
+// A stage as the plane pass and the general stage pass (css_stage.cuh):
+// [curl] -> k_thph -> [explicit viscosity] -> [face sums of open radial
+// faces] -> [SLD of the step's start] -> k_rstage (FP64 RK4 stages of 32-point
+// blocks, closed faces: it holds the MHD slab of 32 radii in one persistent
+// 512-thread CTA an SM) or k_rstage_g
+template <typename TS, typename TO>
+static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, double ca, double cb,
+                            double dsld, bool with_sld) {
+  const CssGeo &g = c->g;
+  const int mag = g.magnetic;
+  if (mag)
+    if (int rc = launch_curl(c, cur + 5 * c->ncell, c->bf, 1)) return rc;
+  int mi;
+  if (int rc = launch_plane(c, cur, &mi)) return rc;
+  if constexpr (sizeof(TS) == 8) {
+    if (c->p.laplacian)
+      if (int rc = launch_lap(c, (const double *)cur)) return rc;
+    if (c->io)
+      if (int rc = launch_inout(c, (const double *)cur)) return rc;
+    if (with_sld)
+      if (int rc = launch_sld(c, (const double *)cur, (const double *)cur + 5 * c->ncell, c->vs, c->tbuf)) return rc;
+  }
+  if constexpr (sizeof(TS) == 8 && sizeof(TO) == 8)
+    if (stage <= 4 && c->mt[0] == 32 && c->mt[1] == 32 && !c->io) return launch_rstage32(c, cur, nx, stage, dtcur, mi);
+  prof_begin(c, KI_RSTAGE);
+  const dim3 gr(g.d[0].nb * ((g.nth + 31) / 32), g.nphi);
+  const size_t smem = stage_smem(mag, g.d[0].maxm, (int)sizeof(TS));
+  const SlabMaps &sc = sizeof(TS) == 4 ? c->fslab[mi - 1] : c->smaps[mi];
+#define CSS_STAGE(K, S)                                                                                              \
+  k_rstage_g<TS, TO, K, S><<<gr, SG_NT, smem, c->stream>>>(g, cur, c->bf, c->dv, c->v0, c->vs, nx, c->tbuf, c->rtw, \
+                                                           c->mt[1], stage, dtcur, ca, cb, dsld, c->flag, sc, c->smaps[3])
+#define CSS_STAGES(K)                                                                           \
+  do {                                                                                          \
+    if (stage >= 5) CSS_STAGE(K, -1);                                                           \
+    else if constexpr (sizeof(TS) == 8 && sizeof(TO) == 8) {                                    \
+      if (stage == 1) CSS_STAGE(K, 1);                                                          \
+      else if (stage == 2) CSS_STAGE(K, 2);                                                     \
+      else if (stage == 3) CSS_STAGE(K, 3);                                                     \
+      else CSS_STAGE(K, 4);                                                                     \
+    } else if constexpr (sizeof(TS) == 8) CSS_STAGE(K, 1); /* mixed: vars0 -> U1 */             \
+    else if constexpr (sizeof(TO) == 8) CSS_STAGE(K, 4);   /* U3 -> vars0 */                    \
+    else if (stage == 2) CSS_STAGE(K, 2);                                                       \
+    else CSS_STAGE(K, 3);                                                                       \
+  } while (0)
+  if (mag) CSS_STAGES(2);
+  else if (c->io) {
+    if constexpr (sizeof(TS) == 8 && sizeof(TO) == 8) CSS_STAGES(1);  // open radial faces: FP64 runs only
+  } else CSS_STAGES(0);
+#undef CSS_STAGES
+#undef CSS_STAGE
   prof_end(c);
   return check_launch(c);
 }
@@ -1454,12 +1589,6 @@ static int step_stages(css_ctx *c, double dt) {
     if (int rc = launch_rhs(c, (const float *)fB, fA, 3, dt)) return rc;
     if (int rc = launch_rhs(c, (const float *)fA, c->v0, 4, dt)) return rc;
     return CSS_OK;
-  }
-  if (c->fused) {
-    if (int rc = launch_stage_fused(c, c->v0, c->vA, 1, dt / 2.0, sld)) return rc;
-    if (int rc = launch_stage_fused(c, c->vA, c->vB, 2, dt / 2.0, false)) return rc;
-    if (int rc = launch_stage_fused(c, c->vB, c->vA, 3, dt, false)) return rc;
-    return launch_stage_fused(c, c->vA, c->v0, 4, dt, false);
   }
   if (int rc = launch_rhs(c, (const double *)c->v0, c->vA, 1, dt / 2.0, 0.0, 0.0, 0.0, sld)) return rc;
   if (int rc = launch_rhs(c, (const double *)c->vA, c->vB, 2, dt / 2.0)) return rc;
@@ -2048,6 +2177,7 @@ extern "C" int css_set_fused(css_ctx *c, int on) {
     return CSS_ERR_ARG;
   }
   c->fused = on ? 1 : 0;
+  c->two = c->fused;  // off: the four-kernel stage
   return CSS_OK;
 }
 

@@ -1,9 +1,11 @@
-// css_fused.cuh -- the RK4 stage in two passes over HBM, for runs whose
-// virtual blocks are 32 points long in r, theta and phi (FP64 state, RK4,
-// closed radial faces, SLaplacian/SLD physics; css_create decides).
+// css_fused.cuh -- the RK stage in two passes over HBM.  The plane pass takes
+// theta and phi blocks of 16 or 32 points and FP64 or FP32 stage states; the
+// slab pass here takes 32-point blocks in r and theta, FP64 RK4 stages and
+// closed radial faces (css_stage.cuh has the others; css_create and
+// launch_stage_two decide).
 //
-//   k_thph    tiles of one (theta block, phi block, radius) plane: the
-//             32x32 plane of the two blocks with 4-point halos in theta and
+//   k_thph    tiles of 32 theta x 32 phi of one radius (one or two blocks in
+//             each direction): the plane with 4-point halos in theta and
 //             phi is staged once in shared memory, and the theta and phi
 //             line solves of every field run at once; Source_Theta_Terms
 //             (+ Lorentz, + Induction_Terms), Phi_Terms (+ Lorentz) and, on
@@ -65,7 +67,13 @@ __host__ __device__ constexpr int thph_foff(int mag, int f) {
   return f * FA_FIELD - ((mag && f == 7) ? 8 * FM : 0);
 }
 
-template <int MAG>
+// FP32 stage states: a field's plane arrives as floats in the upper end of its
+// own FP64 plane (rows of 44 floats, 16-byte multiples; then the eight halo
+// rows) and is widened in place, the background added
+constexpr int FA_FRW = 44;
+constexpr int FA_FOFF = FA_FIELD * 8 - (FM * FA_FRW + 8 * FM) * 4;  // bytes: 6144, 128-byte aligned
+
+template <int MAG, typename TS = double>
 struct ThphCfg {
   static constexpr int NF = MAG ? 8 : 5;     // rho w v u s [bt bp br]
   // derivative tiles: both directions' at once (theta 0-5, phi 6-11 hydro;
@@ -76,11 +84,12 @@ struct ThphCfg {
   // hydro stages the next tile's plane into a second buffer while it
   // computes the current one; MHD (eight fields) has room for one plane,
   // refilled with the next tile's once the solves are done with it
-  static constexpr int NBUF = MAG ? 1 : 2;
+  static constexpr int NBUF = MAG || sizeof(TS) == 4 ? 1 : 2;
   // + one mbarrier per plane buffer
   static constexpr size_t SMEM = 8 * ((size_t)NBUF * PLANE + (size_t)NO * FA_OUT + NBUF);
   // bytes one plane's copies deliver
-  static constexpr unsigned TX = 8u * PLANE;
+  static constexpr unsigned TX =
+      sizeof(TS) == 4 ? 5u * (8 * FA_FIELD - FA_FOFF) + (MAG ? 8u * (2 * FA_FIELD + FA_MAIN) : 0u) : 8u * PLANE;
 };
 static_assert(ThphCfg<1>::SMEM <= 232448, "MHD plane pass: one plane and sixteen tiles fit 227 KB");
 
@@ -90,22 +99,27 @@ static_assert(ThphCfg<1>::SMEM <= 232448, "MHD plane pass: one plane and sixteen
 struct ThIdx {
   __device__ __forceinline__ int operator()(int j) const { return j + 3; }
 };
-// phi line at theta column t: base = the field
+// phi line at theta column t: base = the field; the block's first row is
+// row R0 of the tile, and the tile's last row is len - 1 (the halo rows follow
+// it: len is FM except on the last tile of an odd number of 16-point blocks)
+template <int M, int R0>
 struct PhIdx {
-  int t;
+  int t, len;
   __device__ __forceinline__ int operator()(int j) const {
-    if (j < 1) return FA_MAIN + (j + 3) * FM + t;
-    if (j > FM) return FA_MAIN + (j - FM + 3) * FM + t;
-    return (j - 1) * FA_RW + t + 4;
+    const int r = R0 + j - 1;
+    if (r < 0) return FA_MAIN + (r + 4) * FM + t;
+    if (r >= FM) return FA_MAIN + (r - FM + 4) * FM + t;
+    if (M < FM && R0 == 0 && r >= M && len == M) return FA_MAIN + (r - M + 4) * FM + t;
+    return r * FA_RW + t + 4;
   }
 };
-struct SwzRow {  // theta line p of a derivative tile: element (p, j)
-  int p;
-  __device__ __forceinline__ int operator()(int j) const { return p * FM + (j ^ (p & 15)); }
+struct SwzRow {  // theta line p of a derivative tile: element (p, c + j)
+  int p, c;
+  __device__ __forceinline__ int operator()(int j) const { return p * FM + ((c + j) ^ (p & 15)); }
 };
-struct SwzCol {  // phi line t of a derivative tile: element (j, t)
-  int t;
-  __device__ __forceinline__ int operator()(int j) const { return j * FM + (t ^ (j & 15)); }
+struct SwzCol {  // phi line t of a derivative tile: element (r + j, t)
+  int t, r;
+  __device__ __forceinline__ int operator()(int j) const { return (r + j) * FM + (t ^ ((r + j) & 15)); }
 };
 __device__ __forceinline__ double swz(const double *O, int p, int t) { return O[p * FM + (t ^ (p & 15))]; }
 
@@ -160,9 +174,9 @@ constexpr long long kWaitCycles = 4000000000ll;
 // bit of the step flag a timed-out wait sets (bit 0 is a non-finite state)
 constexpr int kFlagTimeout = 2;
 
-// The tensor maps of one state buffer: 4-D (theta, phi, r, field) FP64,
-// boxes of the plane's main rows (42 theta x 32 phi) and of its phi halo
-// (32 theta x 4 phi).
+// The tensor maps of one state buffer: 4-D (theta, phi, r, field), boxes of
+// the plane's main rows (42 theta x 32 phi; 44 of an FP32 stage state, whose
+// rows are then whole 16-byte units) and of its phi halo (32 theta x 4 phi).
 struct PlaneMaps {
   CUtensorMap main, halo;
 };
@@ -179,116 +193,189 @@ struct SlabMaps {
 // stage input (FP64), bf = B (MHD), dv = tendency (written), tbuf = T
 // (written).
 // ---------------------------------------------------------------------------
+// A tile is 32 x 32 points whatever the blocks: one block of 32 or two of 16
+// in each direction (BT, BP); an odd number of 16-point blocks leaves the
+// last tile half empty.  bt, bp: the tile's first block.
 struct ThphTile {
   int bt, bp, ir, t0, p0;
 };
+template <int BT, int BP>
+__device__ __forceinline__ int thph_tiles(const CssGeo &g) {
+  return g.nr * ((g.d[1].nb * BT + FM - 1) / FM) * ((g.d[2].nb * BP + FM - 1) / FM);
+}
+template <int BT, int BP>
 __device__ __forceinline__ ThphTile thph_tile(const CssGeo &g, int q) {
-  const int nbp = g.d[2].nb, nbt = g.d[1].nb;
+  const int ntp = (g.d[2].nb * BP + FM - 1) / FM, ntt = (g.d[1].nb * BT + FM - 1) / FM;
   ThphTile T;
-  T.bp = q % nbp;
-  const int r = q / nbp;
-  T.bt = r % nbt;
-  T.ir = r / nbt;
-  T.t0 = g.d[1].start[T.bt];
-  T.p0 = g.d[2].start[T.bp];
+  const int tp = q % ntp, r = q / ntp, tt = r % ntt;
+  T.bp = tp * (FM / BP);
+  T.bt = tt * (FM / BT);
+  T.ir = r / ntt;
+  T.t0 = tt * FM;
+  T.p0 = tp * FM;
   return T;
 }
 
 // stage the plane with TMA boxes (called by one thread): per field the main
 // rows over theta t0-4 .. t0+37 (zero outside [0, nth)) and the two 4-row
-// phi halos (periodic; blocks are 32 long, so a halo box never wraps)
-template <int NF>
+// phi halos (periodic; tiles start at multiples of 32 and blocks are 16 or 32
+// long, so a halo box never wraps)
+template <int NF, typename TS>
 __device__ __forceinline__ void thph_stage_tma(const CssGeo &g, const PlaneMaps &mc, const PlaneMaps &mb,
                                                const ThphTile &T, double *F, uint64_t *bar) {
   const int plo = T.p0 >= 4 ? T.p0 - 4 : g.nphi - 4;
   const int phi = T.p0 + FM < g.nphi ? T.p0 + FM : 0;
   constexpr int MAGF = NF == 8;
-  mbar_expect_tx(bar, 8u * ThphCfg<MAGF>::PLANE);
+  mbar_expect_tx(bar, ThphCfg<MAGF, TS>::TX);
 #pragma unroll
   for (int f = 0; f < NF; f++) {
     const PlaneMaps &m = f < 5 ? mc : mb;
     const int w = f < 5 ? f : f - 5;
-    double *Fd = F + thph_foff(MAGF, f);
+    double *Fd = F + thph_foff(MAGF, f), *Hd = Fd + FA_MAIN, *Hh = Hd + 4 * FM;
+    if (sizeof(TS) == 4 && f < 5) {
+      Fd = reinterpret_cast<double *>(reinterpret_cast<char *>(Fd) + FA_FOFF);
+      Hd = reinterpret_cast<double *>(reinterpret_cast<char *>(Fd) + FM * FA_FRW * 4);
+      Hh = reinterpret_cast<double *>(reinterpret_cast<char *>(Hd) + 4 * FM * 4);
+    }
     tma_load_4d(Fd, &m.main, T.t0 - 4, T.p0, T.ir, w, bar);
     if (MAGF && f == 6) continue;  // B_phi: main rows only
-    tma_load_4d(Fd + FA_MAIN, &m.halo, T.t0, plo, T.ir, w, bar);
-    tma_load_4d(Fd + FA_MAIN + 4 * FM, &m.halo, T.t0, phi, T.ir, w, bar);
+    tma_load_4d(Hd, &m.halo, T.t0, plo, T.ir, w, bar);
+    tma_load_4d(Hh, &m.halo, T.t0, phi, T.ir, w, bar);
   }
 }
 
+// widen a plane of FP32 state fields in place (the whole CTA): each thread
+// takes its values into registers, and after a barrier writes them as FP64 at
+// their places, rho and s with their background (theta, r)
+__device__ __forceinline__ void thph_widen(const CssGeo &g, const ThphTile &T, double *F) {
+  constexpr int K = (FA_FIELD + FNT - 1) / FNT;
+  float v[5][K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = threadIdx.x + k * FNT, p = i / FA_RW, c = i - p * FA_RW;
+    if (i < FA_FIELD) {
+      const int o = i < FA_MAIN ? p * FA_FRW + c : FM * FA_FRW + i - FA_MAIN;
+#pragma unroll
+      for (int f = 0; f < 5; f++)
+        v[f][k] = reinterpret_cast<const float *>(reinterpret_cast<const char *>(F + f * FA_FIELD) + FA_FOFF)[o];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = threadIdx.x + k * FNT, p = i / FA_RW, c = i - p * FA_RW;
+    if (i < FA_FIELD) {
+      const int t = i < FA_MAIN ? T.t0 - 4 + c : T.t0 + ((i - FA_MAIN) & (FM - 1));
+      const bool in = t >= 0 && t < g.nth;
+      const size_t b = in ? bgi(g, T.ir, t) : 0;
+#pragma unroll
+      for (int f = 0; f < 5; f++) {
+        double x = (double)v[f][k];
+        if (f == 0 && in) x += __ldg(bg_rho(g) + b);
+        if (f == 4 && in) x += __ldg(bg_s(g) + b);
+        F[f * FA_FIELD + i] = x;
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // theta line solve of derivative tile k (0 dw 1 dv 2 du 3 ds 4 d2s [5 dbp
-// 6 dbr] then d(rho) off the walls), line (phi row) p
-template <int MAG>
-__device__ __forceinline__ void thph_theta_solve(const CssGeo &g, const double *F, double *O, const ThphTile &T,
-                                                 int k, int p) {
+// 6 dbr] then d(rho) off the walls), line (phi row) p, block bt at column C0
+// of the tile
+template <int MAG, int M, int C0>
+__device__ __forceinline__ void thph_theta_solve(const CssGeo &g, const double *F, double *O, int bt, int ir, int k,
+                                                 int p) {
   const CssDir &DT = g.d[1];
-  const int bt = T.bt;
   int f, var, order = 1;
   if (k < 4) { f = 1 + k; var = 2 + k; }
   else if (k == 4) { f = 4; var = 5; order = 2; }
   else if (MAG && k < 7) { f = k + 1; var = k + 3; }  // bp (8), br (9)
   else { f = 0; var = 1; }
   const int bdry = g.ibct[var];
-  const double *x = F + thph_foff(MAG, f) + p * FA_RW;
+  const double *x = F + thph_foff(MAG, f) + p * FA_RW + C0;
   double lo = 0.0, hi = 0.0;
   const int nth = g.nth;
   if (f == 2) {  // stress-free datum cot(theta)*v on the walls (rhs_mpi.f90:414, :444)
     if (DT.lphys[bt]) lo = (g.cosines[0] / g.sines[0]) * x[4];
-    if (DT.rphys[bt]) hi = (g.cosines[nth - 1] / g.sines[nth - 1]) * x[4 + FM - 1];
+    if (DT.rphys[bt]) hi = (g.cosines[nth - 1] / g.sines[nth - 1]) * x[4 + M - 1];
   }
   if (MAG && f == 6 && g.theta_normal_field) {  // (rhs_mpi.f90:421, :451)
     if (DT.lphys[bt]) lo = -(g.cosines[0] / g.sines[0]) * x[4];
-    if (DT.rphys[bt]) hi = -(g.cosines[nth - 1] / g.sines[nth - 1]) * x[4 + FM - 1];
+    if (DT.rphys[bt]) hi = -(g.cosines[nth - 1] / g.sines[nth - 1]) * x[4 + M - 1];
   }
   const int dtype = dtype_of(DT, bt);
   const double dn = DT.dnum[bt];
   if (order == 2) {
     if (g.slaplacian)
-      line_solve_c<2, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 2, bdry), g.tstride, dnum_d2_theta(g, T.ir),
-                          dn * dn, 0, O + k * FA_OUT, SwzRow{p});
+      line_solve_c<2, M>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 2, bdry), g.tstride, dnum_d2_theta(g, ir),
+                         dn * dn, 0, O + k * FA_OUT, SwzRow{p, C0});
   } else {
-    line_solve_c<1, FM>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 1, bdry), g.tstride, dn, dn, 0,
-                        O + k * FA_OUT, SwzRow{p});
+    line_solve_c<1, M>(x, ThIdx{}, dtype, bdry, lo, hi, tabp(g, 1, bt, 1, bdry), g.tstride, dn, dn, 0,
+                       O + k * FA_OUT, SwzRow{p, C0});
   }
 }
 
 // phi line solve of derivative tile k (0 drho 1 dv 2 dw 3 du 4 ds 5 d2s
-// [6 dbt 7 dbr]) into O + k0 + k, line (theta column) t
-template <int MAG>
-__device__ __forceinline__ void thph_phi_solve(const CssGeo &g, const double *F, double *O, const ThphTile &T, int k,
+// [6 dbt 7 dbr]) into O + k0 + k, line (theta column) t, block bp at row R0 of
+// the tile, whose last row is len - 1
+template <int MAG, int M, int R0>
+__device__ __forceinline__ void thph_phi_solve(const CssGeo &g, const double *F, double *O, int bp, int len, int k,
                                                int k0, int t) {
   const int f = k == 0 ? 0 : k == 1 ? 2 : k == 2 ? 1 : k == 3 ? 3 : k <= 5 ? 4 : (k == 6 ? 5 : 7);
-  const double dn = g.d[2].dnum[T.bp];
+  const double dn = g.d[2].dnum[bp];
   const double *x = F + thph_foff(MAG, f);
+  const PhIdx<M, R0> xi{t, len};
   if (k == 5) {
     if (g.slaplacian)
-      line_solve_c<2, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 2, 0), g.tstride, dn, dn * dn, 1,
-                          O + (k0 + k) * FA_OUT, SwzCol{t});
+      line_solve_c<2, M>(x, xi, 3, 0, 0.0, 0.0, tabp(g, 2, bp, 2, 0), g.tstride, dn, dn * dn, 1,
+                         O + (k0 + k) * FA_OUT, SwzCol{t, R0});
   } else {
-    line_solve_c<1, FM>(x, PhIdx{t}, 3, 0, 0.0, 0.0, tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1,
-                        O + (k0 + k) * FA_OUT, SwzCol{t});
+    line_solve_c<1, M>(x, xi, 3, 0, 0.0, 0.0, tabp(g, 2, bp, 1, 0), g.tstride, dn, dn, 1, O + (k0 + k) * FA_OUT,
+                       SwzCol{t, R0});
   }
 }
 
 // d(rho)/dtheta with a zero wall datum on a theta-wall block (bdry ibct(1)),
-// line p, into rtw (k_rstage adds the datum times the unit response)
-__device__ __forceinline__ void thph_wall_rho(const CssGeo &g, const double *F, const ThphTile &T, int p,
+// line p, into rtw (the stage pass adds the datum times the unit response)
+template <int M, int C0>
+__device__ __forceinline__ void thph_wall_rho(const CssGeo &g, const double *F, const ThphTile &T, int bt, int p,
                                               double *__restrict__ rtw) {
   const CssDir &DT = g.d[1];
-  const int bdry = g.ibct[1], side = DT.lphys[T.bt] ? 0 : 1;
-  const double dn = DT.dnum[T.bt];
+  const int bdry = g.ibct[1], side = DT.lphys[bt] ? 0 : 1;
+  const double dn = DT.dnum[bt];
   double *o = rtw + (((size_t)T.ir * g.nphi + T.p0 + p) * 2 + side) * FM;
-  line_solve_c<1, FM>(F + p * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0, 0.0, tabp(g, 1, T.bt, 1, bdry),
-                      g.tstride, dn, dn, 0, o, StridedOut{1});
+  line_solve_c<1, M>(F + p * FA_RW + C0, ThIdx{}, dtype_of(DT, bt), bdry, 0.0, 0.0, tabp(g, 1, bt, 1, bdry),
+                     g.tstride, dn, dn, 0, o, StridedOut{1});
 }
 
-template <int MAG>
-__global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restrict__ cur,
-                                                 const double *__restrict__ bf, double *__restrict__ dv,
-                                                 double *__restrict__ tbuf, double *__restrict__ rtw,
-                                                 const __grid_constant__ PlaneMaps mc,
+// theta derivative k of every block of the tile's row p; the last one is
+// d(rho)/dtheta, which goes to rtw on a wall block
+template <int MAG, int BT>
+__device__ __forceinline__ void thph_theta_row(const CssGeo &g, const double *F, double *O, const ThphTile &T, int k,
+                                               int p, int lenp, double *rtw) {
+  const CssDir &DT = g.d[1];
+  const bool isrho = k == (MAG ? 7 : 5);
+  auto one = [&](auto c0, int bt) {
+    constexpr int C0 = decltype(c0)::value;
+    if (isrho && (DT.lphys[bt] || DT.rphys[bt])) {
+      if (p < lenp) thph_wall_rho<BT, C0>(g, F, T, bt, p, rtw);
+    } else {
+      thph_theta_solve<MAG, BT, C0>(g, F, O, bt, T.ir, k, p);
+    }
+  };
+  one(std::integral_constant<int, 0>{}, T.bt);
+  if constexpr (BT < FM)
+    if (T.bt + 1 < DT.nb) one(std::integral_constant<int, BT>{}, T.bt + 1);
+}
+
+// TS: storage of the stage states; BT, BP: theta and phi block lengths (16 or
+// 32, every block of a direction the same)
+template <int MAG, typename TS, int BT, int BP>
+__global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, double *__restrict__ dv, double *__restrict__ tbuf,
+                                                 double *__restrict__ rtw, const __grid_constant__ PlaneMaps mc,
                                                  const __grid_constant__ PlaneMaps mb, int *flag) {
-  using C = ThphCfg<MAG>;
+  using C = ThphCfg<MAG, TS>;
   constexpr int NA = MAG ? 8 : 5;
   // plane buffers (128-byte aligned boxes: a field is 12800 bytes), the
   // derivative tiles, the buffers' mbarriers
@@ -297,16 +384,16 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
   uint64_t *bar = reinterpret_cast<uint64_t *>(O + (size_t)C::NO * FA_OUT);
   const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5;
   const size_t n = (size_t)g.ncell;
-  const int ntile = g.nr * g.d[1].nb * g.d[2].nb;
+  const int ntile = thph_tiles<BT, BP>(g);
   if (tid == 0) {
     for (int b = 0; b < C::NBUF; b++) mbar_init(bar + b, 1);
     mbar_fence_init();
   }
   __syncthreads();
   if (C::NBUF == 2 && tid == 0 && (int)blockIdx.x < ntile)
-    thph_stage_tma<C::NF>(g, mc, mb, thph_tile(g, blockIdx.x), sm, bar);
+    thph_stage_tma<C::NF, TS>(g, mc, mb, thph_tile<BT, BP>(g, blockIdx.x), sm, bar);
   for (int q = blockIdx.x, i = 0; q < ntile; q += gridDim.x, i++) {
-    const ThphTile T = thph_tile(g, q);
+    const ThphTile T = thph_tile<BT, BP>(g, q);
     const int b = C::NBUF == 2 ? (i & 1) : 0;
     double *F = sm + (size_t)b * C::PLANE;
     const bool more = q + (int)gridDim.x < ntile;
@@ -315,7 +402,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
       // barrier that ended the previous tile
       if (more && tid == 0) {
         fence_proxy_async();
-        thph_stage_tma<C::NF>(g, mc, mb, thph_tile(g, q + gridDim.x), sm + (size_t)(b ^ 1) * C::PLANE,
+        thph_stage_tma<C::NF, TS>(g, mc, mb, thph_tile<BT, BP>(g, q + gridDim.x), sm + (size_t)(b ^ 1) * C::PLANE,
                               bar + (b ^ 1));
       }
     } else if (tid == 0 && i == 0) {
@@ -324,7 +411,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
       // registers (bringing the next tile's lines toward L2 instead, as an
       // earlier form did, cost 11.6 against 9.8 ms a launch)
       fence_proxy_async();
-      thph_stage_tma<C::NF>(g, mc, mb, T, F, bar);
+      thph_stage_tma<C::NF, TS>(g, mc, mb, T, F, bar);
     }
     // this plane's copies: buffer b's (i >> 1)-th use (every use for MHD)
     const unsigned parity = C::NBUF == 2 ? ((unsigned)(i >> 1) & 1u) : ((unsigned)i & 1u);
@@ -339,9 +426,14 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
       }
       return;
     }
-    const CssDir &DT = g.d[1];
-    const bool wall = DT.lphys[T.bt] || DT.rphys[T.bt];
     const int ir = T.ir, it = T.t0 + lane;
+    // rows of the tile, and what of it this lane and the walls take (all of
+    // it with 32-point blocks)
+    const int lenp = BP == FM || T.p0 + FM <= g.nphi ? FM : BP;
+    const bool tin = BT == FM || it < g.nth;
+    const bool wall = BT == FM ? g.d[1].lphys[T.bt] || g.d[1].rphys[T.bt] : it < BT || it >= g.nth - BT;
+    const int itc = BT == FM ? it : min(it, g.nth - 1);
+    if constexpr (sizeof(TS) == 4) thph_widen(g, T, F);
     // ---- T, 1/rho and 1/(rho T) of this thread's two points (rows wrp,
     // wrp + 16, theta t0 + lane), T also to tbuf ----
     double tq[2], rq[2], rtq[2];
@@ -356,18 +448,20 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
         rtq[h] = rq[h] / tq[h];
       }
 #pragma unroll
-      for (int h = 0; h < 2; h++) tbuf[pl + (size_t)(T.p0 + wrp + 16 * h) * g.nth + it] = tq[h];
+      for (int h = 0; h < 2; h++)
+        if (tin && (BP == FM || wrp + 16 * h < lenp)) tbuf[pl + (size_t)(T.p0 + wrp + 16 * h) * g.nth + it] = tq[h];
     }
     // ---- solves: theta (warps 0-5 hydro, 0-7 MHD), phi (warps 6-11 hydro,
     // 8-15 MHD), all at once ----
     {
-      const int nth_t = (MAG ? 7 : 5) + (wall ? 0 : 1);
       const int nthw = MAG ? 8 : 6;  // theta warps; the last one solves d(rho)/dtheta
       if (wrp < nthw) {
-        if (wrp < nth_t) thph_theta_solve<MAG>(g, F, O, T, wrp, lane);
-        else thph_wall_rho(g, F, T, lane, rtw);
+        thph_theta_row<MAG, BT>(g, F, O, T, wrp, lane, lenp, rtw);
       } else if (wrp < (MAG ? 16 : 12)) {
-        thph_phi_solve<MAG>(g, F, O, T, wrp - nthw, C::PHI0, lane);
+        thph_phi_solve<MAG, BP, 0>(g, F, O, T.bp, lenp, wrp - nthw, C::PHI0, lane);
+        if constexpr (BP < FM)
+          if (T.bp + 1 < g.d[2].nb)
+            thph_phi_solve<MAG, BP, BP>(g, F, O, T.bp + 1, lenp, wrp - nthw, C::PHI0, lane);
       }
     }
     __syncthreads();
@@ -385,7 +479,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
       __syncthreads();
       if (more && tid == 0) {
         fence_proxy_async();
-        thph_stage_tma<C::NF>(g, mc, mb, thph_tile(g, q + gridDim.x), F, bar);
+        thph_stage_tma<C::NF, TS>(g, mc, mb, thph_tile<BT, BP>(g, q + gridDim.x), F, bar);
       }
     }
     // ---- theta pointwise (Source_Theta_Terms, Lorentz, induction, and
@@ -395,7 +489,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
     {
       const double rv = g.r_ind[ir], epsr = g.eps[ir];
       const double omsq = rv * g.omega0 * g.omega0, om2 = 2.0 * g.omega0;
-      const double sn = g.sines[it], cs = g.cosines[it], ct = g.cot[it];
+      const double sn = g.sines[itc], cs = g.cosines[itc], ct = g.cot[itc];
       const int dtt = MAG ? 7 : 5;  // tile of d(rho)/dtheta
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -463,7 +557,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
     }
     // ---- phi pointwise (Phi_Terms + Lorentz), then the stores ----
     {
-      const double oors = ri * g.csc[it];
+      const double oors = ri * g.csc[itc];
       const double *OP = O + C::PHI0 * FA_OUT;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -504,6 +598,7 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, const double *__restr
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const size_t id = pl + (size_t)(T.p0 + wrp + 16 * h) * g.nth + it;
+        if (!tin || (BP < FM && wrp + 16 * h >= lenp)) continue;
 #pragma unroll
         for (int f = 0; f < NA; f++) dv[f * n + id] = acc[h][f];
       }
@@ -564,9 +659,9 @@ __global__ void __launch_bounds__(NTH, NBUF == 2 ? 2 : 3) k_curl_pl(CssGeo g, do
     mbar_fence_init();
   }
   __syncthreads();
-  if (NBUF == 2 && tid == 0 && (int)blockIdx.x < ntile) curl_stage_tma(g, m, thph_tile(g, blockIdx.x), sm, bar);
+  if (NBUF == 2 && tid == 0 && (int)blockIdx.x < ntile) curl_stage_tma(g, m, thph_tile<FM, FM>(g, blockIdx.x), sm, bar);
   for (int q = blockIdx.x, i = 0; q < ntile; q += gridDim.x, i++) {
-    const ThphTile T = thph_tile(g, q);
+    const ThphTile T = thph_tile<FM, FM>(g, q);
     const int b = NBUF == 2 ? (i & 1) : 0;
     double *F = sm + (size_t)b * C::NF * FA_FIELD;
     const bool more = q + (int)gridDim.x < ntile;
@@ -575,7 +670,7 @@ __global__ void __launch_bounds__(NTH, NBUF == 2 ? 2 : 3) k_curl_pl(CssGeo g, do
       // barrier that ended the previous tile
       if (more && tid == 0) {
         fence_proxy_async();
-        curl_stage_tma(g, m, thph_tile(g, q + gridDim.x), sm + (size_t)(b ^ 1) * C::NF * FA_FIELD, bar + (b ^ 1));
+        curl_stage_tma(g, m, thph_tile<FM, FM>(g, q + gridDim.x), sm + (size_t)(b ^ 1) * C::NF * FA_FIELD, bar + (b ^ 1));
       }
     } else if (tid == 0 && i == 0) {
       // the first tile's planes; each later tile's copies start once the
@@ -606,11 +701,11 @@ __global__ void __launch_bounds__(NTH, NBUF == 2 ? 2 : 3) k_curl_pl(CssGeo g, do
         const int bdry = g.ibct[wrp == 0 ? 11 : 12];
         const double dn = DT.dnum[T.bt];
         line_solve_c<1, FM>(F + (size_t)(1 + wrp) * FA_FIELD + lane * FA_RW, ThIdx{}, dtype_of(DT, T.bt), bdry, 0.0,
-                            0.0, tabp(g, 1, T.bt, 1, bdry), g.tstride, dn, dn, 0, O + wrp * FA_OUT, SwzRow{lane});
+                            0.0, tabp(g, 1, T.bt, 1, bdry), g.tstride, dn, dn, 0, O + wrp * FA_OUT, SwzRow{lane, 0});
       } else {  // phi lines (line = theta column t = lane): A_r, A_theta
         const double dn = g.d[2].dnum[T.bp];
-        line_solve_c<1, FM>(F + (size_t)(wrp == 2 ? 2 : 0) * FA_FIELD, PhIdx{lane}, 3, 0, 0.0, 0.0,
-                            tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1, O + wrp * FA_OUT, SwzCol{lane});
+        line_solve_c<1, FM>(F + (size_t)(wrp == 2 ? 2 : 0) * FA_FIELD, PhIdx<FM, 0>{lane, FM}, 3, 0, 0.0, 0.0,
+                            tabp(g, 2, T.bp, 1, 0), g.tstride, dn, dn, 1, O + wrp * FA_OUT, SwzCol{lane, 0});
       }
     }
     __syncthreads();
@@ -618,7 +713,7 @@ __global__ void __launch_bounds__(NTH, NBUF == 2 ? 2 : 3) k_curl_pl(CssGeo g, do
     // tile's planes arrive under them
     if (NBUF == 1 && more && tid == 0) {
       fence_proxy_async();
-      curl_stage_tma(g, m, thph_tile(g, q + gridDim.x), F, bar);
+      curl_stage_tma(g, m, thph_tile<FM, FM>(g, q + gridDim.x), F, bar);
     }
     const double invr = g.r_inv[T.ir];
     const size_t pl = plane(g, T.ir);
@@ -872,12 +967,12 @@ __global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssG
     // ---- radial solves: tile k = warp, line = lane ----
     const int dtype = dtype_of(D, T.br);
     if (wrp < C::ND) {
-      const int var[8] = {2, 3, 4, 5, 5, 1, 7, 8};
       const int k = wrp, l = lane;
+      const int var = (0x87155432u >> (4 * k)) & 15;  // field whose closure derivative k takes: 2 3 4 5 5 1 7 8
       if (!(k == 4 && !g.slaplacian)) {
         const int hk = (k <= 3) ? k : (k == 4 ? 3 : (k == 5 ? 4 : k - 1));
         const double *x = H + (size_t)hk * FB_FIELD + 4 * FM + l;
-        const int bdry = g.ibcr[var[k]];
+        const int bdry = g.ibcr[var];
         double lo = 0.0, hi = 0.0;
         if (k == 0 || k == 1) {  // stress-free datum w/r/dxdr (rhs_mpi.f90:578-614)
           if (D.lphys[T.br] && g.bottom_stress_free) lo = x[0] / g.r1 / g.dxdr[0];

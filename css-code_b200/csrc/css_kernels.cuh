@@ -706,15 +706,15 @@ __device__ __forceinline__ void radial_point(const CssGeo &g, int ir, const RadI
 }
 
 // The face-plane relaxation of an open radial boundary at one point of the
-// radial tile: hl is the point's row of the tile (w, v, u, s at 0..3 HS),
-// q its plane index.  Top: rhs_mpi.f90:2042-2066; bottom: :1913-1952.
-__device__ __forceinline__ void inout_face(const CssGeo &g, int j, int m, bool top, const double *hl, int SR,
-                                           size_t HS, size_t q, double &drho, double &dw, double &dvv, double &du,
-                                           double &ds) {
+// radial tile: at(f, d) is field f (0 w, 1 v, 2 u, 3 s) d rows above the
+// point, q its plane index.  Top: rhs_mpi.f90:2042-2066; bottom: :1913-1952.
+template <class AT>
+__device__ __forceinline__ void inout_face(const CssGeo &g, int j, int m, bool top, const AT &at, size_t q,
+                                           double &drho, double &dvv, double &du, double &ds) {
   const double *io = g.inout;
   if (top) {
     if (j != m - 1) return;
-    const double ut = hl[2 * HS], st = hl[3 * HS], ub = hl[2 * HS - SR], sb = hl[3 * HS - SR];
+    const double ut = at(2, 0), st = at(3, 0), ub = at(2, -1), sb = at(3, -1);
     if (g.rain) {
       const double taur = io[IO_TOP_TAUR];
       du = du + (io[IO_TOP_MDVEL] + g.dvel_rain[q] + ub - 2.0 * ut) * taur + io[IO_TOP_MEANU];
@@ -727,18 +727,18 @@ __device__ __forceinline__ void inout_face(const CssGeo &g, int j, int m, bool t
     return;
   }
   if (j != 0) return;
-  const double u0 = hl[2 * HS], s0 = hl[3 * HS], tau = io[IO_BOT_TAU];
+  const double u0 = at(2, 0), s0 = at(3, 0), tau = io[IO_BOT_TAU];
   if (g.bottom_specified) {
     const size_t np = (size_t)g.nth * g.nphi;
     const double tc = io[IO_BOT_TCONST];
     drho = drho + io[IO_BOT_MEANU];
     // the u_theta term is added in k_rhot_update, after Density_Terms_Theta
     // has read the accumulated dw for its wall datum (rhs_mpi.f90:705, :724)
-    dvv = dvv + tau * (tc * g.ashv[2 * np + q] - hl[HS]);
+    dvv = dvv + tau * (tc * g.ashv[2 * np + q] - at(1, 0));
     du = du + tau * (tc * g.ashv[q] - u0);
     ds = ds + tau * ((g.sr[0] + io[IO_BOT_FEN] * g.ashv[3 * np + q]) - s0);
   } else {
-    const double ua = hl[2 * HS + SR], sa = hl[3 * HS + SR];
+    const double ua = at(2, 1), sa = at(3, 1);
     drho = drho + io[IO_BOT_TCONST];
     du = du + tau * (io[IO_BOT_NRAT] * ua - u0) + io[IO_BOT_MEANU];
     ds = ds + tau * (sa - s0 + io[IO_BOT_MEANS]);
@@ -917,7 +917,8 @@ __device__ __forceinline__ void radial_tile(const CssGeo &g, const TV *__restric
         drho = drho - q.u * w1;
         if (top_open) du = du - g.pconst * q.t * (1.0 / q.rho) * w1;
         else du = du - g.pconst * q.t * w1 * (1.0 / q.rho);
-        inout_face(g, j, m, top_open, hl, SR, HS, base + l, drho, dw, dvv, du, ds);
+        inout_face(g, j, m, top_open, [&](int f, int d) { return hl[(size_t)f * HS + (long long)d * SR]; }, base + l,
+                   drho, dvv, du, ds);
       } else {
         if (g.non_uniform) w1 = w1 * g.dxdr[ir];
         drho = drho - q.u * w1;
@@ -1508,9 +1509,7 @@ __global__ void k_sld_vcc(CssGeo g, const double *__restrict__ v, const double *
 // limited value is 0 (opposite signs), q (|qph| >= |q|) or qph: a minmod,
 // evaluated without the division (equal to the reference's product to within
 // its roundings); below tiny the formula as written, k = qph / tiny^2 in
-// hand.  Selections only: lanes on either side of tiny do not diverge (with
-// the branch, 2.10 -> 1.74 ms a launch on 128x256x512; FP64 work did not
-// change, the branch's re-convergence and the second product did).
+// hand.  Selections only: lanes on either side of tiny do not diverge.
 __device__ __forceinline__ double sld_limiter(double q, double qph, double k, double tiny) {
   const double kq = q * k;
   const bool big = fabs(q) >= tiny;

@@ -1,0 +1,81 @@
+"""The general two-pass stage (plane pass over 16- and 32-point blocks, stage
+pass for any radial block) against the four-kernel stage of the same run,
+which tests/test_variants.py, test_inout.py, test_laplacian.py and
+test_mixed.py hold to the oracle.  Cases: both block lengths in either
+direction, tiles left half empty by an odd number of 16-point blocks, radial
+blocks of 10 to 64 points, open faces, explicit viscosity, the TVD schemes and
+FP32 stage states.
+
+Two steps each.  Only the order in which the density-theta term joins the sums
+differs, a rounding; FP64 runs are held to 1e-12 of each field's largest
+magnitude (tests/test_fused.py's bar).  An FP32 stage state can round the
+other way (2^-24 of a perturbation) where the FP64 value lands on a rounding
+boundary: 1e-7 of each field's largest magnitude."""
+import numpy as np
+import pytest
+
+from css_b200 import problem
+from css_b200.context import Simulation
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "hydro-16x16": dict(dims=(40, 48, 80), decomp=(2, 3, 5)),
+    "hydro-16x32": dict(dims=(60, 48, 96), decomp=(3, 3, 3)),
+    "hydro-32x16": dict(dims=(24, 64, 80), decomp=(2, 2, 5)),
+    "hydro-r10": dict(dims=(20, 32, 48), decomp=(2, 2, 3)),
+    "hydro-r64": dict(dims=(128, 64, 96), decomp=(2, 2, 3)),
+    "hydro-noslip": dict(dims=(40, 48, 48), decomp=(2, 3, 3), top_stress_free=0, bottom_stress_free=0,
+                         theta_stress_free=0, mass_diffusion=0, xi_cs=0.9),
+    "mhd-16x16": dict(dims=(40, 48, 80), decomp=(2, 3, 5), magnetic=True),
+    "mhd-32x16": dict(dims=(60, 64, 48), decomp=(3, 2, 3), magnetic=True),
+    "mhd-16x32": dict(dims=(104, 32, 96), decomp=(2, 2, 3), magnetic=True),
+    "mhd-conductor": dict(dims=(40, 48, 48), decomp=(2, 3, 3), magnetic=True, theta_perf_conductor=1,
+                          theta_normal_field=0, top_radial_field=0, bottom_radial_field=0, top_perfect_cond=1,
+                          bottom_perfect_cond=1),
+    "open-both": dict(dims=(64, 64, 96), decomp=(2, 2, 3), top_inout=1, bot_inout=1),
+    "open-rain-16": dict(dims=(40, 48, 48), decomp=(2, 3, 3), top_inout=1, do_entropy_rain=1, delta_s=1e-4),
+    "viscous-mhd": dict(dims=(64, 64, 96), decomp=(2, 2, 3), magnetic=True, laplacian=1),
+    "viscous-16": dict(dims=(40, 48, 48), decomp=(2, 3, 3), laplacian=1),
+    "rk2": dict(dims=(40, 48, 48), decomp=(2, 3, 3), time_stepper=2),
+    "rk3-32": dict(dims=(64, 64, 96), decomp=(2, 2, 3), time_stepper=3),
+    "mixed-32": dict(dims=(64, 64, 96), decomp=(2, 2, 3), precision=1),
+    "mixed-16": dict(dims=(40, 48, 80), decomp=(2, 3, 5), precision=1),
+    "mixed-mhd-32": dict(dims=(64, 64, 96), decomp=(2, 2, 3), magnetic=True, precision=1),
+    "mixed-mhd-16x32": dict(dims=(60, 48, 96), decomp=(3, 3, 3), magnetic=True, precision=1),
+    "mixed-rk3": dict(dims=(40, 48, 48), decomp=(2, 3, 3), precision=1, time_stepper=3),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_general_stage_equals_four_kernels(name, gpu_available):
+    kw = dict(CASES[name])
+    p, prof, v0, dt, _ = problem.build(kw.pop("dims"), decomp=kw.pop("decomp"), magnetic=kw.pop("magnetic", False))
+    for k, val in kw.items():
+        setattr(p, k, val)
+    rng = np.random.default_rng(8)
+    v0 = v0.copy()
+    v0[1:4] = 1e-3 * rng.standard_normal(v0[1:4].shape)
+    if p.laplacian:
+        dt = 0.1 * dt
+    out = []
+    for four in (False, True):
+        sim = Simulation(p, prof)
+        if four:
+            sim.set_fused(False)
+        sim.upload(v0)
+        if p.top_inout or p.bot_inout:
+            sim.inout_init()
+            sim.set_clock(0, 0.0, dt)
+            if p.do_entropy_rain:
+                sim.set_rain_fields(*(1e-3 * rng.standard_normal((2, p.nphi, p.nth)) if not out else rain))
+            rain = sim.rain_fields()
+        n0 = sim.launches()
+        sim.step_rk4(dt, 2)
+        out.append((sim.download(), sim.launches() - n0))
+        sim.close()
+    (two, n2), (four_, n4) = out
+    assert n2 < n4  # the two forms did run
+    bar = 1e-7 if p.precision else 1e-12
+    for i in range(two.shape[0]):
+        assert np.abs(two[i] - four_[i]).max() <= bar * np.abs(four_[i]).max(), (name, i)
