@@ -32,17 +32,6 @@ __device__ __forceinline__ double io_block_sum(double x, double *sh) {
   __syncthreads();
   return r;
 }
-__device__ __forceinline__ double io_block_min(double x, double *sh) {
-  sh[threadIdx.x] = x;
-  __syncthreads();
-  for (int s = IO_NT / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) sh[threadIdx.x] = fmin(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
-  double r = sh[0];
-  __syncthreads();
-  return r;
-}
 
 // One CTA per (theta block, phi block) of the open faces.  part[8*b + k]:
 // top 0 sum u rho sin, 1 sum rho sin, 2 sum s, 3 sum rho sin (dvel_rain +
@@ -51,7 +40,7 @@ __device__ __forceinline__ double io_block_min(double x, double *sh) {
 // them; mynr is the bottom block's own top radius).
 __global__ void __launch_bounds__(IO_NT) k_inout_sums(CssGeo g, const double *__restrict__ v,
                                                       double *__restrict__ part) {
-  __shared__ double sh[IO_NT];
+  __shared__ double sh[8][IO_NT];
   const int jb = blockIdx.x / g.d[2].nb, kb = blockIdx.x - jb * g.d[2].nb;
   const int t0 = g.d[1].start[jb], nt = g.d[1].size[jb], p0 = g.d[2].start[kb], np_ = g.d[2].size[kb];
   const size_t n = (size_t)g.ncell;
@@ -81,25 +70,38 @@ __global__ void __launch_bounds__(IO_NT) k_inout_sums(CssGeo g, const double *__
       umin = fmin(umin, v[3 * n + css_idx(g, it, ip, 1)]);
     }
   }
-  for (int k = 0; k < 7; k++) a[k] = io_block_sum(a[k], sh);
-  umin = io_block_min(umin, sh);
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 7; k++) part[8 * blockIdx.x + k] = a[k];
-    part[8 * blockIdx.x + 7] = fabs(umin);
+  // the eight reductions together, each in io_block_sum's tree order (one
+  // after another, at nine barriers each: 13 against 11 us a launch)
+  for (int k = 0; k < 7; k++) sh[k][threadIdx.x] = a[k];
+  sh[7][threadIdx.x] = umin;
+  __syncthreads();
+  for (int s = IO_NT / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) {
+      for (int k = 0; k < 7; k++) sh[k][threadIdx.x] = sh[k][threadIdx.x] + sh[k][threadIdx.x + s];
+      sh[7][threadIdx.x] = fmin(sh[7][threadIdx.x], sh[7][threadIdx.x + s]);
+    }
+    __syncthreads();
   }
+  if (threadIdx.x < 8) part[8 * blockIdx.x + threadIdx.x] = threadIdx.x < 7 ? sh[threadIdx.x][0] : fabs(sh[7][0]);
 }
 
-// The face scalars of this RHS from the block parts (one thread; at most
+// The face scalars of this RHS from the block parts (one warp; at most
 // CSS_MAXBLK^2 parts).  Every formula follows the reference line cited.
 __global__ void k_inout_scalars(CssGeo g, const double *__restrict__ part, double *io, double deltat,
                                 double sim_time) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int nb = g.d[1].nb * g.d[2].nb, nr = g.nr;
-  double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  // one warp: lane k adds sum k over the blocks, in block order (one thread
+  // for the eight sums: 12.5 us a launch, now 9.5 us on 4 x 8 blocks)
+  const int nb = g.d[1].nb * g.d[2].nb, nr = g.nr, lane = threadIdx.x;
+  double acc = 0.0;
+#pragma unroll 8
   for (int b = 0; b < nb; b++) {
-    for (int k = 0; k < 7; k++) s[k] = s[k] + part[8 * b + k];
-    s[7] = fmax(s[7], part[8 * b + 7]);  // 'csm': the last entry is a max (mhdsph_mpi.f90:1511-1521)
+    const double x = __ldg(part + 8 * b + (lane & 7));
+    acc = (lane & 7) < 7 ? acc + x : fmax(acc, x);  // 'csm': the last entry is a max (mhdsph_mpi.f90:1511-1521)
   }
+  double s[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) s[k] = __shfl_sync(0xffffffffu, acc, k);
+  if (lane != 0) return;
   const double ntot = (double)g.nth * (double)g.nphi;
   const double c_top = sqrt(g.gamm1 * g.cp * g.t0);  // sqrt(gamm1 Cp Tr(nr)), Tr(nr) = T0 (mhdsph_mpi.f90:343)
   if (g.top_inout) {  // rhs_mpi.f90:2003-2017, :1982
