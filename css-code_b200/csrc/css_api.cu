@@ -958,7 +958,7 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   // any radial block whose slab fits shared memory, either storage of the
   // stage states, any stepper, open radial faces and explicit viscosity; radiative
   // diffusion alone sits between the radial terms and the update
-  c->two = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, 8) <= SG_SMEM && !p.do_radheat;
+  c->two = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, p.precision ? 4 : 8) <= SG_SMEM && !p.do_radheat;
   if (c->two) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
   if (p.precision == 1) {  // backgrounds of the FP32 stage states, refreshed at every upload
     ALLOC(c->bg2, 2 * (size_t)nr * nth * sizeof(double));
@@ -1238,7 +1238,10 @@ static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double
 template <typename TS, typename TO>
 static int launch_rhs(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, double ca = 0.0, double cb = 0.0,
                       double dsld = 0.0, bool with_sld = false) {
-  if (stage > 0 && c->two) return launch_stage_two(c, cur, nx, stage, dtcur, ca, cb, dsld, with_sld);
+  // (the FP64 first stage of a mixed run can have a slab too large for it where
+  // the FP32 ones fit)
+  if (stage > 0 && c->two && stage_smem(c->g.magnetic, c->g.d[0].maxm, (int)sizeof(TS)) <= SG_SMEM)
+    return launch_stage_two(c, cur, nx, stage, dtcur, ca, cb, dsld, with_sld);
   const CssGeo &g = c->g;
   const int mag = g.magnetic;
   if (mag) {
