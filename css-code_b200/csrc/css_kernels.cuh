@@ -1706,13 +1706,20 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
   const int itc = min(it, nth - 1), ipc = min(ip, nphi - 1);
   // this launch diffuses fields off .. off+NF-1 and writes the fields of
   // wmask (a field it writes but does not diffuse gets zero)
+  const int lo_item = (int)threadIdx.x - 32 * NF;
+  const bool lo_p = ty < NF, lo_t = lo_item >= 0 && lo_item < NF * SLD_TP;
+  const int lo_f = lo_p ? ty : (lo_t ? lo_item / SLD_TP : 0), lo_row = lo_t ? lo_item % SLD_TP : 0;
+  const double lo_tiny = g.tinyvar[lo_f + off], lo_itiny = g.inv_tinyvar2[lo_f + off];
   const bool hydro_part = (wmask & 0x1Fu) != 0;  // the fields the corrections act on
   const bool edge_lo = t0 == 0, edge_hi = t0 + SLD_TT >= nth;
-  // theta faces of this thread: the upper face of its cell, and for warp 1
-  // the lower face of row tx (lane < SLD_TP); their sin(face) factors
+  // theta faces of this thread: the upper face of its cell; their sin(face) factors
   const int gt_hi = t0 + tx + 1;
   const bool th_hi_in = gt_hi > 0 && gt_hi < nth;
-  const bool lo_t = ty == 1 && tx < SLD_TP, lo_p = ty == 0;
+  // the tile's lower faces, shared out over the warps: warp f < NF takes field
+  // f's 32 phi faces of row 0, the next warps the theta faces of column 0, a
+  // lane per (field, row).  On warps 0 and 1
+  // alone the other six waited at the barrier for half again their own work:
+  // 1.77 against 1.69 ms on 128x256x512, 517 against 493 us on MHD 128x128x256.
   const bool th_lo_in = t0 > 0 && t0 < nth;
   const SldCopy cp = sld_copy_plan(g, t0, p0);
   // per-field r window: x(ir-1), x(ir), x(ir+1), x(ir+2), and the de of the
@@ -1793,15 +1800,10 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
     const double st_hi =
         th_hi_in ? (g.sld_coef * sqrt(0.5 * (V[ty + 1][tx + 2] + V[ty + 1][tx + 1]))) * __ldg(g.sld_th + gt_hi) : 0.0;
     const double sp_hi = g.sld_coef * sqrt(0.5 * (V[ty + 1][tx + 1] + V[ty + 2][tx + 1]));
-    double s_lo = 0.0;
-    if (lo_p) s_lo = g.sld_coef * sqrt(0.5 * (V[0][tx + 1] + V[1][tx + 1]));
-    else if (lo_t && th_lo_in) s_lo = (g.sld_coef * sqrt(0.5 * (V[tx + 1][1] + V[tx + 1][0]))) * __ldg(g.sld_th + t0);
     // face fluxes of every field: each thread takes the upper theta face and
-    // the upper phi face of its cell; warp 0 also the phi faces of row 0,
-    // warp 1 the theta faces of column 0.  Unrolled over the fields: their
-    // limiter chains are independent, and with every field index static the
-    // longer code no longer costs instruction-cache stalls (2.21 -> 2.03 ms
-    // on 128x256x512)
+    // the upper phi face of its cell.  Unrolled over the fields: their limiter
+    // chains are independent, and with every field index static the longer
+    // code does not cost instruction-cache stalls
 #pragma unroll
     for (int f = 0; f < NF; f++) {
       const double tiny = g.tinyvar[f + off], itiny = g.inv_tinyvar2[f + off];
@@ -1809,12 +1811,18 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
       FT[f][ty][tx + 1] = th_hi_in ? st_hi * sld_face(xr[0], xr[1], xr[2], xr[3], tiny, itiny) : 0.0;
       FP[f][ty + 1][tx] = sp_hi * sld_face(X[f][ty + 1][tx + 2], X[f][ty + 2][tx + 2], X[f][ty + 3][tx + 2],
                                            X[f][ty + 4][tx + 2], tiny, itiny);
-      if (lo_p) {
-        FP[f][0][tx] = s_lo * sld_face(X[f][0][tx + 2], X[f][1][tx + 2], X[f][2][tx + 2], X[f][3][tx + 2], tiny, itiny);
-      } else if (lo_t) {
-        const double *xl = &X[f][tx + 2][0];
-        FT[f][tx][0] = th_lo_in ? s_lo * sld_face(xl[0], xl[1], xl[2], xl[3], tiny, itiny) : 0.0;
-      }
+    }
+    if (lo_p) {
+      const double s_lo = g.sld_coef * sqrt(0.5 * (V[0][tx + 1] + V[1][tx + 1]));
+      FP[lo_f][0][tx] = s_lo * sld_face(X[lo_f][0][tx + 2], X[lo_f][1][tx + 2], X[lo_f][2][tx + 2],
+                                        X[lo_f][3][tx + 2], lo_tiny, lo_itiny);
+    } else if (lo_t) {
+      const double *xl = &X[lo_f][lo_row + 2][0];
+      double d = 0.0;
+      if (th_lo_in)
+        d = (g.sld_coef * sqrt(0.5 * (V[lo_row + 1][1] + V[lo_row + 1][0]))) * __ldg(g.sld_th + t0) *
+            sld_face(xl[0], xl[1], xl[2], xl[3], lo_tiny, lo_itiny);
+      FT[lo_f][lo_row][0] = d;
     }
     // the velocities of this cell, taken from the tile when they are diffused
     // fields (before the barrier: the next radius's copies reuse the buffer)
