@@ -321,8 +321,10 @@ static int setup_mt() {
   CSS_SMEM_ATTR(k_curl_theta<MT, TLC, float>);
   CSS_SMEM_ATTR(k_curl_phi<MT, TLC, double>);
   CSS_SMEM_ATTR(k_curl_phi<MT, TLC, float>);
-  CSS_SMEM_ATTR(k_curl_r<MT, TLC, double>);
-  CSS_SMEM_ATTR(k_curl_r<MT, TLC, float>);
+  if constexpr (MT > 0 && TLC > 0) {
+    CSS_SMEM_ATTR(k_curl_r<MT, TLC, double>);
+    CSS_SMEM_ATTR(k_curl_r<MT, TLC, float>);
+  }
   if constexpr (MT > 0 && TLC > 0) CSS_SMEM_ATTR(k_phi_terms_p<MT, TLC>);
 #undef CSS_SMEM_ATTR
   return CSS_OK;
@@ -395,6 +397,8 @@ static int setup_kernels() {
   CSS_LINE_ATTR(k_adj_s<0, 2, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 1, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 2, 0>);
+  CSS_LINE_ATTR(k_curl_rg<double>);
+  CSS_LINE_ATTR(k_curl_rg<float>);
   CSS_LINE_ATTR(k_adj_t<1, 0>);
   CSS_LINE_ATTR(k_adj_t<2, 0>);
 #undef CSS_LINE_ATTR
@@ -1045,13 +1049,27 @@ static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
   TL = c->tl_r;
   dim3 gr(g.d[0].nb * ((g.nth + TL - 1) / TL), g.nphi);
   prof_begin(c, KI_CURL_R);
-  LAUNCH_MT(0, TL, k_curl_r, (TS), gr, smem_line(2, 2, 0, mr, TL), g, a, out, TL, apply_bc);
+  switch (c->mt[0] * 100 + TL) {
+    case 1616: k_curl_r<16, 16, TS><<<gr, 128, smr, c->stream>>>(g, a, out, TL, apply_bc); break;
+    case 3216: k_curl_r<32, 16, TS><<<gr, 128, smr, c->stream>>>(g, a, out, TL, apply_bc); break;
+    case 1608: k_curl_r<16, 8, TS><<<gr, 128, smr, c->stream>>>(g, a, out, TL, apply_bc); break;
+    default: k_curl_r<32, 8, TS><<<gr, 128, smr, c->stream>>>(g, a, out, TL, apply_bc); break;
+  }
   prof_end(c);
   return check_launch(c);
 }
 
+  if (!c->mt[0]) {  // run-time block length
+    const int nt = line_threads(mr);
+    const dim3 gl((g.nth * g.nphi + nt - 1) / nt, g.d[0].nb, 2);
+    prof_begin(c, KI_CURL_R);
+    k_curl_rg<TS><<<gl, nt, (size_t)nt * mr * 8, c->stream>>>(g, a, out, apply_bc);
+    prof_end(c);
+    return check_launch(c);
+  }
 // RHS of one stage on `cur`; if stage > 0 also the stage update into `nx`
 // the persistent phi kernel: as many CTAs as fit on the device at once
+  const size_t smr = smem_line(2, 2, 0, mr, TL);
 template <int MT, int TLC>
 static void launch_phi_p(css_ctx *c, const double *cur) {
   const CssGeo &g = c->g;
@@ -1064,10 +1082,6 @@ static void launch_phi_p(css_ctx *c, const double *cur) {
   const int grid = (int)std::min<long long>(ntile, (long long)std::max(per_sm, 1) * c->nsm);
   k_phi_terms_p<MT, TLC><<<grid, 128, smem, c->stream>>>(g, cur, c->bf, c->dv, c->tbuf);
 }
-
-// threads of a CTA whose lanes keep a line of m doubles in shared memory:
-// 128 while that is at most 48 KB, fewer for longer lines
-static int line_threads(int m) { return m <= 48 ? 128 : (m <= 96 ? 64 : 32); }
 
 // n <= DERIV_MAX derivatives along one direction in one launch
 static int launch_derivs(css_ctx *c, int dir, const DerivItem *it, int n, cudaStream_t st) {
@@ -1208,7 +1222,8 @@ static int launch_rad(css_ctx *c, const double *cur) {
   return check_launch(c);
 }
 
-static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb);
+static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb,
+                      bool have_vcc = false);
 
 // Open radial boundaries: the face sums and scalars of this RHS, after the
 // mass total's refresh at the first call of every ufreq-th step

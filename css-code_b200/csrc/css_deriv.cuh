@@ -452,4 +452,64 @@ __global__ void __launch_bounds__(64) k_adj_t(CssGeo g, const double *__restrict
   }
 }
 
+// ---------------------------------------------------------------------------
+// The radial parts of B = curl A for radial blocks of run-time length: a lane
+// takes a (theta, phi) column, z 0 r A_theta for B_phi, z 1 r A_phi for
+// B_theta, read straight from global memory (the arithmetic of k_curl_r).
+// In tiles of 8 to 16 lines, as k_curl_r takes the 16- and 32-point blocks, a
+// CTA had few lanes solving: 199 us a launch against 81 (FP32), 198 against
+// 86 (FP64) on the ensemble's ragged shells.
+// ---------------------------------------------------------------------------
+template <typename TS>
+struct CurlLine {  // r A along r, from the block's first radius
+  const TS *p;
+  const double *r;
+  size_t ps;
+  __device__ __forceinline__ double operator[](int k) const {
+    return (double)__ldg(p + (long long)k * (long long)ps) * __ldg(r + k);
+  }
+};
+struct CurlIdx {
+  __device__ __forceinline__ int operator()(int j) const { return j - 1; }
+};
+template <typename TS>
+__global__ void __launch_bounds__(DV_NT) k_curl_rg(CssGeo g, const TS *__restrict__ a, double *__restrict__ out,
+                                                   int apply_bc) {
+  extern __shared__ double sm[];
+  const CssDir &D = g.d[0];
+  const int b = blockIdx.y, z = blockIdx.z, m = D.size[b], r0 = D.start[b], ts = blockDim.x;
+  const int line = blockIdx.x * blockDim.x + threadIdx.x;
+  if (line >= g.nth * g.nphi) return;
+  const size_t n = (size_t)g.ncell, ps = (size_t)g.nth * g.nphi, base = (size_t)r0 * ps + line;
+  double *t = sm + threadIdx.x;
+  const int bdry = g.ibcr[z == 0 ? 10 : 11];
+  line_solve_g<1>(CurlLine<TS>{a + z * n + base, g.r_ind + r0, ps}, CurlIdx{}, m, dtype_of(D, b), bdry, 0.0, 0.0,
+                  tabp(g, 0, b, 1, bdry), g.tstride, D.dnum[b], D.dnum[b], 0, t, ts, t, StridedOut{ts});
+  const int it = line % g.nth;
+  const bool wall = apply_bc && (it == 0 || it == g.nth - 1);
+  double *o = out + (z == 0 ? n : 0) + base;  // B_phi, B_theta
+  for (int j0 = 0; j0 < m; j0 += 4) {
+    double in[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) in[k] = j0 + k < m ? o[(size_t)(j0 + k) * ps] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (j0 + k >= m) continue;
+      const int ir = r0 + j0 + k;
+      double d = t[(j0 + k) * ts];
+      if (g.non_uniform) d = d * g.dxdr[ir];
+      double v = z == 0 ? in[k] + d * g.r_inv[ir] : in[k] - d * g.r_inv[ir];
+      if (apply_bc) {  // Compute_B's face zeroing (derivatives.f90:1830-1892)
+        if (wall && (z == 0) == !g.theta_perf_conductor) v = 0.0;
+        const bool lo = ir == 0, hi = ir == g.nr - 1;
+        if ((lo && g.bottom_radial_field) || (hi && g.top_radial_field)) v = 0.0;
+        const bool br0 = (wall && !g.theta_perf_conductor) || (lo && !g.bottom_radial_field && g.bottom_perfect_cond) ||
+                         (hi && !g.top_radial_field && g.top_perfect_cond);
+        if (z == 0 && br0) out[2 * n + base + (size_t)(j0 + k) * ps] = 0.0;
+      }
+      o[(size_t)(j0 + k) * ps] = v;
+    }
+  }
+}
+
 }  // namespace css

@@ -16,6 +16,7 @@ import pytest
 
 from css_b200 import problem
 from css_b200.context import Simulation
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +44,8 @@ CASES = {
     "mixed-16": dict(dims=(40, 48, 80), decomp=(2, 3, 5), precision=1),
     "mixed-mhd-32": dict(dims=(64, 64, 96), decomp=(2, 2, 3), magnetic=True, precision=1),
     "mixed-mhd-16x32": dict(dims=(60, 48, 96), decomp=(3, 3, 3), magnetic=True, precision=1),
+    # FP64 slab too large for shared memory, FP32 ones not: stage 1 alone takes the four kernels
+    "mixed-mhd-r60": dict(dims=(120, 32, 48), decomp=(2, 2, 3), magnetic=True, precision=1),
     "mixed-rk3": dict(dims=(40, 48, 48), decomp=(2, 3, 3), precision=1, time_stepper=3),
 }
 
@@ -79,3 +82,23 @@ def test_general_stage_equals_four_kernels(name, gpu_available):
     bar = 1e-7 if p.precision else 1e-12
     for i in range(two.shape[0]):
         assert np.abs(two[i] - four_[i]).max() <= bar * np.abs(four_[i]).max(), (name, i)
+
+
+@pytest.mark.parametrize("nr", [44, 100, 200])  # radial blocks of 22, 50 and 100 points
+@pytest.mark.parametrize("perfect", [0, 1])
+def test_curl_of_any_radial_block(nr, perfect, gpu_available):
+    """B of a magnetic run whose radial blocks have a run-time length
+    (k_curl_rg: 128, 64 and 32 lines a CTA) against the oracle, both forms of
+    the walls' conditions; the FP64 bar of one derivative pass, 1e-12."""
+    p, prof, v0, _, _ = problem.build((nr, 28, 66), decomp=(2, 2, 3), magnetic=True)
+    p.theta_perf_conductor, p.theta_normal_field = perfect, 1 - perfect
+    p.top_radial_field = p.bottom_radial_field = 1 - perfect
+    p.top_perfect_cond = p.bottom_perfect_cond = perfect
+    v0 = v0.copy()
+    v0[5:] = np.random.default_rng(3).standard_normal(v0[5:].shape)
+    sim = Simulation(p, prof)
+    b = sim.rhs(v0, 1)[0][5:]
+    sim.close()
+    want = O.Oracle(p, prof).rhs(v0, 1)[0][5:]
+    for i in range(3):
+        assert np.abs(b[i] - want[i]).max() <= 1e-12 * np.abs(want[i]).max(), i
