@@ -121,6 +121,19 @@ __device__ __forceinline__ void load_phi_tile(const CssGeo &g, const TS *__restr
   }
 }
 
+// r tile: S[(j+4)*SR + l], lines = theta indices tb..tb+TL-1 at fixed phi
+template <typename TS>
+__device__ __forceinline__ void load_r_tile(const CssGeo &g, const TS *__restrict__ f, double *S, int SR, int r0,
+                                            int m, int tb, int TL, int ip, bool halo) {
+  int w = m + 8;
+  for (int idx = threadIdx.x; idx < TL * w; idx += blockDim.x) {
+    int jj = idx / TL, l = idx - jj * TL;
+    int gr = r0 + jj - 4, gt = tb + l;
+    if ((!halo && (jj < 4 || jj >= m + 4)) || gr < 0 || gr >= g.nr || gt >= g.nth) continue;
+    S[jj * SR + l] = (double)__ldg(f + css_idx(g, gt, ip, gr));
+  }
+}
+
 // copies the LU tables (g1|g2|g3, 1-based, m+2 each) of one block into dst
 __device__ __forceinline__ void stage_table(const CssGeo &g, int dir, int blk, int order, int bdry, int m,
                                             double *dst) {
@@ -1384,8 +1397,13 @@ __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__
   const size_t HS = (size_t)(m + 8) * SR, OS = (size_t)m * SR;
   double *H = sm;  // 0: r*A_theta, 1: r*A_phi
   double *O = H + 2 * HS;
-  const TS *fs[2] = {a, a + n};
-  tiles_ct<2, MT, TLC, 0>(g, fs, H, HS, SR, r0, tb, ip);
+  if constexpr (MT > 0 && TLC > 0) {
+    const TS *fs[2] = {a, a + n};
+    tiles_ct<2, MT, TLC, 0>(g, fs, H, HS, SR, r0, tb, ip);
+  } else {
+    load_r_tile(g, a, H, SR, r0, m, tb, TL, ip, true);
+    load_r_tile(g, a + n, H + HS, SR, r0, m, tb, TL, ip, true);
+  }
   __syncthreads();
   for (int idx = threadIdx.x; idx < TL * (m + 8); idx += blockDim.x) {
     int jj = idx / TL, l = idx - jj * TL;
@@ -1688,10 +1706,6 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
   const int itc = min(it, nth - 1), ipc = min(ip, nphi - 1);
   // this launch diffuses fields off .. off+NF-1 and writes the fields of
   // wmask (a field it writes but does not diffuse gets zero)
-  const int lo_item = (int)threadIdx.x - 32 * NF;
-  const bool lo_p = ty < NF, lo_t = lo_item >= 0 && lo_item < NF * SLD_TP;
-  const int lo_f = lo_p ? ty : (lo_t ? lo_item / SLD_TP : 0), lo_row = lo_t ? lo_item % SLD_TP : 0;
-  const double lo_tiny = g.tinyvar[lo_f + off], lo_itiny = g.inv_tinyvar2[lo_f + off];
   const bool hydro_part = (wmask & 0x1Fu) != 0;  // the fields the corrections act on
   const bool edge_lo = t0 == 0, edge_hi = t0 + SLD_TT >= nth;
   // theta faces of this thread: the upper face of its cell; their sin(face) factors
@@ -1703,6 +1717,10 @@ __global__ void __launch_bounds__(SLD_TT * SLD_TP, 2) k_sld(CssGeo g, const doub
   // alone the other six waited at the barrier for half again their own work:
   // 1.77 against 1.69 ms on 128x256x512, 517 against 493 us on MHD 128x128x256.
   const bool th_lo_in = t0 > 0 && t0 < nth;
+  const int lo_item = (int)threadIdx.x - 32 * NF;
+  const bool lo_p = ty < NF, lo_t = lo_item >= 0 && lo_item < NF * SLD_TP;
+  const int lo_f = lo_p ? ty : (lo_t ? lo_item / SLD_TP : 0), lo_row = lo_t ? lo_item % SLD_TP : 0;
+  const double lo_tiny = g.tinyvar[lo_f + off], lo_itiny = g.inv_tinyvar2[lo_f + off];
   const SldCopy cp = sld_copy_plan(g, t0, p0);
   // per-field r window: x(ir-1), x(ir), x(ir+1), x(ir+2), and the de of the
   // lower r face of the current radius
