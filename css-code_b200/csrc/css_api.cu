@@ -393,12 +393,12 @@ static int setup_kernels() {
   CSS_LINE_ATTR(k_deriv_s<0, 0>);
   CSS_LINE_ATTR(k_deriv_s<2, 0>);
   CSS_LINE_ATTR(k_deriv_t<0>);
+  CSS_LINE_ATTR(k_curl_rg<double>);
+  CSS_LINE_ATTR(k_curl_rg<float>);
   CSS_LINE_ATTR(k_adj_s<0, 1, 0>);
   CSS_LINE_ATTR(k_adj_s<0, 2, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 1, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 2, 0>);
-  CSS_LINE_ATTR(k_curl_rg<double>);
-  CSS_LINE_ATTR(k_curl_rg<float>);
   CSS_LINE_ATTR(k_adj_t<1, 0>);
   CSS_LINE_ATTR(k_adj_t<2, 0>);
 #undef CSS_LINE_ATTR
@@ -996,6 +996,10 @@ static int check_launch(css_ctx *c) {
   return CSS_OK;
 }
 
+// threads of a CTA whose lanes keep a line of m doubles in shared memory:
+// 128 while that is at most 48 KB, fewer for longer lines
+static int line_threads(int m) { return m <= 48 ? 128 : (m <= 96 ? 64 : 32); }
+
 template <typename TS>
 static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
   const CssGeo &g = c->g;
@@ -1046,8 +1050,17 @@ static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
     prof_end(c);
     return check_launch(c);
   }
+  if (!c->mt[0]) {  // run-time block length
+    const int nt = line_threads(mr);
+    const dim3 gl((g.nth * g.nphi + nt - 1) / nt, g.d[0].nb, 2);
+    prof_begin(c, KI_CURL_R);
+    k_curl_rg<TS><<<gl, nt, (size_t)nt * mr * 8, c->stream>>>(g, a, out, apply_bc);
+    prof_end(c);
+    return check_launch(c);
+  }
   TL = c->tl_r;
   dim3 gr(g.d[0].nb * ((g.nth + TL - 1) / TL), g.nphi);
+  const size_t smr = smem_line(2, 2, 0, mr, TL);
   prof_begin(c, KI_CURL_R);
   switch (c->mt[0] * 100 + TL) {
     case 1616: k_curl_r<16, 16, TS><<<gr, 128, smr, c->stream>>>(g, a, out, TL, apply_bc); break;
@@ -1059,17 +1072,8 @@ static int launch_curl(css_ctx *c, const TS *a, double *out, int apply_bc) {
   return check_launch(c);
 }
 
-  if (!c->mt[0]) {  // run-time block length
-    const int nt = line_threads(mr);
-    const dim3 gl((g.nth * g.nphi + nt - 1) / nt, g.d[0].nb, 2);
-    prof_begin(c, KI_CURL_R);
-    k_curl_rg<TS><<<gl, nt, (size_t)nt * mr * 8, c->stream>>>(g, a, out, apply_bc);
-    prof_end(c);
-    return check_launch(c);
-  }
 // RHS of one stage on `cur`; if stage > 0 also the stage update into `nx`
 // the persistent phi kernel: as many CTAs as fit on the device at once
-  const size_t smr = smem_line(2, 2, 0, mr, TL);
 template <int MT, int TLC>
 static void launch_phi_p(css_ctx *c, const double *cur) {
   const CssGeo &g = c->g;
@@ -1222,8 +1226,7 @@ static int launch_rad(css_ctx *c, const double *cur) {
   return check_launch(c);
 }
 
-static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb,
-                      bool have_vcc = false);
+static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb);
 
 // Open radial boundaries: the face sums and scalars of this RHS, after the
 // mass total's refresh at the first call of every ufreq-th step

@@ -121,19 +121,6 @@ __device__ __forceinline__ void load_phi_tile(const CssGeo &g, const TS *__restr
   }
 }
 
-// r tile: S[(j+4)*SR + l], lines = theta indices tb..tb+TL-1 at fixed phi
-template <typename TS>
-__device__ __forceinline__ void load_r_tile(const CssGeo &g, const TS *__restrict__ f, double *S, int SR, int r0,
-                                            int m, int tb, int TL, int ip, bool halo) {
-  int w = m + 8;
-  for (int idx = threadIdx.x; idx < TL * w; idx += blockDim.x) {
-    int jj = idx / TL, l = idx - jj * TL;
-    int gr = r0 + jj - 4, gt = tb + l;
-    if ((!halo && (jj < 4 || jj >= m + 4)) || gr < 0 || gr >= g.nr || gt >= g.nth) continue;
-    S[jj * SR + l] = (double)__ldg(f + css_idx(g, gt, ip, gr));
-  }
-}
-
 // copies the LU tables (g1|g2|g3, 1-based, m+2 each) of one block into dst
 __device__ __forceinline__ void stage_table(const CssGeo &g, int dir, int blk, int order, int bdry, int m,
                                             double *dst) {
@@ -1397,13 +1384,8 @@ __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__
   const size_t HS = (size_t)(m + 8) * SR, OS = (size_t)m * SR;
   double *H = sm;  // 0: r*A_theta, 1: r*A_phi
   double *O = H + 2 * HS;
-  if constexpr (MT > 0 && TLC > 0) {
-    const TS *fs[2] = {a, a + n};
-    tiles_ct<2, MT, TLC, 0>(g, fs, H, HS, SR, r0, tb, ip);
-  } else {
-    load_r_tile(g, a, H, SR, r0, m, tb, TL, ip, true);
-    load_r_tile(g, a + n, H + HS, SR, r0, m, tb, TL, ip, true);
-  }
+  const TS *fs[2] = {a, a + n};
+  tiles_ct<2, MT, TLC, 0>(g, fs, H, HS, SR, r0, tb, ip);
   __syncthreads();
   for (int idx = threadIdx.x; idx < TL * (m + 8); idx += blockDim.x) {
     int jj = idx / TL, l = idx - jj * TL;
