@@ -379,14 +379,18 @@ static int setup_kernels() {
   if (int rc2 = setup_stage<float, float, 2, 2, 3, -1>()) return rc2;
   if (int rc2 = setup_stage<float, double, 0, 4, -1>()) return rc2;
   if (int rc2 = setup_stage<float, double, 2, 4, -1>()) return rc2;
-  CSS_FUSED_ATTR((k_rstage<0, 1>), RstageCfg<0>);
-  CSS_FUSED_ATTR((k_rstage<0, 2>), RstageCfg<0>);
-  CSS_FUSED_ATTR((k_rstage<0, 3>), RstageCfg<0>);
-  CSS_FUSED_ATTR((k_rstage<0, 4>), RstageCfg<0>);
-  CSS_FUSED_ATTR((k_rstage<1, 1>), RstageCfg<1>);
-  CSS_FUSED_ATTR((k_rstage<1, 2>), RstageCfg<1>);
-  CSS_FUSED_ATTR((k_rstage<1, 3>), RstageCfg<1>);
-  CSS_FUSED_ATTR((k_rstage<1, 4>), RstageCfg<1>);
+#define CSS_RSTAGE_ATTR(S, T, U)                       \
+  CSS_FUSED_ATTR((k_rstage<0, S, T, U>), RstageCfg<0>); \
+  CSS_FUSED_ATTR((k_rstage<1, S, T, U>), RstageCfg<1>)
+  CSS_RSTAGE_ATTR(1, double, double);
+  CSS_RSTAGE_ATTR(2, double, double);
+  CSS_RSTAGE_ATTR(3, double, double);
+  CSS_RSTAGE_ATTR(4, double, double);
+  CSS_RSTAGE_ATTR(1, double, float);
+  CSS_RSTAGE_ATTR(2, float, float);
+  CSS_RSTAGE_ATTR(3, float, float);
+  CSS_RSTAGE_ATTR(4, float, double);
+#undef CSS_RSTAGE_ATTR
 #undef CSS_FUSED_ATTR
   // run-time block lengths: up to 256 points a line
 #define CSS_LINE_ATTR(...) CUDA_TRY(cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
@@ -1454,29 +1458,42 @@ static int launch_plane(css_ctx *c, const TS *cur, int *map) {
   return check_launch(c);
 }
 
-// the stage pass of an FP64 RK4 run with closed radial faces and 32-point
-// blocks in r and theta (k_rstage); mi: the state buffer `cur` is
-static int launch_rstage32(css_ctx *c, const double *cur, double *nx, int stage, double dtcur, int mi) {
+// the stage pass of an RK4 run with closed radial faces and 32-point blocks
+// in r and theta (k_rstage); mi: the state buffer `cur` is
+template <typename TS, typename TO>
+static int launch_rstage32(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, int mi) {
   const CssGeo &g = c->g;
   const int mag = g.magnetic;
   // hydro: one tile per CTA; MHD: persistent, one CTA per SM
   const int nrtile = g.d[0].nb * g.d[1].nb * g.nphi;
   const dim3 gb(mag ? std::min(c->nsm, nrtile) : nrtile);
   prof_begin(c, KI_RSTAGE);
-#define CSS_RSTAGE(M, S)                                                                                      \
-  k_rstage<M, S><<<gb, RstageCfg<M>::NT, RstageCfg<M>::SMEM, c->stream>>>(g, cur, c->bf, c->dv, c->v0, c->vs, nx, c->tbuf, \
-                                                              c->rtw, dtcur, c->flag, c->smaps[mi], c->smaps[3], \
-                                                              c->smaps[4])
-  switch (stage + (mag ? 10 : 0)) {
-    case 1: CSS_RSTAGE(0, 1); break;
-    case 2: CSS_RSTAGE(0, 2); break;
-    case 3: CSS_RSTAGE(0, 3); break;
-    case 4: CSS_RSTAGE(0, 4); break;
-    case 11: CSS_RSTAGE(1, 1); break;
-    case 12: CSS_RSTAGE(1, 2); break;
-    case 13: CSS_RSTAGE(1, 3); break;
-    case 14: CSS_RSTAGE(1, 4); break;
-    default: set_err("launch_rstage32: stage %d", stage); return CSS_ERR_ARG;
+  const SlabMaps &sc = sizeof(TS) == 4 ? c->fslab[mi - 1] : c->smaps[mi];
+#define CSS_RSTAGE(S)                                                                                               \
+  do {                                                                                                              \
+    if (mag)                                                                                                        \
+      k_rstage<1, S, TS, TO><<<gb, RstageCfg<1>::NT, RstageCfg<1>::SMEM, c->stream>>>(                              \
+          g, c->bf, c->dv, c->v0, c->vs, nx, c->tbuf, c->rtw, dtcur, c->flag, sc, c->smaps[3], c->smaps[4]);        \
+    else                                                                                                            \
+      k_rstage<0, S, TS, TO><<<gb, RstageCfg<0>::NT, RstageCfg<0>::SMEM, c->stream>>>(                              \
+          g, c->bf, c->dv, c->v0, c->vs, nx, c->tbuf, c->rtw, dtcur, c->flag, sc, c->smaps[3], c->smaps[4]);        \
+  } while (0)
+  if constexpr (sizeof(TS) == 8 && sizeof(TO) == 8) {
+    switch (stage) {
+      case 1: CSS_RSTAGE(1); break;
+      case 2: CSS_RSTAGE(2); break;
+      case 3: CSS_RSTAGE(3); break;
+      case 4: CSS_RSTAGE(4); break;
+      default: set_err("launch_rstage32: stage %d", stage); return CSS_ERR_ARG;
+    }
+  } else if constexpr (sizeof(TS) == 8) {  // mixed: vars0 -> U1
+    CSS_RSTAGE(1);
+  } else if constexpr (sizeof(TO) == 8) {  // U3 -> vars0
+    CSS_RSTAGE(4);
+  } else if (stage == 2) {
+    CSS_RSTAGE(2);
+  } else {
+    CSS_RSTAGE(3);
   }
 #undef CSS_RSTAGE
   prof_end(c);
@@ -1485,9 +1502,13 @@ static int launch_rstage32(css_ctx *c, const double *cur, double *nx, int stage,
 
 // A stage as the plane pass and the general stage pass (css_stage.cuh):
 // [curl] -> k_thph -> [explicit viscosity] -> [face sums of open radial
-// faces] -> [SLD of the step's start] -> k_rstage (FP64 RK4 stages of 32-point
-// blocks, closed faces: it holds the MHD slab of 32 radii in one persistent
-// 512-thread CTA an SM) or k_rstage_g
+// faces] -> [SLD of the step's start] -> k_rstage (RK4 stages of 32-point
+// radial and theta blocks, closed faces: unrolled solves, and for MHD one
+// persistent 512-thread CTA an SM whose next slab arrives under the pointwise
+// phases; FP32 stages of MHD 128x128x256 take 434 us there against 540 in
+// k_rstage_g, stage 1, whose FP64 slab leaves that one CTA of 256 threads an
+// SM, 406 against 743; mixed hydro 128x256x512 steps 8.80 against 9.59 ms) or
+// k_rstage_g
 template <typename TS, typename TO>
 static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur, double ca, double cb,
                             double dsld, bool with_sld) {
@@ -1505,8 +1526,7 @@ static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double
     if (with_sld)
       if (int rc = launch_sld(c, (const double *)cur, (const double *)cur + 5 * c->ncell, c->vs, c->tbuf)) return rc;
   }
-  if constexpr (sizeof(TS) == 8 && sizeof(TO) == 8)
-    if (stage <= 4 && c->mt[0] == 32 && c->mt[1] == 32 && !c->io) return launch_rstage32(c, cur, nx, stage, dtcur, mi);
+  if (stage <= 4 && c->mt[0] == 32 && c->mt[1] == 32 && !c->io) return launch_rstage32(c, cur, nx, stage, dtcur, mi);
   prof_begin(c, KI_RSTAGE);
   const dim3 gr(g.d[0].nb * ((g.nth + 31) / 32), g.nphi);
   const size_t smem = stage_smem(mag, g.d[0].maxm, (int)sizeof(TS));

@@ -873,32 +873,68 @@ __global__ void __launch_bounds__(CR_NT, 4) k_curl_rs(CssGeo g, double *__restri
 
 // the slab of tile T [and the wall rows of d(rho)/dtheta] by TMA boxes: per
 // field the 40 radial rows r0-4 .. r0+35 of the 32 theta values (zero
-// outside [0, nr)), on one mbarrier armed with the byte count
-template <int MAG>
+// outside [0, nr)), on one mbarrier armed with the byte count.  An FP32 stage
+// state arrives in the upper half of each field's FP64 slab.
+template <int MAG, typename TS>
 __device__ __forceinline__ void rstage_stage_tma(const CssGeo &g, const RstageTile &T, double *H, double *W,
                                                  const SlabMaps &sc, const SlabMaps &sb, const SlabMaps &sw,
                                                  uint64_t *bar) {
   using C = RstageCfg<MAG>;
+  constexpr int HALF = sizeof(TS) == 4 ? FB_FIELD / 2 : 0;
   const bool lw = g.d[1].lphys[T.bt], hw = g.d[1].rphys[T.bt];
-  mbar_expect_tx(bar, 8u * (C::NH * FB_FIELD + ((lw || hw) ? FB_OUT : 0)));
+  mbar_expect_tx(bar, 8u * (C::NH * FB_FIELD - 5 * HALF + ((lw || hw) ? FB_OUT : 0)));
 #pragma unroll
   for (int f = 0; f < C::NH; f++) {
     // H order w v u s rho [bt bp]: fields 1 2 3 4 0 of the state, 0 1 of B
     const CUtensorMap *m = f < 5 ? &sc.slab : &sb.slab;
     const int w = f < 4 ? f + 1 : (f == 4 ? 0 : f - 5);
-    tma_load_4d(H + (size_t)f * FB_FIELD, m, T.t0, T.ip, T.r0 - 4, w, bar);
+    tma_load_4d(H + (size_t)f * FB_FIELD + (f < 5 ? HALF : 0), m, T.t0, T.ip, T.r0 - 4, w, bar);
   }
   if (lw || hw) tma_load_4d(W, &sw.slab, 0, lw ? 0 : 1, T.ip, T.r0, bar);
+}
+
+// widen a slab of FP32 state fields in place (the whole CTA), rho and s with
+// their background (as thph_widen)
+template <int NT>
+__device__ __forceinline__ void rstage_widen(const CssGeo &g, const RstageTile &T, double *H) {
+  constexpr int K = (FB_FIELD + NT - 1) / NT;
+  float v[5][K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = threadIdx.x + k * NT;
+    if (i < FB_FIELD)
+#pragma unroll
+      for (int f = 0; f < 5; f++) v[f][k] = reinterpret_cast<const float *>(H + f * FB_FIELD + FB_FIELD / 2)[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = threadIdx.x + k * NT, r = T.r0 - 4 + i / FM, t = T.t0 + (i & (FM - 1));
+    if (i < FB_FIELD) {
+      const bool in = r >= 0 && r < g.nr;
+      const size_t b = in ? bgi(g, r, t) : 0;
+#pragma unroll
+      for (int f = 0; f < 5; f++) {
+        double x = (double)v[f][k];
+        if (f == 3 && in) x += __ldg(bg_s(g) + b);
+        if (f == 4 && in) x += __ldg(bg_rho(g) + b);
+        H[f * FB_FIELD + i] = x;
+      }
+    }
+  }
+  __syncthreads();
 }
 
 // STG: the RK4 stage (1..4), compiled in:
 //   1: vs = (sld ? vs + dv/6 : dv); nx = v0 + dtcur*dv
 //   2,3: vs = vs + dv/3;            nx = v0 + dtcur*dv
 //   4: vs + dv/6 accumulated;       nx = v0 + dtcur*(vs + dv/6)  (nx is v0)
-template <int MAG, int STG>
-__global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssGeo g, const double *__restrict__ cur,
+// TS, TO: storage of the stage input and of the next stage state (FP32 in a
+// mixed run's inner stages, rho and s about their background)
+template <int MAG, int STG, typename TS, typename TO>
+__global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssGeo g,
                                                               const double *__restrict__ bf, const double *dv,
-                                                              const double *v0, double *vs, double *nx,
+                                                              const double *v0, double *vs, TO *nx,
                                                               const double *__restrict__ tbuf,
                                                               const double *__restrict__ rtw, double dtcur,
                                                               int *flag, const __grid_constant__ SlabMaps sc,
@@ -952,7 +988,7 @@ __global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssG
     // ---- the slab: the first tile's copies now, each later tile's issued
     // under the previous tile's pointwise phases (MHD) ----
     const bool lw = DT.lphys[T.bt], hw = DT.rphys[T.bt];
-    if (i == 0 && tid == 0) rstage_stage_tma<MAG>(g, T, H, W, sc, sb, sw, bar);
+    if (i == 0 && tid == 0) rstage_stage_tma<MAG, TS>(g, T, H, W, sc, sb, sw, bar);
     const unsigned parity = (unsigned)i & 1u;
     if (__syncthreads_or(!mbar_wait_bounded(bar, parity, kWaitCycles))) {
       // copies that never complete: report them and stop, after giving the
@@ -964,6 +1000,7 @@ __global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssG
       return;
     }
 
+    if constexpr (sizeof(TS) == 4) rstage_widen<C::NT>(g, T, H);
     // ---- radial solves: tile k = warp, line = lane ----
     const int dtype = dtype_of(D, T.br);
     if (wrp < C::ND) {
@@ -1044,7 +1081,7 @@ __global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssG
       __syncthreads();
       if (more && tid == 0) {
         fence_proxy_async();
-        rstage_stage_tma<MAG>(g, rstage_tile(g, q + gridDim.x), H, W, sc, sb, sw, bar);
+        rstage_stage_tma<MAG, TS>(g, rstage_tile(g, q + gridDim.x), H, W, sc, sb, sw, bar);
       }
     }
     // ---- radial pointwise: PPT points per thread (row j = warp + NW h, t = lane) ----
@@ -1187,7 +1224,12 @@ __global__ void __launch_bounds__(RstageCfg<MAG>::NT, MAG ? 1 : 2) k_rstage(CssG
           }
         }
         if (!isfinite(o)) bad = 1;
-        nx[qi] = o;
+        double bgv = 0.0;
+        if constexpr (sizeof(TO) == 4) {
+          if (iv == 0) bgv = bg_rho(g)[bgi(g, ir, it)];
+          else if (iv == 4) bgv = bg_s(g)[bgi(g, ir, it)];
+        }
+        nx[qi] = st_store<TO>(o, bgv);
       }
     }
   }
