@@ -1230,7 +1230,8 @@ static int launch_rad(css_ctx *c, const double *cur) {
   return check_launch(c);
 }
 
-static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb);
+static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb,
+                      bool have_vcc = false);
 
 // Open radial boundaries: the face sums and scalars of this RHS, after the
 // mass total's refresh at the first call of every ufreq-th step
@@ -1371,13 +1372,16 @@ static int launch_rhs(css_ctx *c, const TS *cur, TO *nx, int stage, double dtcur
 
 // slope-limited diffusion tendency of `v` (A in av for MHD; B must be in
 // c->bf) into dout
-static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb) {
+static int launch_sld(css_ctx *c, const double *v, const double *av, double *dout, const double *tb, bool have_vcc) {
   const CssGeo &g = c->g;
   int nb = 148 * 16;
-  prof_begin(c, KI_SLD_VCC);
-  k_sld_vcc<<<nb, 256, 0, c->stream>>>(g, v, c->bf, c->vcc);
-  prof_end(c);
-  if (int rc = check_launch(c)) return rc;
+  if (!have_vcc) {  // the two-pass stage's plane pass has left it
+    prof_begin(c, KI_SLD_VCC);
+    if (g.magnetic) k_sld_vcc<1><<<nb, 256, 0, c->stream>>>(g, v, c->bf, c->vcc);
+    else k_sld_vcc<0><<<nb, 256, 0, c->stream>>>(g, v, c->bf, c->vcc);
+    prof_end(c);
+    if (int rc = check_launch(c)) return rc;
+  }
   prof_begin(c, KI_SLD);
   // radii a CTA marches over: the chunk that takes the fewest radii in a row
   // over the waves of two CTAs an SM, where a chunk's start (its windows, the
@@ -1421,7 +1425,7 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
   if (g.do_ohmic_heating) {
     if (int rc = launch_curl(c, (const double *)(dout + 5 * c->ncell), c->cda, 0)) return rc;
     prof_begin(c, KI_SLD_OHMIC);
-    k_sld_ohmic<<<nb, 256, 0, c->stream>>>(g, v, c->bf, c->cda, dout);
+    k_sld_ohmic<<<nb, 256, 0, c->stream>>>(g, v, c->bf, c->cda, dout, tb);
     prof_end(c);
     if (int rc = check_launch(c)) return rc;
   }
@@ -1429,9 +1433,9 @@ static int launch_sld(css_ctx *c, const double *v, const double *av, double *dou
 }
 
 // the plane pass of a stage (k_thph: the theta and phi sweeps of `cur`),
-// persistent, one CTA per SM
+// persistent, one CTA per SM; vcc: NULL or where the SLD's speed^2 goes
 template <typename TS>
-static int launch_plane(css_ctx *c, const TS *cur, int *map) {
+static int launch_plane(css_ctx *c, const TS *cur, int *map, double *vcc) {
   const void *bufs[3] = {c->v0, c->vA, c->vB};
   int mi = 0;
   while (mi < 3 && bufs[mi] != (const void *)cur) mi++;
@@ -1441,7 +1445,7 @@ static int launch_plane(css_ctx *c, const TS *cur, int *map) {
   const dim3 ga(c->nsm);
   prof_begin(c, KI_THPH);
 #define CSS_THPH(M, BT, BP)                                                                                       \
-  k_thph<M, TS, BT, BP><<<ga, FNT, ThphCfg<M, TS>::SMEM, c->stream>>>(c->g, c->dv, c->tbuf, c->rtw, mc, mb, c->flag)
+  k_thph<M, TS, BT, BP><<<ga, FNT, ThphCfg<M, TS>::SMEM, c->stream>>>(c->g, c->dv, c->tbuf, c->rtw, vcc, mc, mb, c->flag)
   switch ((c->g.magnetic ? 10000 : 0) + c->mt[1] * 100 + c->mt[2]) {
     case 3232: CSS_THPH(0, 32, 32); break;
     case 3216: CSS_THPH(0, 32, 16); break;
@@ -1517,14 +1521,16 @@ static int launch_stage_two(css_ctx *c, const TS *cur, TO *nx, int stage, double
   if (mag)
     if (int rc = launch_curl(c, cur + 5 * c->ncell, c->bf, 1)) return rc;
   int mi;
-  if (int rc = launch_plane(c, cur, &mi)) return rc;
+  if (int rc = launch_plane(c, cur, &mi, with_sld ? c->vcc : nullptr)) return rc;
   if constexpr (sizeof(TS) == 8) {
     if (c->p.laplacian)
       if (int rc = launch_lap(c, (const double *)cur)) return rc;
     if (c->io)
       if (int rc = launch_inout(c, (const double *)cur)) return rc;
     if (with_sld)
-      if (int rc = launch_sld(c, (const double *)cur, (const double *)cur + 5 * c->ncell, c->vs, c->tbuf)) return rc;
+      if (int rc = launch_sld(c, (const double *)cur, (const double *)cur + 5 * c->ncell, c->vs, c->tbuf,
+                              true))
+        return rc;
   }
   if (stage <= 4 && c->mt[0] == 32 && c->mt[1] == 32 && !c->io) return launch_rstage32(c, cur, nx, stage, dtcur, mi);
   prof_begin(c, KI_RSTAGE);

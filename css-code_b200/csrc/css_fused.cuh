@@ -371,9 +371,13 @@ __device__ __forceinline__ void thph_theta_row(const CssGeo &g, const double *F,
 
 // TS: storage of the stage states; BT, BP: theta and phi block lengths (16 or
 // 32, every block of a direction the same)
+// vcc: where not NULL, the SLD's speed^2 of the state is written too (k_sld_vcc's
+// arithmetic; a step's first stage, whose state the SLD diffuses).  The pass has
+// every operand in hand: it takes 25 us longer on MHD 128x128x256 where a pass
+// of its own took 42, 6 against 80 on hydro 128x256x512
 template <int MAG, typename TS, int BT, int BP>
 __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, double *__restrict__ dv, double *__restrict__ tbuf,
-                                                 double *__restrict__ rtw, const __grid_constant__ PlaneMaps mc,
+                                                 double *__restrict__ rtw, double *__restrict__ vcc, const __grid_constant__ PlaneMaps mc,
                                                  const __grid_constant__ PlaneMaps mb, int *flag) {
   using C = ThphCfg<MAG, TS>;
   constexpr int NA = MAG ? 8 : 5;
@@ -435,10 +439,12 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, double *__restrict__ 
     const int itc = BT == FM ? it : min(it, g.nth - 1);
     if constexpr (sizeof(TS) == 4) thph_widen(g, T, F);
     // ---- T, 1/rho and 1/(rho T) of this thread's two points (rows wrp,
-    // wrp + 16, theta t0 + lane), T also to tbuf ----
+    // wrp + 16, theta t0 + lane), T also to tbuf.  Before the solves in hydro
+    // runs too: on the four warps that solve nothing there, with a read back
+    // after the barrier, the pass took 7 % longer ----
     double tq[2], rq[2], rtq[2];
+    const size_t pl = plane(g, ir);
     {
-      const size_t pl = plane(g, ir);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int ic = (wrp + 16 * h) * FA_RW + lane + 4;
@@ -480,6 +486,16 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, double *__restrict__ 
       if (more && tid == 0) {
         fence_proxy_async();
         thph_stage_tma<C::NF, TS>(g, mc, mb, thph_tile<BT, BP>(g, q + gridDim.x), F, bar);
+      }
+    }
+    if (vcc) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int p = wrp + 16 * h;
+        if (!tin || (BP < FM && p >= lenp)) continue;
+        const size_t id = pl + (size_t)(T.p0 + p) * g.nth + it;
+        vcc[id] = sld_speed2<MAG>(g, ir, id, pv[h][1], pv[h][2], pv[h][3], rq[h], MAG ? pv[h][4] : 0.0,
+                                  MAG ? pv[h][5] : 0.0, MAG ? pv[h][6] : 0.0);
       }
     }
     // ---- theta pointwise (Source_Theta_Terms, Lorentz, induction, and
@@ -594,7 +610,6 @@ __global__ void __launch_bounds__(FNT, 1) k_thph(CssGeo g, double *__restrict__ 
         }
         acc[h][0] = drho; acc[h][1] = dw; acc[h][2] = dvv; acc[h][3] = du; acc[h][4] = ds;
       }
-      const size_t pl = plane(g, ir);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const size_t id = pl + (size_t)(T.p0 + wrp + 16 * h) * g.nth + it;
