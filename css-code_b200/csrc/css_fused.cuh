@@ -794,17 +794,20 @@ __device__ __forceinline__ RstageTile rstage_tile(const CssGeo &g, int q) {
 // solved along r (one warp each, one theta column per lane) and
 // B_phi += d(r A_theta)/dr / r, B_theta -= d(r A_phi)/dr / r (times dxdr on a
 // non-uniform grid), then Compute_B's face zeroing (derivatives.f90:
-// 1830-1892) -- the arithmetic of k_curl_r, in the same order.
+// 1830-1892) -- the arithmetic of k_curl_r, in the same order.  B_r has no
+// radial part: only the faces that zero it write it (read and written at every
+// point, 16 of 68 bytes a cell, the pass took 68 us on MHD 128x128x256 and
+// 1.86 ms on 256x512x1024, now 64 and 1.61).
 constexpr int CR_NT = 128;
 constexpr int CR_PPT = FM * FM / CR_NT;
 constexpr size_t CR_SMEM = 8 * (2 * (size_t)FB_FIELD + 2 * (size_t)FB_OUT + 1);
 
-// Four CTAs per SM (128 registers, 80 bytes spilled): 2.13-2.17 ms per curl
-// on MHD 256x512x1024, against 2.30 with three (164 registers), 2.33 with
-// six (80 registers, 272 bytes spilled) and 3.07 with six CTAs of 64
-// threads that load their B parts after the solves; the two-pass form's
-// k_curl_r takes 2.46.
-__global__ void __launch_bounds__(CR_NT, 4) k_curl_rs(CssGeo g, double *__restrict__ out,
+// Five CTAs per SM (96 registers, 56 bytes spilled), 256x512x1024: 1.61 ms a
+// curl, against 1.71 with four (128 registers, no spill) and 1.66 with six (80
+// registers, 128 bytes); on 128x128x256 64, 63 and 67 us.  Six CTAs of 64
+// threads that load their B parts after the solves were half again slower, the
+// tile kernel k_curl_r by a tenth.
+__global__ void __launch_bounds__(CR_NT, 5) k_curl_rs(CssGeo g, double *__restrict__ out,
                                                    const __grid_constant__ SlabMaps ms, int apply_bc, int *flag) {
   extern __shared__ __align__(128) double sm[];
   double *H = sm;                   // 0: A_theta, 1: A_phi, then times r
@@ -826,14 +829,13 @@ __global__ void __launch_bounds__(CR_NT, 4) k_curl_rs(CssGeo g, double *__restri
   }
   // this thread's points (row j = r - r0, theta column lane): the theta
   // and phi parts of B, loaded while the slab arrives
-  double in_t[CR_PPT], in_p[CR_PPT], in_r[CR_PPT];
+  double in_t[CR_PPT], in_p[CR_PPT];
 #pragma unroll
   for (int k = 0; k < CR_PPT; k++) {
     const int j = wrp + 4 * k;
     const size_t id = css_idx(g, T.t0 + lane, T.ip, T.r0 + j);
     in_t[k] = out[id];
     in_p[k] = out[n + id];
-    in_r[k] = out[2 * n + id];
   }
   if (__syncthreads_or(!mbar_wait_bounded(bar, 0u, kWaitCycles))) {
     if (tid == 0) {
@@ -865,22 +867,7 @@ __global__ void __launch_bounds__(CR_NT, 4) k_curl_rs(CssGeo g, double *__restri
     d = O[FB_OUT + j * FM + lane];
     if (g.non_uniform) d = d * g.dxdr[ir];
     double bt_ = in_t[k] - d * g.r_inv[ir];
-    double br_ = in_r[k];
-    if (apply_bc) {
-      if (it == 0 || it == g.nth - 1) {
-        if (g.theta_perf_conductor) bt_ = 0.0;
-        else { bp_ = 0.0; br_ = 0.0; }
-      }
-      if (ir == 0) {
-        if (g.bottom_radial_field) { bt_ = 0.0; bp_ = 0.0; }
-        else if (g.bottom_perfect_cond) br_ = 0.0;
-      }
-      if (ir == g.nr - 1) {
-        if (g.top_radial_field) { bt_ = 0.0; bp_ = 0.0; }
-        else if (g.top_perfect_cond) br_ = 0.0;
-      }
-      out[2 * n + id] = br_;
-    }
+    if (apply_bc && curl_faces(g, it, ir, bt_, bp_)) out[2 * n + id] = 0.0;
     out[id] = bt_;
     out[n + id] = bp_;
   }

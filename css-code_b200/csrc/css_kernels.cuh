@@ -1369,6 +1369,25 @@ __global__ void __launch_bounds__(256, 2) k_curl_tp(CssGeo g, const TS *__restri
   }
 }
 
+// Compute_B's face zeroing (derivatives.f90:1830-1892) of B_theta and B_phi
+// at one point; true where B_r is zeroed too
+__device__ __forceinline__ bool curl_faces(const CssGeo &g, int it, int ir, double &bt, double &bp) {
+  bool br0 = false;
+  if (it == 0 || it == g.nth - 1) {
+    if (g.theta_perf_conductor) bt = 0.0;
+    else { bp = 0.0; br0 = true; }
+  }
+  if (ir == 0) {
+    if (g.bottom_radial_field) { bt = 0.0; bp = 0.0; }
+    else if (g.bottom_perfect_cond) br0 = true;
+  }
+  if (ir == g.nr - 1) {
+    if (g.top_radial_field) { bt = 0.0; bp = 0.0; }
+    else if (g.top_perfect_cond) br0 = true;
+  }
+  return br0;
+}
+
 template <int MT, int TLC, typename TS>
 __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__ a, double *__restrict__ out,
                                                 int TL, int apply_bc) {
@@ -1406,7 +1425,7 @@ __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__
   constexpr int PPT = (MT > 0 && TLC > 0) ? (MT * TLC + NT - 1) / NT : 1;
   const int stride = (MT > 0 && TLC > 0) ? NT : (int)blockDim.x;
   for (int pt0 = threadIdx.x; pt0 < TL * m; pt0 += PPT * stride) {
-  double in_t[PPT], in_p[PPT], in_r[PPT];
+  double in_t[PPT], in_p[PPT];
 #pragma unroll
   for (int k = 0; k < PPT; k++) {
     const int pt = pt0 + k * stride, j = pt / TL, l = pt - j * TL;
@@ -1414,7 +1433,6 @@ __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__
       const size_t id = css_idx(g, tb + l, ip, r0 + j);
       in_t[k] = out[id];
       in_p[k] = out[n + id];
-      in_r[k] = out[2 * n + id];
     }
   }
 #pragma unroll
@@ -1430,22 +1448,7 @@ __global__ void __launch_bounds__(128) k_curl_r(CssGeo g, const TS *__restrict__
     d = O[OS + (size_t)j * SR + l];
     if (g.non_uniform) d = d * g.dxdr[ir];
     double bt_ = in_t[k] - d * g.r_inv[ir];
-    double br_ = in_r[k];
-    if (apply_bc) {
-      if (it == 0 || it == g.nth - 1) {
-        if (g.theta_perf_conductor) bt_ = 0.0;
-        else { bp_ = 0.0; br_ = 0.0; }
-      }
-      if (ir == 0) {
-        if (g.bottom_radial_field) { bt_ = 0.0; bp_ = 0.0; }
-        else if (g.bottom_perfect_cond) br_ = 0.0;
-      }
-      if (ir == g.nr - 1) {
-        if (g.top_radial_field) { bt_ = 0.0; bp_ = 0.0; }
-        else if (g.top_perfect_cond) br_ = 0.0;
-      }
-      out[2 * n + id] = br_;
-    }
+    if (apply_bc && curl_faces(g, it, ir, bt_, bp_)) out[2 * n + id] = 0.0;
     out[id] = bt_;
     out[n + id] = bp_;
   }
