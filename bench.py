@@ -769,11 +769,10 @@ def run_closure(args):
            "data": "synthetic",
            "config": {"workload": args.workload, "rows": nc, "layers": list(d), "train_batch": batch,
                       "l2": "features (%.0f MB) larger than L2" % (nc * C.XPAD * 2 / 1e6)},
-           # a training step: 4 weight transposes, 4 GEMMs forward and 7 backward (k_gemm_bf16; the
-           # weight gradients add a split-K partial sum each), 4 bias/GELU, loss, 4 column sums,
-           # 3 GELU backward, 8 Adam
+           # a training step: 4 products forward (bias and GELU in their epilogue), loss, 4 weight
+           # gradients, 3 products backward (GELU backward in theirs), one update of every tensor
            "training": {"rows_per_s": batch * world / (tr_ms / 1e3), "ms_per_step": tr_ms, "tflops": tr_tf,
-                        "own_kernels_per_step": 39},
+                        "own_kernels_per_step": 13},
            "inference_per_layer_gemms": {"ms": gemm_ms, "rows_per_s": nc * world / (gemm_ms / 1e3)},
            "inference_fused_mma_sync": {"ms": other_ms["mma"], "rows_per_s": nc * world / (other_ms["mma"] / 1e3)},
            "kernel": "k_mlp_tc (one launch: weights in shared memory, 128-row tiles, tcgen05.mma kind::f16 with "
