@@ -1,7 +1,7 @@
 // css_fused.cuh -- the RK stage in two passes over HBM.  The plane pass takes
 // theta and phi blocks of 16 or 32 points and FP64 or FP32 stage states; the
-// slab pass here takes 32-point blocks in r and theta, FP64 RK4 stages and
-// closed radial faces (css_stage.cuh has the others; css_create and
+// slab pass here takes 32-point blocks in r and theta, RK4 stages of either
+// storage and closed radial faces (css_stage.cuh has the others; css_create and
 // launch_stage_two decide).
 //
 //   k_thph    tiles of 32 theta x 32 phi of one radius (one or two blocks in

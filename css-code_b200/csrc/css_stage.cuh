@@ -13,7 +13,8 @@
 // global reads (238 bytes a cell hydro, 376 MHD in FP64).  Per stage,
 // measured against the radial and update kernels: 100x176x304 in blocks of
 // 20 radii 696 -> 379 us, open faces on 64x128x256 209 -> 162 us, FP32 stage
-// states of MHD 128x128x256 650 -> 543 us.  Reading the lines from global
+// states of MHD 128x128x256 650 -> 540 us (434 in k_rstage, which takes
+// 32-point blocks).  Reading the lines from global
 // memory instead of a TMA slab took 436 us on the first of them.
 #pragma once
 #include "css_deriv.cuh"
@@ -48,7 +49,7 @@ struct RIdx {
 __host__ __device__ constexpr size_t stage_smem(int mag, int m, int ts) {
   return (size_t)32 * (m + 8) * (5 * ts + (mag ? 16 : 0)) + 8 * ((size_t)(mag ? 8 : 6) * m * 32 + 32 + 1);
 }
-constexpr size_t SG_SMEM = 227 * 1024;  // a run whose FP64 slab and tiles are larger keeps the four-kernel stage
+constexpr size_t SG_SMEM = 227 * 1024;  // a stage whose slab and tiles are larger takes the four kernels
 
 // rows of 32 theta a warp takes at a time, and CTAs an SM (registers):
 // closed hydro slabs of short blocks leave room for three CTAs, the others
