@@ -116,6 +116,7 @@ struct css_ctx {
                                     // 2 one pass from TMA-staged planes (k_curl_pl) where the maps exist
   int nsm = 148;                    // SMs of the device
   cudaStream_t own_stream;
+  unsigned long long cfg = 0;       // raised by every call that changes what a step launches or passes by value
   // per-kernel event timing (css_profile)
   int profiling;
   std::vector<cudaEvent_t> ev;     // pairs (start, stop)
@@ -2218,6 +2219,7 @@ extern "C" int css_autotune(css_ctx *c, int reps, int *chosen) {
 // the autotuner's choices set by hand: tile heights (lines per CTA) of the
 // r, theta and phi kernels and the persistent phi kernel (0/1); a height a
 // direction does not offer is refused
+  c->cfg++;
 extern "C" int css_set_fused(css_ctx *c, int on) {
   if (!c) { set_err("css_set_fused: NULL"); return CSS_ERR_ARG; }
   if (on && !c->fused_ok) {
@@ -2237,6 +2239,7 @@ extern "C" int css_set_tiles(css_ctx *c, int tl_r, int tl_theta, int tl_phi, int
   const int tl[3] = {tl_r, tl_theta, tl_phi};
   const int mag = c->g.magnetic;
   for (int d = 0; d < 3; d++) {
+  c->cfg++;
     const int t = tl[d], m = c->g.d[d].maxm;
     bool ok = c->mt[d] ? (t == 8 || t == 16) : (t == 4 || t == 8 || t == 16);
     if (ok && !c->mt[d]) {
@@ -2258,12 +2261,16 @@ extern "C" int css_set_curl_pass(css_ctx *c, int mode) {
 }
 
 // ---------------------------------------------------------------------------
+  c->cfg++;
 // Batched ensemble: one RK4 step of every member is captured once into a
 // CUDA graph (each member's kernels on a stream of its own, forked from and
 // joined to the ensemble's root stream, so small members run side by side)
 // and the graph is replayed for every step.  Members keep their own state,
 // parameters and tables; the graph is captured again when a time step
-// changes.
+// changes, or a member's choice of kernels or attached speed^2 (its cfg): a
+// captured launch holds both by value, the speed^2 as a pointer its owner may
+// have freed since.
+  c->cfg++;
 // ---------------------------------------------------------------------------
 struct css_ensemble {
   std::vector<css_ctx *> m;
@@ -2280,6 +2287,7 @@ struct css_ensemble {
 };
 
 extern "C" void css_ensemble_destroy(css_ensemble *e) {
+  std::vector<unsigned long long> cfg;  // the members' cfg at capture
   if (!e) return;
   if (e->exec) cudaGraphExecDestroy(e->exec);
   if (e->graph) cudaGraphDestroy(e->graph);
@@ -2371,7 +2379,9 @@ extern "C" int css_ensemble_step(css_ensemble *e, const double *dt, int nsteps) 
   for (int i = 0; i < nm; i++)
     if (!(dt[i] > 0.0)) { set_err("css_ensemble_step: dt[%d] must be positive", i); return CSS_ERR_ARG; }
   bool same = e->exec != nullptr;
-  for (int i = 0; i < nm && same; i++) same = (e->dt[i] == dt[i]);
+  e->cfg.resize(nm);
+  for (int i = 0; i < nm; i++) e->cfg[i] = e->m[i]->cfg;
+  for (int i = 0; i < nm && same; i++) same = e->dt[i] == dt[i] && e->cfg[i] == e->m[i]->cfg;
   // order after whatever each member's own stream has queued (uploads)
   for (int i = 0; i < nm; i++) {
     CUDA_TRY(cudaEventRecord(e->join[i], e->m[i]->stream));
@@ -2626,6 +2636,7 @@ extern "C" int css_box_filter(css_ctx *c, int f, double *fields, double *targets
     return CSS_ERR_ARG;
   }
   const size_t n = c->ncell;
+  if (c->g.speed2 != speed2) c->cfg++;
   if (c->g.magnetic)
     if (int rc = launch_curl(c, (const double *)(c->v0 + 5 * n), c->bf, 1)) return rc;
   k_box_filter<<<148 * 8, 256, 0, c->stream>>>(c->g, c->v0, c->g.magnetic ? c->bf : nullptr, f, c->p.nth / f,

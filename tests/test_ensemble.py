@@ -175,6 +175,60 @@ def test_ensemble_step_equals_members_stepped_alone(gpu_available):
 
 
 @pytest.mark.gpu
+def test_settings_changed_after_the_capture(gpu_available):
+    """A speed^2 attached, replaced and detached (its tensor freed) and another
+    form of the stage, the curl and the tiles between steps of one dt: the
+    ensemble follows each, bit for bit as the members stepped alone."""
+    import torch
+    from css_b200 import closure as C
+    from css_b200.context import Simulation
+    specs = [dict(nr=32, nth=32, nphi=48, ra=1e5, ro=0.7, magnetic=mag, pm=2.0, decomp=(2, 2, 3))
+             for mag in (False, True)]
+    members = [E.build_member(s, seed=41 + i) for i, s in enumerate(specs)]
+    n = 32 * 32 * 48
+    # both below the prescribed speed^2, which this dt is stable for
+    level = min((m[0].sld_speedh + m[0].sld_speedr) ** 2 for m in members)
+    s2 = [torch.full((n,), f * level, dtype=torch.float64, device="cuda") for f in (0.01, 0.1)]
+    torch.cuda.synchronize()
+
+    def settings(k, sims):
+        if k == 1:
+            C.Closure.attach(sims[0], s2[0])
+            sims[1].set_curl_pass(0)
+        elif k == 2:
+            C.Closure.attach(sims[0], s2[1])
+            sims[1].set_tiles(8, 8, 8)
+        elif k == 3:
+            C.Closure.attach(sims[0], None)
+            sims[1].set_fused(False)
+
+    final = []
+    for together in (False, True):
+        sims = [Simulation(p, prof) for p, prof, _, _ in members]
+        for sim, (_, _, v0, _) in zip(sims, members):
+            sim.upload(v0)
+        ens = E.Ensemble(sims)
+        states = []
+        for k in range(4):
+            settings(k, sims)
+            if together:
+                ens.step([m[3] for m in members], 1)
+            else:
+                for sim, m in zip(sims, members):
+                    sim.step_rk4(m[3], 1)
+            states.append([sim.download() for sim in sims])
+        ens.close()
+        for sim in sims:
+            sim.close()
+        final.append(states)
+    for k in range(4):
+        for a, b in zip(final[0][k], final[1][k]):
+            assert np.array_equal(a, b), k
+    # the attached speed^2 did act
+    assert not np.array_equal(final[0][1][0], final[0][2][0])
+
+
+@pytest.mark.gpu
 def test_ensemble_member_matches_oracle(gpu_available):
     from css_b200.context import Simulation
     from oracle import oracle as O
