@@ -115,8 +115,8 @@ struct css_ctx {
   int curl_tp = 2;                  // B = curl A's theta and phi parts: 0 two passes, 1 one pass (k_curl_tp),
                                     // 2 one pass from TMA-staged planes (k_curl_pl) where the maps exist
   int nsm = 148;                    // SMs of the device
-  cudaStream_t own_stream;
   unsigned long long cfg = 0;       // raised by every call that changes what a step launches or passes by value
+  cudaStream_t own_stream;
   // per-kernel event timing (css_profile)
   int profiling;
   std::vector<cudaEvent_t> ev;     // pairs (start, stop)
@@ -2209,6 +2209,7 @@ extern "C" int css_autotune(css_ctx *c, int reps, int *chosen) {
     *tl[d] = best;
     if (d == 2) c->phi_pers = best_pers;
   }
+  c->cfg++;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c->profiling = prof_was;
@@ -2219,7 +2220,6 @@ extern "C" int css_autotune(css_ctx *c, int reps, int *chosen) {
 // the autotuner's choices set by hand: tile heights (lines per CTA) of the
 // r, theta and phi kernels and the persistent phi kernel (0/1); a height a
 // direction does not offer is refused
-  c->cfg++;
 extern "C" int css_set_fused(css_ctx *c, int on) {
   if (!c) { set_err("css_set_fused: NULL"); return CSS_ERR_ARG; }
   if (on && !c->fused_ok) {
@@ -2229,6 +2229,7 @@ extern "C" int css_set_fused(css_ctx *c, int on) {
   }
   c->fused = on ? 1 : 0;
   c->two = c->fused;  // off: the four-kernel stage
+  c->cfg++;
   return CSS_OK;
 }
 
@@ -2239,7 +2240,6 @@ extern "C" int css_set_tiles(css_ctx *c, int tl_r, int tl_theta, int tl_phi, int
   const int tl[3] = {tl_r, tl_theta, tl_phi};
   const int mag = c->g.magnetic;
   for (int d = 0; d < 3; d++) {
-  c->cfg++;
     const int t = tl[d], m = c->g.d[d].maxm;
     bool ok = c->mt[d] ? (t == 8 || t == 16) : (t == 4 || t == 8 || t == 16);
     if (ok && !c->mt[d]) {
@@ -2251,17 +2251,18 @@ extern "C" int css_set_tiles(css_ctx *c, int tl_r, int tl_theta, int tl_phi, int
   }
   if (phi_persistent && !c->mt[2]) { set_err("css_set_tiles: the persistent phi kernel needs 16- or 32-point blocks"); return CSS_ERR_ARG; }
   c->tl_r = tl_r; c->tl_theta = tl_theta; c->tl_phi = tl_phi; c->phi_pers = phi_persistent ? 1 : 0;
+  c->cfg++;
   return CSS_OK;
 }
 
 extern "C" int css_set_curl_pass(css_ctx *c, int mode) {
   if (!c || mode < 0 || mode > 2) { set_err("css_set_curl_pass: NULL context or mode not 0..2"); return CSS_ERR_ARG; }
   c->curl_tp = mode;
+  c->cfg++;
   return CSS_OK;
 }
 
 // ---------------------------------------------------------------------------
-  c->cfg++;
 // Batched ensemble: one RK4 step of every member is captured once into a
 // CUDA graph (each member's kernels on a stream of its own, forked from and
 // joined to the ensemble's root stream, so small members run side by side)
@@ -2270,13 +2271,13 @@ extern "C" int css_set_curl_pass(css_ctx *c, int mode) {
 // changes, or a member's choice of kernels or attached speed^2 (its cfg): a
 // captured launch holds both by value, the speed^2 as a pointer its owner may
 // have freed since.
-  c->cfg++;
 // ---------------------------------------------------------------------------
 struct css_ensemble {
   std::vector<css_ctx *> m;
   std::vector<cudaStream_t> ms;
   std::vector<cudaEvent_t> join;
   std::vector<double> dt;
+  std::vector<unsigned long long> cfg;  // the members' cfg at capture
   cudaStream_t root = nullptr;
   cudaEvent_t fork = nullptr;
   cudaGraph_t graph = nullptr;
@@ -2287,7 +2288,6 @@ struct css_ensemble {
 };
 
 extern "C" void css_ensemble_destroy(css_ensemble *e) {
-  std::vector<unsigned long long> cfg;  // the members' cfg at capture
   if (!e) return;
   if (e->exec) cudaGraphExecDestroy(e->exec);
   if (e->graph) cudaGraphDestroy(e->graph);
@@ -2369,6 +2369,8 @@ static int ensemble_capture(css_ensemble *e, const double *dt) {
   e->graph = g;
   CUDA_TRY(cudaGraphInstantiate(&e->exec, e->graph, 0));
   e->dt.assign(dt, dt + nm);
+  e->cfg.resize(nm);
+  for (int i = 0; i < nm; i++) e->cfg[i] = e->m[i]->cfg;
   e->launches_per_step = l1;
   return CSS_OK;
 }
@@ -2379,8 +2381,6 @@ extern "C" int css_ensemble_step(css_ensemble *e, const double *dt, int nsteps) 
   for (int i = 0; i < nm; i++)
     if (!(dt[i] > 0.0)) { set_err("css_ensemble_step: dt[%d] must be positive", i); return CSS_ERR_ARG; }
   bool same = e->exec != nullptr;
-  e->cfg.resize(nm);
-  for (int i = 0; i < nm; i++) e->cfg[i] = e->m[i]->cfg;
   for (int i = 0; i < nm && same; i++) same = e->dt[i] == dt[i] && e->cfg[i] == e->m[i]->cfg;
   // order after whatever each member's own stream has queued (uploads)
   for (int i = 0; i < nm; i++) {
@@ -2626,6 +2626,7 @@ extern "C" int css_spectrum(css_ctx *c, int kind, double *out) {
 // ---------------------------------------------------------------------------
 extern "C" int css_set_sld_speed2(css_ctx *c, const double *speed2) {
   if (!c) { set_err("css_set_sld_speed2: NULL context"); return CSS_ERR_ARG; }
+  if (c->g.speed2 != speed2) c->cfg++;
   c->g.speed2 = speed2;
   return CSS_OK;
 }
@@ -2636,7 +2637,6 @@ extern "C" int css_box_filter(css_ctx *c, int f, double *fields, double *targets
     return CSS_ERR_ARG;
   }
   const size_t n = c->ncell;
-  if (c->g.speed2 != speed2) c->cfg++;
   if (c->g.magnetic)
     if (int rc = launch_curl(c, (const double *)(c->v0 + 5 * n), c->bf, 1)) return rc;
   k_box_filter<<<148 * 8, 256, 0, c->stream>>>(c->g, c->v0, c->g.magnetic ? c->bf : nullptr, f, c->p.nth / f,
