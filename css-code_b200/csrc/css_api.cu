@@ -78,6 +78,7 @@ struct css_ctx {
   // adjoints of css_deriv (torch backward): edge-row tables of the blocks per
   // (direction, order, bdry), built on first use
   double *adjE[3][2][5] = {};
+  std::mutex adj_mu;                // their first use (autograd calls the backward from threads of its own)
   PlaneMaps pmaps[5];               // two-pass stage: TMA maps of v0, vA, vB, bf (plane kernel) and vs (curl)
   int vs_map = 0;                   // pmaps[4] and vs_slab hold vs's maps
   SlabMaps vs_slab;
@@ -1815,6 +1816,7 @@ extern "C" int css_dbydp_cyclic(css_ctx *c, const double *x, double *dx, int ord
 // unit inputs (zero boundary data)
 static int adjoint_tables(css_ctx *c, int dir, int order, int bdry) {
   const int ob = dir == 2 ? 0 : bdry;
+  std::lock_guard<std::mutex> lock(c->adj_mu);
   if (c->adjE[dir][order - 1][ob]) return CSS_OK;
   const CssDir &D = c->g.d[dir];
   std::vector<double> E((size_t)D.nb * ADJ_TAB, 0.0);
@@ -1851,9 +1853,17 @@ static int adjoint_tables(css_ctx *c, int dir, int order, int bdry) {
     set_err("css_deriv_adjoint: device allocation failed");
     return CSS_ERR_NOMEM;
   }
-  if (cudaMemcpy(dE, E.data(), E.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
+  // on the device before any stream's kernel can read it: a copy from pageable
+  // memory may return once the data is staged, and nothing orders the caller's
+  // stream behind it, so the host waits for the stream it went up on
+  cudaStream_t up = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking);
+  if (!e) e = cudaMemcpyAsync(dE, E.data(), E.size() * 8, cudaMemcpyHostToDevice, up);
+  if (!e) e = cudaStreamSynchronize(up);
+  if (up) cudaStreamDestroy(up);
+  if (e) {
     cudaFree(dE);
-    set_err("css_deriv_adjoint: table copy failed");
+    set_err("css_deriv_adjoint: table copy: %s", cudaGetErrorString(e));
     return CSS_ERR_CUDA;
   }
   c->adjE[dir][order - 1][ob] = dE;

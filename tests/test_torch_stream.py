@@ -30,3 +30,38 @@ def test_default_stream_orders_with_torch(gpu_available):
         assert torch.equal(got, want)
     del b
     sim.close()
+
+
+@pytest.mark.parametrize("direction", [0, 1, 2])
+def test_first_backward_on_a_side_stream(direction, gpu_available):
+    """The first adjoint of a (direction, order, closure) makes its tables:
+    they are on the device before the kernel that reads them, on any stream and
+    with several threads calling first at once.  The same bits as a second
+    call."""
+    import threading
+    import torch
+    from css_b200 import torch_ops  # noqa: F401
+    p, prof, _, _, _ = problem.build((32, 48, 60), decomp=(2, 2, 3))
+    g = torch.randn(p.nr, p.nphi, p.nth, generator=torch.Generator().manual_seed(5), dtype=torch.float64).cuda()
+    torch.cuda.synchronize()
+    for order in (1, 2):
+        for bdry in (range(5) if direction < 2 else (0,)):
+            sim = Simulation(p, prof)
+            first = [None] * 4
+
+            def call(k):
+                s = torch.cuda.Stream()
+                with torch.cuda.stream(s):
+                    first[k] = torch.ops.css.deriv_adjoint(g, sim.h.value, direction, order, bdry)
+                s.synchronize()
+
+            threads = [threading.Thread(target=call, args=(k,)) for k in range(4)]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            again = torch.ops.css.deriv_adjoint(g, sim.h.value, direction, order, bdry)
+            torch.cuda.synchronize()
+            for a in first:
+                assert torch.equal(a, again), (order, bdry)
+            sim.close()
