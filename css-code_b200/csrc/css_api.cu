@@ -987,6 +987,14 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   c->maps = c->two && plane_maps(c);
   if (!c->maps) c->two = c->fused_ok = 0;
   c->fused = c->fused_ok;
+  // the backgrounds' zeros and the cyclic tables went up on the legacy stream,
+  // which the run's and its callers' non-blocking streams do not wait for
+  e = cudaStreamSynchronize(cudaStreamLegacy);
+  if (e != cudaSuccess) {
+    set_err("css_create: %s", cudaGetErrorString(e));
+    css_destroy(c);
+    return CSS_ERR_CUDA;
+  }
   *out = c;
   return CSS_OK;
 }
@@ -2902,17 +2910,18 @@ extern "C" int css_mlp_create(int n_in, int width, int n_out, int max_rows, unsi
         const double u = next();
         if (k < kr && j < mr) w[(size_t)k * M + j] = (float)(a * (2.0 * u - 1.0));
       }
-    if (!e) e = cudaMemcpy(m->W[l], w.data(), w.size() * 4, cudaMemcpyHostToDevice);
+    // on the network's stream, in front of the kernel that reads them
+    if (!e) e = cudaMemcpyAsync(m->W[l], w.data(), w.size() * 4, cudaMemcpyHostToDevice, m->st);
     for (float *p : {m->mW[l], m->vW[l]})
-      if (!e) e = cudaMemcpy(p, z.data(), z.size() * 4, cudaMemcpyHostToDevice);
+      if (!e) e = cudaMemcpyAsync(p, z.data(), z.size() * 4, cudaMemcpyHostToDevice, m->st);
     for (float *p : {m->B[l], m->mB[l], m->vB[l]})
-      if (!e) e = cudaMemcpy(p, zb.data(), zb.size() * 4, cudaMemcpyHostToDevice);
+      if (!e) e = cudaMemcpyAsync(p, zb.data(), zb.size() * 4, cudaMemcpyHostToDevice, m->st);
     if (!e) {
       k_to_bf16<<<64, 256, 0, m->st>>>(m->W[l], m->Wb[l], (size_t)K * M);
       e = cudaGetLastError();
     }
+    if (!e) e = cudaStreamSynchronize(m->st);
   }
-  if (!e) e = cudaStreamSynchronize(m->st);
   if (e) {
     set_err("css_mlp_create: %s", cudaGetErrorString(e));
     css_mlp_destroy(m);
@@ -3080,8 +3089,8 @@ extern "C" int css_mlp_params(css_mlp *m, int l, float *w, float *b, int set) {
   if (!m || l < 0 || l > 3) { set_err("css_mlp_params: bad argument"); return CSS_ERR_ARG; }
   const size_t K = m->dims[l], M = m->dims[l + 1];
   if (set) {
-    if (w) CUDA_TRY(cudaMemcpy(m->W[l], w, K * M * 4, cudaMemcpyHostToDevice));
-    if (b) CUDA_TRY(cudaMemcpy(m->B[l], b, M * 4, cudaMemcpyHostToDevice));
+    if (w) CUDA_TRY(cudaMemcpyAsync(m->W[l], w, K * M * 4, cudaMemcpyHostToDevice, m->st));
+    if (b) CUDA_TRY(cudaMemcpyAsync(m->B[l], b, M * 4, cudaMemcpyHostToDevice, m->st));
     k_to_bf16<<<64, 256, 0, m->st>>>(m->W[l], m->Wb[l], K * M);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(m->st));

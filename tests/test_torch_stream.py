@@ -65,3 +65,38 @@ def test_first_backward_on_a_side_stream(direction, gpu_available):
             for a in first:
                 assert torch.equal(a, again), (order, bdry)
             sim.close()
+
+
+def test_host_data_is_in_place_before_the_first_kernel(gpu_available):
+    """What a call sends up from host memory is there for the first kernel that
+    reads it: the cyclic derivative right after a run is made, and the network's
+    BF16 weights right after its parameters are set, each equal to a second
+    call after the device has come to rest."""
+    import ctypes
+    import numpy as np
+    import torch
+    from css_b200 import _lib
+    from css_b200 import closure as C
+    p, prof, _, _, _ = problem.build((20, 32, 48), decomp=(2, 2, 3))
+    x = torch.randn(p.nr, p.nphi, p.nth, generator=torch.Generator().manual_seed(7), dtype=torch.float64).cuda()
+    net = C.Mlp(135, 128, 12, max_rows=64, seed=3)
+    net.set_forward("gemm")
+    xr = torch.randn(64, 144, generator=torch.Generator().manual_seed(8)).to(torch.bfloat16).cuda()
+    rng = np.random.default_rng(2)
+    torch.cuda.synchronize()
+    for k in range(8):
+        sim, out = Simulation(p, prof), [torch.empty_like(x) for _ in range(2)]
+        s = torch.cuda.Stream()
+        for o in out:
+            _lib.check(_lib.lib().css_dbydp_cyclic_dev(sim.h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(o.data_ptr()),
+                                                       2, ctypes.c_void_p(s.cuda_stream)))
+            torch.cuda.synchronize()
+        assert torch.equal(out[0], out[1]), k
+        sim.close()
+        for l in range(4):
+            kk, m = net.dims[l], net.dims[l + 1]
+            net.set_params(l, rng.standard_normal((kk, m)) * 0.1, rng.standard_normal(m) * 0.1)
+        a = net.forward(xr, 64)
+        torch.cuda.synchronize()
+        assert torch.equal(a, net.forward(xr, 64)), k
+    net.close()
