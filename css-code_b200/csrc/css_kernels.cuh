@@ -1501,14 +1501,15 @@ __global__ void k_sld_vcc(CssGeo g, const double *__restrict__ v, const double *
 // limited value is 0 (opposite signs), q (|qph| >= |q|) or qph: a minmod,
 // evaluated without the division (equal to the reference's product to within
 // its roundings); below tiny the formula as written, k = qph / tiny^2 in
-// hand.  Selections only: lanes on either side of tiny do not diverge.
+// hand.  Selections only: lanes on either side of tiny do not diverge.  The
+// zero is q * 0: an infinite or NaN q gives NaN there, as the product with the
+// limited ratio does, so a face beside a non-finite cell is not finite.
 __device__ __forceinline__ double sld_limiter(double q, double qph, double k, double tiny) {
   const double kq = q * k;
   const bool big = fabs(q) >= tiny;
   const bool whole = big ? fabs(qph) >= fabs(q) : __double2hiint(kq) >= 0x3FF00000;  // kq >= 1
   const double part = big ? qph : q * kq;
-  const double r = whole ? q : part;
-  return (__double2hiint(q) ^ __double2hiint(qph)) < 0 ? 0.0 : r;
+  return kq > 0.0 ? (whole ? q : part) : q * 0.0;
 }
 
 // limited face difference delta at the face whose neighbours are
