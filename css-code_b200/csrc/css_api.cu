@@ -108,8 +108,8 @@ struct css_ctx {
   int tl_theta, tl_phi, tl_r;
   int phi_pers = 0;                 // 1: persistent double-buffered phi kernel (autotuned)
   int fused_ok = 0;                 // the run qualifies for the two-pass RK4 stage of 32-point blocks (css_fused.cuh)
-  int fused = 0;                    // 1: FP64 RK4 stages run k_thph + k_rstage
-  int two = 0;                      // 1: the other stages run k_thph + k_rstage_g (css_stage.cuh)
+  int two_ok = 0;                   // it qualifies for that form or the general one (css_stage.cuh)
+  int two = 0;                      // 1: the stages run in two passes (launch_stage_two)
   int maps = 0;                     // the TMA maps of the FP64 state buffers exist
   PlaneMaps fmaps[2];               // vA, vB as FP32 stage states (mixed precision)
   SlabMaps fslab[2];
@@ -970,8 +970,8 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   // any radial block whose slab fits shared memory, either storage of the
   // stage states, any stepper, open radial faces and explicit viscosity; radiative
   // diffusion alone sits between the radial terms and the update
-  c->two = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, p.precision ? 4 : 8) <= SG_SMEM && !p.do_radheat;
-  if (c->two) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
+  c->two_ok = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, p.precision ? 4 : 8) <= SG_SMEM && !p.do_radheat;
+  if (c->two_ok) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
   if (p.precision == 1) {  // backgrounds of the FP32 stage states, refreshed at every upload
     ALLOC(c->bg2, 2 * (size_t)nr * nth * sizeof(double));
     cudaMemset(c->bg2, 0, 2 * (size_t)nr * nth * sizeof(double));
@@ -984,9 +984,9 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
     ALLOC(c->cyc, CY.size() * sizeof(double));
     cudaMemcpy(c->cyc, CY.data(), CY.size() * sizeof(double), cudaMemcpyHostToDevice);
   }
-  c->maps = c->two && plane_maps(c);
-  if (!c->maps) c->two = c->fused_ok = 0;
-  c->fused = c->fused_ok;
+  c->maps = c->two_ok && plane_maps(c);
+  if (!c->maps) c->two_ok = c->fused_ok = 0;
+  c->two = c->two_ok;
   // the backgrounds' zeros and the cyclic tables went up on the legacy stream,
   // which the run's and its callers' non-blocking streams do not wait for
   e = cudaStreamSynchronize(cudaStreamLegacy);
@@ -2235,24 +2235,33 @@ extern "C" int css_autotune(css_ctx *c, int reps, int *chosen) {
   return rc;
 }
 
-// the autotuner's choices set by hand: tile heights (lines per CTA) of the
-// r, theta and phi kernels and the persistent phi kernel (0/1); a height a
-// direction does not offer is refused
+// the form of the stage: 0 four kernels, 1 two passes of 32-point blocks, 2
+// two passes in whichever form the run qualifies for
 extern "C" int css_set_fused(css_ctx *c, int on) {
   if (!c) { set_err("css_set_fused: NULL"); return CSS_ERR_ARG; }
-  if (on && !c->fused_ok) {
+  if (on == 2 && !c->two_ok) {
+    set_err("css_set_fused: two passes need theta and phi blocks of 16 or 32 points, a radial block whose slab "
+            "fits shared memory and no radiative diffusion");
+    return CSS_ERR_ARG;
+  }
+  if (on && on != 2 && !c->fused_ok) {
     set_err("css_set_fused: the two-pass stage needs 32-point blocks in r, theta and phi and an FP64 RK4 run "
             "with closed radial faces, no explicit viscosity, radiative diffusion or prescribed bottom");
     return CSS_ERR_ARG;
   }
-  c->fused = on ? 1 : 0;
-  c->two = c->fused;  // off: the four-kernel stage
+  c->two = on ? 1 : 0;
   c->cfg++;
   return CSS_OK;
 }
 
-extern "C" int css_get_fused(css_ctx *c) { return c ? c->fused : -1; }
+extern "C" int css_get_fused(css_ctx *c) {
+  if (!c) return -1;
+  return c->two ? (c->fused_ok ? 1 : 2) : 0;
+}
 
+// the autotuner's choices set by hand: tile heights (lines per CTA) of the
+// r, theta and phi kernels and the persistent phi kernel (0/1); a height a
+// direction does not offer is refused
 extern "C" int css_set_tiles(css_ctx *c, int tl_r, int tl_theta, int tl_phi, int phi_persistent) {
   if (!c) { set_err("css_set_tiles: NULL"); return CSS_ERR_ARG; }
   const int tl[3] = {tl_r, tl_theta, tl_phi};

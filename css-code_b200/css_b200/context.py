@@ -131,9 +131,10 @@ class Simulation:
         return out
 
     def set_fused(self, on):
-        """Two-pass RK4 stage on or off (css_set_fused); on is refused for a
-        run that does not qualify."""
-        check(_lib.lib().css_set_fused(self.h, 1 if on else 0))
+        """Two-pass RK4 stage of 32-point blocks on or off (css_set_fused); on
+        is refused for a run that does not qualify.  2: two passes in whichever
+        form the run qualifies for."""
+        check(_lib.lib().css_set_fused(self.h, 2 if on == 2 else (1 if on else 0)))
 
     def set_curl_pass(self, mode):
         """B = curl A's theta and phi parts (css_set_curl_pass): 2 from
@@ -143,7 +144,14 @@ class Simulation:
 
     @property
     def fused(self):
-        return bool(_lib.lib().css_get_fused(self.h))
+        """The stages take the two passes of 32-point blocks."""
+        return self.stage_form == 1
+
+    @property
+    def stage_form(self):
+        """What the stages run (css_get_fused): 0 four kernels, 1 two passes of
+        32-point blocks, 2 the general two passes."""
+        return _lib.lib().css_get_fused(self.h)
 
     def set_tiles(self, tl_r, tl_theta, tl_phi, phi_persistent=False):
         """The autotuner's choices by hand (css_set_tiles)."""

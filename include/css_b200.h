@@ -370,11 +370,15 @@ int css_set_tiles(css_ctx *ctx, int tl_r, int tl_theta, int tl_phi, int phi_pers
  * explicit viscosity, radiative diffusion or prescribed bottom.
  * css_set_fused(ctx, 0) selects the four-kernel stage (same results to
  * rounding); css_set_fused(ctx, 1) on a run that does not qualify fails
- * with CSS_ERR_ARG.  css_get_fused returns the current choice.
+ * with CSS_ERR_ARG.
  * Other runs with theta and phi blocks of 16 or 32 points take the same two
  * passes in a general form (any radial block that fits, FP32 stage states,
- * open radial faces, explicit viscosity, the TVD schemes); css_set_fused(ctx,
- * 0) selects the four kernels for them too, and css_get_fused is 0.        */
+ * open radial faces, explicit viscosity, the TVD schemes).  css_set_fused(ctx,
+ * 0) selects the four kernels for them too; css_set_fused(ctx, 2) selects two
+ * passes in whichever form the run qualifies for, and fails with CSS_ERR_ARG
+ * where neither does.  css_get_fused returns the form in use: 0 four kernels,
+ * 1 the 32-point form, 2 the general one, so that css_set_fused(ctx, saved)
+ * restores what css_get_fused had returned.                                */
 int css_set_fused(css_ctx *ctx, int on);
 int css_get_fused(css_ctx *ctx);
 /* B = curl A (VectorCurlA, derivatives.f90:1769-1828) of magnetic runs,

@@ -84,6 +84,43 @@ def test_general_stage_equals_four_kernels(name, gpu_available):
         assert np.abs(two[i] - four_[i]).max() <= bar * np.abs(four_[i]).max(), (name, i)
 
 
+@pytest.mark.parametrize("dims,decomp,form,kw", [
+    ((40, 48, 80), (2, 3, 5), 2, {}), ((64, 64, 96), (2, 2, 3), 2, dict(precision=1)),
+    ((64, 64, 96), (2, 2, 3), 1, {}), ((40, 48, 72), (2, 2, 3), 0, {})])
+def test_form_is_put_back(dims, decomp, form, kw, gpu_available):
+    """Switched off and set back to what it was, every run steps in the form it
+    had, bit for bit; what a run does not qualify for is refused."""
+    from css_b200 import _lib
+    from css_b200._lib import CssError
+    p, prof, v0, dt, _ = problem.build(dims, decomp=decomp)
+    for k, val in kw.items():
+        setattr(p, k, val)
+    sims = [Simulation(p, prof) for _ in range(2)]
+    was = _lib.lib().css_get_fused(sims[1].h)
+    assert was == form == sims[1].stage_form and sims[1].fused == (form == 1)
+    sims[1].set_fused(False)
+    assert sims[1].stage_form == 0 and not sims[1].fused
+    if form != 1:
+        with pytest.raises(CssError):
+            sims[1].set_fused(True)
+    if form == 0:
+        with pytest.raises(CssError):
+            sims[1].set_fused(2)
+    else:
+        sims[1].set_fused(2)
+        assert sims[1].stage_form == form
+        sims[1].set_fused(False)
+    _lib.check(_lib.lib().css_set_fused(sims[1].h, was))
+    assert sims[1].stage_form == form
+    for sim in sims:
+        sim.upload(v0)
+        sim.step_rk4(dt, 2)
+    assert np.array_equal(sims[0].download(), sims[1].download())
+    assert sims[0].launches() == sims[1].launches()
+    for sim in sims:
+        sim.close()
+
+
 @pytest.mark.parametrize("nr", [44, 100, 200])  # radial blocks of 22, 50 and 100 points
 @pytest.mark.parametrize("perfect", [0, 1])
 def test_curl_of_any_radial_block(nr, perfect, gpu_available):
