@@ -308,6 +308,17 @@ def run_reference_ensemble(args, world):
     return 0
 
 
+# Simulation.stage_form in words
+STAGE_FORMS = {0: "four-kernel", 1: "two-pass (k_thph + k_rstage)",
+               2: "two-pass, general form (k_thph + k_rstage / k_rstage_g)"}
+
+
+def sweep_tiles(sim):
+    """Lines per CTA of the four-kernel stage's sweeps, the fastest of those
+    timed (no result changes); two-pass stages have fixed tiles."""
+    return (0, 0, 0) if sim.stage_form else sim.autotune(reps=3)
+
+
 def run_ours(args):
     import numpy as np
     import torch
@@ -328,9 +339,7 @@ def run_ours(args):
     stream = torch.cuda.current_stream(dev)
     sim.set_stream(stream.cuda_stream)
     sim.upload(v0)
-    # lines per CTA of the four-kernel stage's sweeps (no result changes);
-    # the two-pass stage has fixed tiles
-    tiles = (0, 0, 0) if sim.fused else sim.autotune(reps=3)
+    tiles = sweep_tiles(sim)
     for _ in range(args.warmup):
         sim.step_rk4(dt, 1)
     torch.cuda.synchronize()
@@ -420,7 +429,7 @@ def run_ours(args):
         "dtype": "f64" if args.precision == "fp64" else "f32-storage/f64", "data": "synthetic",
         "config": {"workload": args.workload, "grid": [p.nr, p.nth, p.nphi], "decomposition": [p.nnr, p.nnt, p.nnp],
                    "precision": args.precision, "tile_lines_r_theta_phi": list(tiles),
-                   "stage": "two-pass (k_thph + k_rstage)" if sim.fused else "four-kernel",
+                   "stage": STAGE_FORMS[sim.stage_form],
                    "fields": nv, "dt": dt, "l2": "state (%.0f MB per buffer) larger than L2, no flush" % (state_bytes / 1e6),
                    "parallelism": "replicas" if world > 1 else "single-gpu"},
         "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": state_bytes, "d2h_bytes_per_step": state_bytes,

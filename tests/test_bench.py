@@ -46,3 +46,24 @@ def test_byte_model():
     # the update kernel, averaged over the four stages
     assert bench.kernel_alg_bytes("rhot_update", 5) == 8.0 * (3 + 15 + 35 / 4.0)
     assert bench.kernel_alg_bytes("no_such_kernel", 5) is None
+
+
+def test_stage_of_the_run():
+    """The line names the form the run's stages take, and only runs of the
+    four-kernel form have their tiles timed (a mixed run takes two passes)."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    class Run:
+        def __init__(self, form):
+            self.stage_form, self.fused, self.tuned = form, form == 1, 0
+
+        def autotune(self, reps):
+            self.tuned += 1
+            return (16, 8, 16)
+
+    for form in (0, 1, 2):
+        run = Run(form)
+        assert bench.sweep_tiles(run) == ((0, 0, 0) if form else (16, 8, 16)) and run.tuned == (form == 0)
+        assert bench.STAGE_FORMS[form].startswith("two-pass" if form else "four-kernel")
+    assert len(set(bench.STAGE_FORMS.values())) == 3
