@@ -971,7 +971,12 @@ extern "C" int css_create(const css_params *pp, const double *prof, css_ctx **ou
   // stage states, any stepper, open radial faces and explicit viscosity; radiative
   // diffusion alone sits between the radial terms and the update
   c->two_ok = c->mt[1] && c->mt[2] && stage_smem(mag, g.d[0].maxm, p.precision ? 4 : 8) <= SG_SMEM && !p.do_radheat;
-  if (c->two_ok) ALLOC(c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double));
+  if (c->two_ok && cudaMalloc(&c->rtw, (size_t)nr * nphi * 2 * 32 * sizeof(double)) != cudaSuccess) {
+    // a run that fits without it takes the four kernels, which need no such buffer
+    cudaGetLastError();
+    c->rtw = nullptr;
+    c->two_ok = c->fused_ok = 0;
+  }
   if (p.precision == 1) {  // backgrounds of the FP32 stage states, refreshed at every upload
     ALLOC(c->bg2, 2 * (size_t)nr * nth * sizeof(double));
     cudaMemset(c->bg2, 0, 2 * (size_t)nr * nth * sizeof(double));

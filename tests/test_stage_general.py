@@ -121,6 +121,42 @@ def test_form_is_put_back(dims, decomp, form, kw, gpu_available):
         sim.close()
 
 
+def test_no_room_for_the_two_passes(gpu_available):
+    """A run that fits the device's memory but for the two passes' own buffer
+    is made all the same and steps through the four kernels: as a run switched
+    to them, bit for bit."""
+    import torch
+    p, prof, v0, dt, _ = problem.build((40, 32, 1024), decomp=(2, 2, 32))
+    rtw = p.nr * p.nphi * 64 * 8
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    sim = Simulation(p, prof)  # kernels of both forms loaded
+    sim.upload(v0)
+    sim.step_rk4(dt, 1)
+    sim.set_fused(False)
+    sim.upload(v0)
+    sim.step_rk4(dt, 2)
+    want = sim.download()
+    with_all = free()
+    sim.close()
+    need = free() - with_all
+    # leave what the run needs less half of that buffer
+    hog = torch.empty(free() - need + rtw // 2, dtype=torch.uint8, device="cuda")
+    try:
+        sim = Simulation(p, prof)
+        assert sim.stage_form == 0
+        sim.upload(v0)
+        sim.step_rk4(dt, 2)
+        assert np.array_equal(sim.download(), want)
+        sim.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("nr", [44, 100, 200])  # radial blocks of 22, 50 and 100 points
 @pytest.mark.parametrize("perfect", [0, 1])
 def test_curl_of_any_radial_block(nr, perfect, gpu_available):
