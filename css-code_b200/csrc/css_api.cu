@@ -1115,12 +1115,12 @@ static int launch_derivs(css_ctx *c, int dir, const DerivItem *it, int n, cudaSt
   for (int k = 0; k < n; k++) B.it[k] = it[k];
   const int nb = g.d[dir].nb, m = g.d[dir].maxm, mt = c->mt[dir];
   if (dir == 1) {
-    const int warps = 2 * 8 * dv_theta_warp(m) <= 200 * 1024 ? 2 : 1, nl = g.nphi * g.nr;
-    const size_t smem = (size_t)warps * dv_theta_warp(m) * 8;
-    const dim3 grid((nl + 32 * warps - 1) / (32 * warps), nb, n);
-    if (mt == 32) k_deriv_t<32><<<grid, 32 * warps, smem, st>>>(g, B);
-    else if (mt == 16) k_deriv_t<16><<<grid, 32 * warps, smem, st>>>(g, B);
-    else k_deriv_t<0><<<grid, 32 * warps, smem, st>>>(g, B);
+    const int tiles = mt ? 2 : 1, nl = g.nphi * g.nr;  // of 32 lines, a CTA
+    const size_t smem = (size_t)tiles * dv_theta_warp(m, mt > 0) * 8;
+    const dim3 grid((nl + 32 * tiles - 1) / (32 * tiles), nb, n);
+    if (mt == 32) k_deriv_t<32><<<grid, 64, smem, st>>>(g, B);
+    else if (mt == 16) k_deriv_t<16><<<grid, 64, smem, st>>>(g, B);
+    else k_deriv_t<0><<<grid, 128, smem, st>>>(g, B);
     return check_launch(c);
   }
   const int nl = dir == 0 ? g.nth * g.nphi : g.nth * g.nr;

@@ -2,11 +2,11 @@
 // the explicit viscosity and the radiative diffusion, torch.ops.css.deriv)
 // and their adjoints.
 //
-// Every kernel gives a line to a lane and 32 lines to a warp, and no warp
-// waits for another.  Along r and phi the 32 lines are consecutive theta, so
-// a lane reads its line straight from global memory (256 bytes a warp load)
-// into registers, solves it and stores it: nothing is staged.  Along theta a
-// warp transposes its 32 lines through a tile of its own.  These passes are
+// Every kernel gives a line to a lane and 32 lines to a warp.  Along r and phi
+// the 32 lines are consecutive theta, so a lane reads its line straight from
+// global memory (256 bytes a warp load) into registers, solves it and stores
+// it: nothing is staged.  Along theta a warp transposes its 32 lines through a
+// tile.  On large grids these passes are
 // bound by HBM (a field in, a field out: 268 MB, 41 us at 6550 GB/s on
 // 128x256x512).  Measured there, r / theta / phi: 63 / 88 / 45 us forward and
 // 53 / 76 / 63 us adjoint, against 297 / 235 / 253 us with 16-line tiles
@@ -51,10 +51,21 @@ struct GlobOut {
   __device__ __forceinline__ long long operator()(int j) const { return j * s; }
 };
 
+// 8 bytes from global to shared memory without a register between
+__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+// k / d of 0 <= k < 32 * 264 by a multiplication (inv = inv_of(d), d <= 264)
+__device__ __forceinline__ unsigned inv_of(int d) { return 0xFFFFFFFFu / (unsigned)d + 1u; }
+__device__ __forceinline__ int div_by(int k, unsigned inv) { return (int)__umulhi((unsigned)k, inv); }
+
 // A line of run-time length m >= 10: line_solve_a's arithmetic with the
 // forward values in a column of shared memory (t[j * ts], which may be the
-// output column itself) and the interior points read once, four ahead of the
-// row that needs them.
+// output column itself, or the input line where that is as dense: point j is
+// read before row j is written) and the interior points read once, four ahead
+// of the row that needs them.
 template <int ORDER, class P, class X, class O>
 __device__ __forceinline__ void line_solve_g(P xb, const X &xi, int m, int dtype, int bdry,
                                              double bclo, double bchi, const double *__restrict__ G, int gs,
@@ -74,17 +85,19 @@ __device__ __forceinline__ void line_solve_g(P xb, const X &xi, int m, int dtype
     rm1 = d2_row_hi1(xb, xi, m, dtype);
     rm = d2_row_hi2(xb, xi, m, dtype, bdry, bchi, dnum);
   }
+  double w[8];  // x(j-2) .. x(j+1) of the next row, then the four points after them
+#pragma unroll
+  for (int k = 0; k < 8; k++) w[k] = xb[xi(k + 1)];
   double v = __ldg(g2 + 1) * r1;
   t[0] = v;
   v = phi ? __ldg(g2 + 2) * (r2 + a1 * v) : __ldg(g2 + 2) * r2 + __ldg(g3 + 2) * v;
   t[ts] = v;
-  double w[8];  // x(j-2) .. x(j+1) of the next row, then the four points after them
-#pragma unroll
-  for (int k = 0; k < 8; k++) w[k] = xb[xi(k + 1)];
   for (int j = 3; j <= m - 2; j += 4) {
-    double nx[4];
+    double nx[4], c[4];  // c: the rows' coefficients (a table holds m + 2)
 #pragma unroll
     for (int k = 0; k < 4; k++) nx[k] = j + 6 + k <= m ? xb[xi(j + 6 + k)] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) c[k] = __ldg(g2 + j + k);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (j + k <= m - 2) {
@@ -92,7 +105,7 @@ __device__ __forceinline__ void line_solve_g(P xb, const X &xi, int m, int dtype
             ORDER == 1 ? (7.0 / 9.0) * (w[k + 3] - w[k + 1]) + (1.0 / 36.0) * (w[k + 4] - w[k])
                        : HaloD2::c1 * (w[k + 3] - 2.0 * w[k + 2] + w[k + 1]) +
                              HaloD2::c2 * (w[k] - 2.0 * w[k + 2] + w[k + 4]);
-        v = __ldg(g2 + j + k) * (d + a1 * v);
+        v = c[k] * (d + a1 * v);
         t[(j + k - 1) * ts] = v;
       }
     }
@@ -112,10 +125,20 @@ __device__ __forceinline__ void line_solve_g(P xb, const X &xi, int m, int dtype
     v = __ldg(g2 + m) * rm + __ldg(g3 + m) * v;
   }
   ob[oi(m - 1)] = scale * v;
-#pragma unroll 4
-  for (int j = m - 1; j >= 1; j--) {
-    v = t[(j - 1) * ts] + __ldg(g1 + j + 1) * v;
-    ob[oi(j - 1)] = scale * v;
+  for (int j0 = m - 1; j0 >= 1; j0 -= 4) {  // four rows' values in hand before the chain
+    double q[4], c[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int j = max(j0 - k, 1);
+      q[k] = t[(j - 1) * ts];
+      c[k] = __ldg(g1 + j + 1);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (j0 - k >= 1) {
+        v = q[k] + c[k] * v;
+        ob[oi(j0 - k - 1)] = scale * v;
+      }
   }
 }
 
@@ -164,25 +187,31 @@ __global__ void __launch_bounds__(DV_NT, M == 32 ? 3 : 4) k_deriv_s(CssGeo g, co
 
 // doubles of shared memory a warp's theta tile takes: 32 lines with their
 // halos, then 32 solved lines; both strides odd, so the 32 lanes of a solve
-// touch distinct banks
+// touch distinct banks.  Lines of run-time length are solved in place.
 __host__ __device__ constexpr int dv_theta_in(int m) { return (m + 8) | 1; }
 __host__ __device__ constexpr int dv_theta_out(int m) { return m | 1; }
-__host__ __device__ constexpr int dv_theta_warp(int m) { return 32 * (dv_theta_in(m) + dv_theta_out(m)); }
+__host__ __device__ constexpr int dv_theta_warp(int m, bool fixed) {
+  return 32 * (dv_theta_in(m) + (fixed ? dv_theta_out(m) : 0));
+}
 
-// Derivatives along theta.  grid: x = groups of 32 lines / warps, y = block,
-// z = derivative.  A line is a (phi, r) row; consecutive rows are contiguous
-// in memory.
+// Derivatives along theta.  grid: x = groups of 32 lines / tiles a CTA, y =
+// block, z = derivative.  A line is a (phi, r) row; consecutive rows are
+// contiguous in memory.  M > 0: a warp has its own tile, two a CTA.  M = 0: a
+// CTA of 128 threads brings one tile by asynchronous copies and stores it, its
+// first warp solves it in place: 21 us on 64x500x96 in theta blocks of 100
+// points and 16.5 us on 20x200x30, where a warp that loaded, solved into a
+// second tile and stored alone took 86 and 45 us.
 template <int M>
-__global__ void __launch_bounds__(64) k_deriv_t(CssGeo g, const __grid_constant__ DerivBatch B) {
+__global__ void __launch_bounds__(M > 0 ? 64 : 128) k_deriv_t(CssGeo g, const __grid_constant__ DerivBatch B) {
   extern __shared__ double sm[];
   const DerivItem &I = B.it[blockIdx.z];
   const CssDir &D = g.d[1];
   const int b = blockIdx.y, m = M > 0 ? M : D.size[b], t0 = D.start[b];
   const int lane = threadIdx.x & 31, nlines = g.nphi * g.nr, nth = g.nth;
-  const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+  const int row0 = (M > 0 ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x) * 32;
   if (row0 >= nlines) return;
   const int SI = dv_theta_in(m), SO = dv_theta_out(m), w = m + 8;
-  double *X = sm + (size_t)(threadIdx.x >> 5) * dv_theta_warp(M > 0 ? M : D.maxm), *O = X + 32 * SI;
+  double *X = sm + (M > 0 ? (size_t)(threadIdx.x >> 5) * dv_theta_warp(M, true) : 0), *O = X + 32 * SI;
   const double *src = I.x + (size_t)row0 * nth + t0 - 4;
   const int nrow = min(32, nlines - row0);
   if constexpr (M > 0) {
@@ -203,19 +232,22 @@ __global__ void __launch_bounds__(64) k_deriv_t(CssGeo g, const __grid_constant_
       }
     }
   } else {
-    for (int l = 0; l < nrow; l++)
-      for (int c = lane; c < w; c += 32) {
-        const int t = t0 - 4 + c;
-        X[l * SI + c] = t >= 0 && t < nth ? __ldg(src + (size_t)l * nth + c) : 0.0;
-      }
+    const unsigned inv = inv_of(w);
+    for (int k = threadIdx.x; k < nrow * w; k += blockDim.x) {
+      const int l = div_by(k, inv), c = k - l * w, t = t0 - 4 + c;
+      if (t >= 0 && t < nth) cp_async8(X + l * SI + c, src + (size_t)l * nth + c);
+      else X[l * SI + c] = 0.0;
+    }
+    cp_async_wait();
+    __syncthreads();
   }
   __syncwarp();
   const int row = row0 + lane;
-  if (row < nlines) {
+  if (row < nlines && (M > 0 || threadIdx.x < 32)) {
     const double lo = (D.lphys[b] && I.lo) ? __ldg(I.lo + row) : 0.0;
     const double hi = (D.rphys[b] && I.hi) ? __ldg(I.hi + row) : 0.0;
     const int dtype = dtype_of(D, b), ir = row / g.nphi;
-    const double *x = X + lane * SI + 4;
+    double *const x = X + lane * SI + 4;
     const double *G = tabp(g, 1, b, I.order, I.bdry);
     const double dn = D.dnum[b];
     // D2bydt2's Neumann datum takes the radial spacing
@@ -224,25 +256,31 @@ __global__ void __launch_bounds__(64) k_deriv_t(CssGeo g, const __grid_constant_
         line_solve_c<1, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, O + lane * SO,
                            StridedOut{1});
       else
-        line_solve<1>(x, 1, m, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, O + lane * SO, 1);
+        line_solve_g<1>((const double *)x, StridedIn{1}, m, dtype, I.bdry, lo, hi, G, g.tstride, dn, dn, 0, x, 1, x,
+                        StridedOut{1});
     } else {
       const double d2 = dnum_d2_theta(g, ir);
       if constexpr (M > 0)
         line_solve_c<2, M>(x, StridedIn{1}, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, O + lane * SO,
                            StridedOut{1});
       else
-        line_solve<2>(x, 1, m, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, O + lane * SO, 1);
+        line_solve_g<2>((const double *)x, StridedIn{1}, m, dtype, I.bdry, lo, hi, G, g.tstride, d2, dn * dn, 0, x, 1,
+                        x, StridedOut{1});
     }
   }
-  __syncwarp();
+  if (M > 0) __syncwarp();
+  else __syncthreads();
   double *dst = I.out + (size_t)row0 * nth + t0;
   if constexpr (M == 32) {
 #pragma unroll 8
     for (int l = 0; l < nrow; l++) dst[(size_t)l * nth + lane] = O[l * SO + lane];
   } else {
-    for (int k = lane; k < nrow * m; k += 32) {
-      const int l = k / m, c = k - l * m;
-      dst[(size_t)l * nth + c] = O[l * SO + c];
+    const double *const o = M > 0 ? O : X + 4;
+    const int so = M > 0 ? SO : SI;
+    const unsigned inv = inv_of(m);
+    for (int k = M > 0 ? lane : threadIdx.x; k < nrow * m; k += M > 0 ? 32 : blockDim.x) {
+      const int l = div_by(k, inv), c = k - l * m;
+      dst[(size_t)l * nth + c] = o[l * so + c];
     }
   }
 }
