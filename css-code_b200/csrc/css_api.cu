@@ -407,6 +407,12 @@ static int setup_kernels() {
   CSS_LINE_ATTR(k_adj_s<0, 2, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 1, 0>);
   CSS_LINE_ATTR(k_adj_s<2, 2, 0>);
+  CSS_LINE_ATTR(k_adj_w<0, 1>);
+  CSS_LINE_ATTR(k_adj_w<0, 2>);
+  CSS_LINE_ATTR(k_adj_w<1, 1>);
+  CSS_LINE_ATTR(k_adj_w<1, 2>);
+  CSS_LINE_ATTR(k_adj_w<2, 1>);
+  CSS_LINE_ATTR(k_adj_w<2, 2>);
   CSS_LINE_ATTR(k_adj_t<1, 0>);
   CSS_LINE_ATTR(k_adj_t<2, 0>);
 #undef CSS_LINE_ATTR
@@ -1883,8 +1889,34 @@ static int adjoint_tables(css_ctx *c, int dir, int order, int bdry) {
   return CSS_OK;
 }
 
+// Blocks of a line a CTA takes side by side (k_adj_w), or 0: whole lines walked
+// (k_adj_s, k_adj_t).  Where the lines give an SM few warps, the walk is a
+// chain of blocks on an idle chip.  Run-time block lengths, groups against the
+// walk: 25 against 133 us on 8192 lines of 32 blocks of 10 points, 82 against
+// 162 on 32768 of 16 of 20, 147 against 136 on 65536 of 6 of 48.  16 and 32
+// points, which the walk keeps in registers: along theta 27 against 41 us on
+// 8192 lines of 10 of 32, 82 against 72 on 24576; along r 23 against 25 on
+// 4096 and 49 against 29 on 16384.
+static int adj_warps(const css_ctx *c, int dir, int nl) {
+  const CssDir &D = c->g.d[dir];
+  if (nl / 32 >= c->nsm * (c->mt[dir] ? (dir == 1 ? 4 : 1) : 8)) return 0;
+  int w = std::min(D.nb, 8);
+  while (w > 1 && adj_w_smem(dir, D.maxm, w) * 8 > 200 * 1024) w--;
+  return w;
+}
+template <int DIR, int ORDER>
+static bool launch_adj_w(css_ctx *c, const double *E, const double *gin, double *gout, int bdry, cudaStream_t st) {
+  const CssGeo &g = c->g;
+  const int nl = DIR == 0 ? g.nth * g.nphi : (DIR == 1 ? g.nphi * g.nr : g.nth * g.nr);
+  const int w = adj_warps(c, DIR, nl);
+  if (!w) return false;
+  k_adj_w<DIR, ORDER><<<(unsigned)((nl + 31) / 32), dim3(32, w), (size_t)adj_w_smem(DIR, g.d[DIR].maxm, w) * 8, st>>>(
+      g, E, gin, gout, bdry);
+  return true;
+}
 template <int DIR, int ORDER>
 static void launch_adj_s(css_ctx *c, const double *E, const double *gin, double *gout, int bdry, cudaStream_t st) {
+  if (launch_adj_w<DIR, ORDER>(c, E, gin, gout, bdry, st)) return;
   const CssGeo &g = c->g;
   const int nl = DIR == 0 ? g.nth * g.nphi : g.nth * g.nr, m = g.d[DIR].maxm, mt = c->mt[DIR];
   const int nt = mt ? DV_NT : line_threads(m);
@@ -1895,6 +1927,7 @@ static void launch_adj_s(css_ctx *c, const double *E, const double *gin, double 
 }
 template <int ORDER>
 static void launch_adj_t(css_ctx *c, const double *E, const double *gin, double *gout, int bdry, cudaStream_t st) {
+  if (launch_adj_w<1, ORDER>(c, E, gin, gout, bdry, st)) return;
   const CssGeo &g = c->g;
   const int m = g.d[1].maxm, mt = c->mt[1];
   const size_t smem = 2 * (size_t)32 * adj_theta_stride(m) * 8;

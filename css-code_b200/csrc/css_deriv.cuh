@@ -316,31 +316,44 @@ __host__ __device__ constexpr int adj_theta_stride(int m) { return (m + 4) | 1; 
 template <int ORDER, int M>
 __device__ __forceinline__ void adj_block(double *t, int ts, int m_, const double *__restrict__ G, int gs,
                                           const double *__restrict__ E, double scale, double lo[4], double hi[4]) {
+  // run-time lengths: four rows' points and coefficients in hand before the chain
   constexpr int CH = M > 0 ? M : 4;
   const int m = M > 0 ? M : m_;
   const double *g1 = G, *g2 = G + gs, *g3 = G + 2 * gs;
   double v = 0.0;
   for (int j0 = 1; j0 <= m; j0 += CH) {  // U^-T, ascending
-    double q[CH];
+    double q[CH], c[4];
 #pragma unroll
     for (int k = 0; k < CH; k++) q[k] = j0 + k <= m ? t[(j0 + k - 1) * ts] : 0.0;
+    if constexpr (M == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) c[k] = __ldg(g1 + min(j0 + k, m));
+    }
 #pragma unroll
     for (int k = 0; k < CH; k++)
       if (j0 + k <= m) {
-        v = j0 + k > 1 ? q[k] + __ldg(g1 + j0 + k) * v : q[k];
+        v = j0 + k > 1 ? q[k] + (M > 0 ? __ldg(g1 + j0 + k) : c[k & 3]) * v : q[k];
         t[(j0 + k - 1) * ts] = v;
       }
   }
   v = 0.0;
   for (int j0 = m; j0 >= 1; j0 -= CH) {  // L^-T, descending
-    double q[CH];
+    double q[CH], c[4], d[4];
 #pragma unroll
     for (int k = 0; k < CH; k++) q[k] = j0 - k >= 1 ? t[(j0 - k - 1) * ts] : 0.0;
+    if constexpr (M == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int j = max(j0 - k, 1);
+        c[k] = __ldg(g3 + j + 1);
+        d[k] = __ldg(g2 + j);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < CH; k++)
       if (j0 - k >= 1) {
-        v = j0 - k < m ? q[k] + __ldg(g3 + j0 - k + 1) * v : q[k];
-        t[(j0 - k - 1) * ts] = (scale * __ldg(g2 + j0 - k)) * v;
+        v = j0 - k < m ? q[k] + (M > 0 ? __ldg(g3 + j0 - k + 1) : c[k & 3]) * v : q[k];
+        t[(j0 - k - 1) * ts] = (scale * (M > 0 ? __ldg(g2 + j0 - k) : d[k & 3])) * v;
       }
   }
   const double y1 = t[0], y2 = t[ts], ym1 = t[(m - 2) * ts], ym = t[(m - 1) * ts];
@@ -487,6 +500,116 @@ __global__ void __launch_bounds__(64) k_adj_t(CssGeo g, const double *__restrict
       for (int k = 0; k < 4; k++) t[k - 4] = t[m - 4 + k];
     }
     __syncwarp();
+  }
+}
+
+// Adjoint on few lines: W warps a CTA take W blocks in a row of the same 32
+// lines, so that the sweeps of a line's blocks run side by side where the
+// lines alone leave the chip idle (adj_warps has the line and both sides).  What a block adds to its neighbours passes
+// through shared memory (two buffers in turn, one barrier a group of blocks);
+// the last four points of a group wait for the next group's first block.
+// Block lengths at run time; the same sums in the same order as above.
+// tile: 32 lines of a block, theta rows at an odd stride
+__host__ __device__ constexpr int adj_w_tile(int dir, int m) { return 32 * (dir == 1 ? m | 1 : m); }
+__host__ __device__ constexpr int adj_w_smem(int dir, int m, int w) {  // doubles
+  return w * (adj_w_tile(dir, m) + 2 * 8 * 32) + 2 * 8 * 32 + 8 * 32;
+}
+template <int DIR, int ORDER>
+__global__ void __launch_bounds__(256) k_adj_w(CssGeo g, const double *__restrict__ E, const double *__restrict__ gin,
+                                               double *__restrict__ gout, int bdry) {
+  extern __shared__ double sm[];
+  const CssDir &D = g.d[DIR];
+  const int W = blockDim.y, wy = threadIdx.y, lane = threadIdx.x, nb = D.nb;
+  const int nlines = DIR == 0 ? g.nth * g.nphi : (DIR == 1 ? g.nphi * g.nr : g.nth * g.nr);
+  const int line0 = blockIdx.x * 32, line = line0 + lane, nrow = min(32, nlines - line0);
+  const bool live = lane < nrow;
+  const size_t s = DIR == 0 ? (size_t)g.nth * g.nphi : (DIR == 1 ? 1 : g.nth);
+  const size_t base = DIR == 0 ? line : (DIR == 1 ? (size_t)line * g.nth
+                                                  : line % g.nth + (size_t)(line / g.nth) * g.nth * g.nphi);
+  const int SR = DIR == 1 ? D.maxm | 1 : 1, ts = DIR == 1 ? 1 : 32;
+  double *const T = sm + (size_t)wy * adj_w_tile(DIR, D.maxm), *const t = T + lane * SR;
+  double *const ex = sm + (size_t)W * adj_w_tile(DIR, D.maxm);  // [2][W][8][32]: lo, hi of the blocks of a group
+  double *const carry = ex + 2 * W * 8 * 32;                    // [2][8][32]: a group's waiting points, its last hi
+  double *const wrap = carry + 2 * 8 * 32;                      // [8][32]: phi's first four points, first lo
+  double lo[4], hi[4];
+  int last = 0;  // the last point of this warp's last block
+  for (int c0 = 0, par = 0; c0 < nb; c0 += W, par ^= 1) {
+    const int b = c0 + wy, m = b < nb ? D.size[b] : 0, a0 = b < nb ? D.start[b] : 0;
+    double *const e = ex + (size_t)par * W * 8 * 32 + lane;
+    if (b < nb) {
+      if (DIR == 1) {
+        const double *src = gin + (size_t)line0 * g.nth + a0;
+        const unsigned inv = inv_of(m);
+        for (int k = lane; k < nrow * m; k += 32) {
+          const int l = div_by(k, inv), c = k - l * m;
+          cp_async8(T + l * SR + c, src + (size_t)l * g.nth + c);
+        }
+      } else if (live) {
+        const double *src = gin + base + (size_t)a0 * s;
+        for (int k = 0; k < m; k++) cp_async8(t + k * 32, src + (size_t)k * s);
+      }
+      cp_async_wait();
+      __syncwarp();
+      if (live) {
+        const double dn = D.dnum[b];
+        adj_block<ORDER, 0>(t, ts, m, tabp(g, DIR, b, ORDER, bdry), g.tstride, E + (size_t)b * ADJ_TAB,
+                            ORDER == 1 ? dn : dn * dn, lo, hi);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          e[(wy * 8 + k) * 32] = lo[k];
+          e[(wy * 8 + 4 + k) * 32] = hi[k];
+        }
+      }
+      last = m - 1;
+    }
+    __syncthreads();
+    if (b >= nb) continue;
+    const double *const cin = carry + (par ^ 1) * 8 * 32 + lane;
+    double *const cout = carry + par * 8 * 32 + lane, *const wr = wrap + lane;
+    const bool next = b + 1 < nb, held = next && wy + 1 == W;
+    if (live) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (DIR == 2 && b == 0) {  // waits for the last block
+          wr[k * 32] = t[k * ts];
+          wr[(4 + k) * 32] = lo[k];
+        } else {
+          t[k * ts] += wy > 0 ? e[((wy - 1) * 8 + 4 + k) * 32] : (c0 > 0 ? cin[(4 + k) * 32] : 0.0);
+        }
+        if (wy == 0 && c0 > 0) gout[base + (size_t)(a0 - 4 + k) * s] = cin[k * 32] + lo[k];
+        if (held) {
+          cout[k * 32] = t[(m - 4 + k) * ts];
+          cout[(4 + k) * 32] = hi[k];
+        } else if (next) {
+          t[(m - 4 + k) * ts] += e[((wy + 1) * 8 + k) * 32];
+        }
+      }
+    }
+    const int k0 = DIR == 2 && b == 0 ? 4 : 0, k1 = held || (DIR == 2 && !next) ? m - 4 : m;
+    if (DIR == 1) {
+      __syncwarp();
+      double *dst = gout + (size_t)line0 * g.nth + a0;
+      const unsigned inv = inv_of(k1);
+      for (int k = lane; k < nrow * k1; k += 32) {
+        const int l = div_by(k, inv), c = k - l * k1;
+        dst[(size_t)l * g.nth + c] = T[l * SR + c];
+      }
+      __syncwarp();
+    } else if (live) {
+#pragma unroll 8
+      for (int k = k0; k < k1; k++) gout[base + (size_t)(a0 + k) * s] = t[k * 32];
+    }
+  }
+  if (DIR == 2) {
+    __syncthreads();
+    if ((nb - 1) % W == wy && live) {
+      const double *const wr = wrap + lane;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        gout[base + (size_t)(g.nphi - 4 + k) * s] = t[(last - 3 + k) * 32] + wr[(4 + k) * 32];
+        gout[base + (size_t)k * s] = wr[k * 32] + hi[k];
+      }
+    }
   }
 }
 

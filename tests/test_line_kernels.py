@@ -1,8 +1,10 @@
 """The derivative and adjoint line kernels at the block lengths where they
 differ: 16 and 32 points (a line in registers), other lengths (run-time
 sweeps in shared memory), lengths that lower the threads of a CTA (above 48
-and 96 points) and the warps of a theta tile (200 points), and line counts
-that leave the last warp partly empty.  Forward against the oracle at the
+and 96 points) and the blocks a CTA takes side by side (200 points), line
+counts that leave the last warp partly empty, and the adjoint on few lines
+(groups of blocks, with a group left over) and on many (a walk of each
+line).  Forward against the oracle at the
 derivative bar; adjoint by <D x, y> = <x, D^T y> at 1e-13 of the sum of the
 products' magnitudes (rounding of sums of 1e5 terms)."""
 import numpy as np
@@ -40,7 +42,15 @@ def test_derivatives_at_block_length(dims, decomp, gpu_available):
     sim.close()
 
 
-@pytest.mark.parametrize("dims,decomp", SHAPES)
+# adjoint alone: lines of 9 to 18 blocks (groups of 8 and a rest), and 40000 or
+# more lines along r, theta and phi in turn, of 16 and 32 points and others
+ADJOINT = SHAPES + [((90, 36, 40), (9, 2, 4)), ((36, 90, 40), (2, 9, 4)), ((36, 40, 180), (2, 4, 18)),
+                    ((32, 192, 224), (2, 6, 7)), ((224, 32, 192), (7, 2, 6)), ((192, 224, 48), (6, 7, 3)),
+                    ((64, 192, 224), (2, 6, 7)), ((224, 64, 192), (7, 2, 6)), ((192, 224, 96), (6, 7, 3)),
+                    ((20, 200, 200), (2, 4, 5)), ((200, 24, 200), (4, 2, 5)), ((200, 200, 30), (4, 4, 3))]
+
+
+@pytest.mark.parametrize("dims,decomp", ADJOINT)
 def test_adjoint_at_block_length(dims, decomp, gpu_available):
     import torch
     from css_b200 import torch_ops  # noqa: F401
