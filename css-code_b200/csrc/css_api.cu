@@ -2735,14 +2735,20 @@ extern "C" int css_closure_scales(int nct, int ncp, int ncr, const double *field
 
 extern "C" int css_closure_features(int nct, int ncp, int ncr, const double *fields, const float *scale, void *x) {
   if (!fields || !scale || !x || nct < 1 || ncp < 1 || ncr < 1) { set_err("css_closure_features: bad argument"); return CSS_ERR_ARG; }
-  // segments of phi: long ones recompute fewer columns at their ends (two a
-  // segment), but every SM should hold its four CTAs
-  const int ntc = (nct + CF_T - 1) / CF_T;
-  int seg = 32;
-  while (seg > 4 && (long long)ntc * ncr * ((ncp + seg - 1) / seg) < 4 * 148) seg /= 2;
-  const dim3 grid(ntc, (ncp + seg - 1) / seg, ncr);
-  k_closure_features<<<grid, CF_NT>>>(fields, nct, ncp, ncr, scale, seg,
-                                         (uintptr_t)x % 16 == 0, (__nv_bfloat16 *)x);
+  if (nct <= CF_ROWS) {
+    k_closure_feature_rows<<<148 * 8, 128>>>(fields, nct, ncp, ncr, scale, (__nv_bfloat16 *)x);
+  } else {
+    // segments of phi: long ones recompute fewer columns at their ends (two a
+    // segment), but every SM should hold its four CTAs
+    const int ntc = (nct + CF_T - 1) / CF_T;
+    int seg = 32;
+    while (seg > 4 && (long long)ntc * ncr * ((ncp + seg - 1) / seg) < 4 * 148) seg /= 2;
+    for (int r0 = 0; r0 < ncr; r0 += 65535) {
+      const dim3 grid(ntc, (ncp + seg - 1) / seg, std::min(ncr - r0, 65535));
+      k_closure_features<<<grid, CF_NT>>>(fields, nct, ncp, ncr, r0, scale, seg, (uintptr_t)x % 16 == 0,
+                                          (__nv_bfloat16 *)x);
+    }
+  }
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaDeviceSynchronize());
   return CSS_OK;

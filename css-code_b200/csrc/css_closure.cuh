@@ -101,12 +101,13 @@ __device__ __forceinline__ void cl_quantities(const double *__restrict__ F, int 
 constexpr int CF_T = 64, CF_NT = 288;            // 16 rows of 18 vectors a sweep; 3 (CF_T + 2) column cells
 constexpr int CF_COL = 3 * CL_NQ * (CF_T + 2);   // one phi column: [r][q][theta]
 static_assert(3 * (CF_T + 2) <= CF_NT, "a thread computes at most one cell of a column");
+// A grid has at most 65535 radii (its z): ir0 is the first of this launch.
 __global__ void __launch_bounds__(CF_NT) k_closure_features(const double *__restrict__ F, int nct, int ncp, int ncr,
-                                                            const float *__restrict__ scale, int seg, int vec,
+                                                            int ir0, const float *__restrict__ scale, int seg, int vec,
                                                             __nv_bfloat16 *__restrict__ X) {
   // four columns, then zeros for the pad
   __shared__ unsigned short Q[4 * CF_COL + CF_T + 2];
-  const int t0 = blockIdx.x * CF_T, ir = blockIdx.z, p0 = blockIdx.y * seg, p1 = min(p0 + seg, ncp);
+  const int t0 = blockIdx.x * CF_T, ir = ir0 + blockIdx.z, p0 = blockIdx.y * seg, p1 = min(p0 + seg, ncp);
   const int nt = min(CF_T, nct - t0), ch = threadIdx.x % 18, row0 = threadIdx.x / 18;
   const size_t nc = (size_t)nct * ncp * ncr;
   const double sc[CL_NQ] = {(double)scale[0], (double)scale[1], (double)scale[2], (double)scale[3], (double)scale[4]};
@@ -180,6 +181,30 @@ __global__ void __launch_bounds__(CF_NT) k_closure_features(const double *__rest
     }
     column((s + 3) & 3);
     __syncthreads();
+  }
+}
+
+// The same, a thread a row: grids of one or two theta, whose columns of 3 to
+// 12 cells leave most of a CTA above idle (90000 rows: 150 and 255 us here,
+// 378 there; from three theta on, the columns are faster).
+constexpr int CF_ROWS = 2;
+__global__ void k_closure_feature_rows(const double *__restrict__ F, int nct, int ncp, int ncr,
+                                       const float *__restrict__ scale, __nv_bfloat16 *__restrict__ X) {
+  const size_t nc = (size_t)nct * ncp * ncr;
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
+    const int it = (int)(c % nct), ip = (int)((c / nct) % ncp), ir = (int)(c / ((size_t)nct * ncp));
+    __nv_bfloat16 *row = X + c * CL_XPAD;
+    int col = 0;
+    for (int dr = -1; dr <= 1; dr++)
+      for (int dt = -1; dt <= 1; dt++)
+        for (int dp = -1; dp <= 1; dp++) {
+          double q[CL_NQ];
+          cl_quantities(F, nct, ncp, ncr, min(max(it + dt, 0), nct - 1), (ip + dp + ncp) % ncp,
+                        min(max(ir + dr, 0), ncr - 1), q);
+#pragma unroll
+          for (int k = 0; k < CL_NQ; k++) row[col++] = __float2bfloat16_rn((float)(q[k] / (double)scale[k]));
+        }
+    for (; col < CL_XPAD; col++) row[col] = __float2bfloat16_rn(0.0f);
   }
 }
 

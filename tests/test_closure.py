@@ -449,3 +449,19 @@ def test_gradients_at_row_counts(n, gpu_available):
         gw, gb = net.grads(l)
         assert np.linalg.norm(gw - grads[l][0]) <= 2e-2 * np.linalg.norm(grads[l][0]), l
         assert np.linalg.norm(gb - grads[l][1]) <= 2e-2 * np.linalg.norm(grads[l][1]), l
+
+
+@pytest.mark.parametrize("dims", [(1, 9, 2), (2, 4, 4), (3, 4, 4), (1, 1, 65538), (3, 1, 65538)])
+def test_features_of_narrow_and_tall_grids(dims, gpu_available):
+    """One and two theta (a thread a row) and three, and more radii than a
+    launch's grid holds, bit for bit against numpy."""
+    import torch
+    from css_b200 import _lib
+    nct, ncp, ncr = dims
+    F = np.random.default_rng(ncr).standard_normal((7, ncr, ncp, nct))
+    qs = np.array([1.0, 2.0, 0.5, 3.0, 0.7], np.float32)
+    fd, qd = torch.from_numpy(F.reshape(-1)).cuda(), torch.from_numpy(qs).cuda()
+    x = torch.empty(nct * ncp * ncr * 144, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().css_closure_features(nct, ncp, ncr, fd.data_ptr(), qd.data_ptr(), x.data_ptr()))
+    assert np.array_equal(x.float().cpu().numpy().reshape(-1, 144), numpy_features(F, qs))
