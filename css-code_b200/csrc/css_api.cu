@@ -1874,12 +1874,10 @@ static int adjoint_tables(css_ctx *c, int dir, int order, int bdry) {
   }
   // on the device before any stream's kernel can read it: a copy from pageable
   // memory may return once the data is staged, and nothing orders the caller's
-  // stream behind it, so the host waits for the stream it went up on
-  cudaStream_t up = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking);
-  if (!e) e = cudaMemcpyAsync(dE, E.data(), E.size() * 8, cudaMemcpyHostToDevice, up);
-  if (!e) e = cudaStreamSynchronize(up);
-  if (up) cudaStreamDestroy(up);
+  // stream behind it, so the host waits for the stream it went up on (the run's
+  // own, which no caller can be capturing)
+  cudaError_t e = cudaMemcpyAsync(dE, E.data(), E.size() * 8, cudaMemcpyHostToDevice, c->own_stream);
+  if (!e) e = cudaStreamSynchronize(c->own_stream);
   if (e) {
     cudaFree(dE);
     set_err("css_deriv_adjoint: table copy: %s", cudaGetErrorString(e));
