@@ -297,6 +297,30 @@ def test_every_tile_variant_gives_the_same_bits(gpu_available, spec):
             sim.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("spec", [SMALL[1], SMALL[2]])
+def test_every_tile_variant_of_the_four_kernels(gpu_available, spec):
+    """The tile heights are the four-kernel stage's (and the curl's); the runs
+    above take the two-pass stage."""
+    from css_b200.context import Simulation
+    p, prof, v0, dt = E.build_member(spec, seed=13)
+    out = []
+    for tl, pers in [(16, False), (8, False), (16, True), (8, True), (0, False)]:
+        sim = Simulation(p, prof)
+        sim.set_fused(False)
+        sim.set_curl_pass(0)
+        sim.upload(v0)
+        if tl:
+            sim.set_tiles(tl, tl, tl, pers)
+        else:
+            sim.autotune(reps=2)
+        sim.step_rk4(dt, 2)
+        out.append(sim.download())
+        sim.close()
+    for o in out[1:]:
+        assert np.array_equal(o, out[0])
+
+
 MIX = SMALL + [  # a member on 32^3 blocks (the two-pass stage for FP64)
     {"nr": 64, "nth": 64, "nphi": 96, "ra": 1e5, "ro": 0.8, "magnetic": True, "pm": 2.5, "decomp": (2, 2, 3)},
 ]

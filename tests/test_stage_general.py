@@ -1,7 +1,8 @@
 """The general two-pass stage (plane pass over 16- and 32-point blocks, stage
 pass for any radial block) against the four-kernel stage of the same run,
-which tests/test_variants.py, test_inout.py, test_laplacian.py and
-test_mixed.py hold to the oracle.  Cases: both block lengths in either
+and that stage of every case against the oracle (the runs of
+tests/test_variants.py, test_laplacian.py and test_mixed.py have 16- and
+32-point blocks and step in two passes).  Cases: both block lengths in either
 direction, tiles left half empty by an odd number of 16-point blocks, radial
 blocks of 10 to 64 points, open faces, explicit viscosity, the TVD schemes and
 FP32 stage states.
@@ -82,6 +83,94 @@ def test_general_stage_equals_four_kernels(name, gpu_available):
     bar = 1e-7 if p.precision else 1e-12
     for i in range(two.shape[0]):
         assert np.abs(two[i] - four_[i]).max() <= bar * np.abs(four_[i]).max(), (name, i)
+
+
+# a prescribed bottom (ASH slices), with 16- and 32-point theta blocks
+ASH = {
+    "ash-16": dict(dims=(40, 48, 80), decomp=(2, 3, 5), bot_inout=1, bottom_specified=1, ufreq=2),
+    "ash-32": dict(dims=(64, 64, 96), decomp=(2, 2, 3), top_inout=1, bot_inout=1, bottom_specified=1, ufreq=2),
+}
+# the four kernels alone: 24-point theta and phi blocks, which have no two-pass
+# stage, with FP32 stage states
+FOUR = {
+    "mixed-24": dict(dims=(40, 48, 72), decomp=(2, 2, 3), precision=1),
+    "mixed-mhd-24": dict(dims=(40, 48, 72), decomp=(2, 2, 3), magnetic=True, precision=1),
+}
+
+
+def case(kw):
+    """Parameters, profiles, a stirred state and a time step."""
+    kw = dict(kw)
+    p, prof, v0, dt, _ = problem.build(kw.pop("dims"), decomp=kw.pop("decomp"), magnetic=kw.pop("magnetic", False))
+    for k, val in kw.items():
+        setattr(p, k, val)
+    v = v0.copy()
+    v[1:4] = 1e-3 * np.random.default_rng(8).standard_normal(v[1:4].shape)
+    if p.laplacian:
+        dt = 0.1 * dt
+    return p, prof, v, dt
+
+
+def open_faces(p, run, v, dt):
+    """The open faces' state of a run (device or oracle), from the seeds above."""
+    if not (p.top_inout or p.bot_inout):
+        return
+    rng = np.random.default_rng(9)
+    if isinstance(run, Simulation):
+        run.inout_init()
+    else:
+        run.inout_init(v)
+    run.set_clock(0, 2.01e5 if p.bottom_specified else 0.0, dt)
+    if p.do_entropy_rain:
+        sq = np.stack([rng.uniform(p.th1, p.th2, 12), rng.uniform(p.phi1, p.phi2, 12), rng.uniform(0.02, 0.08, 12),
+                       np.ones(12), rng.uniform(-2e-3, -1e-3, 12), rng.uniform(-2e-4, -1e-4, 12)], axis=1)
+        run.build_squalls(sq)
+    if p.bottom_specified:
+        run.set_ash_slices(1e-3 * rng.standard_normal((4, 4, p.nphi, p.nth)),
+                           np.array([1.9e5, 2.0e5, 2.1e5, 2.2e5]), 1.3)
+
+
+@pytest.mark.parametrize("name", list(ASH))
+def test_prescribed_bottom(name, gpu_available):
+    """The general stage under a prescribed bottom: the four kernels to a
+    rounding and the oracle to 1e-10, as the runs of tests/test_inout.py."""
+    p, prof, v, dt = case(ASH[name])
+    out = []
+    for four in (False, True):
+        sim = Simulation(p, prof)
+        assert sim.stage_form == 2
+        if four:
+            sim.set_fused(False)
+        sim.upload(v)
+        open_faces(p, sim, v, dt)
+        sim.step_rk4(dt, 3)
+        out.append(sim.download())
+        sim.close()
+    orc = O.Oracle(p, prof)
+    open_faces(p, orc, v, dt)
+    want = orc.step(v, dt, 3)
+    for i in range(5):
+        assert np.abs(out[0][i] - out[1][i]).max() <= 1e-12 * np.abs(out[1][i]).max(), (name, i)
+        assert np.abs(out[0][i] - want[i]).max() <= 1e-10 * np.abs(want[i]).max(), (name, i)
+
+
+@pytest.mark.parametrize("name", list(CASES) + list(ASH) + list(FOUR))
+def test_four_kernels_against_the_oracle(name, gpu_available):
+    """Two steps at the bars of the whole runs: FP64 1e-10 of each field's
+    largest magnitude (tests/test_gpu_parity.py), FP32 stage states 1e-6 for
+    rho and s and 1e-5 for the others (tests/test_mixed.py)."""
+    p, prof, v, dt = case({**CASES, **ASH, **FOUR}[name])
+    sim, orc = Simulation(p, prof), O.Oracle(p, prof)
+    sim.set_fused(False)
+    sim.upload(v)
+    open_faces(p, sim, v, dt)
+    open_faces(p, orc, v, dt)
+    sim.step_rk4(dt, 2)
+    got, want = sim.download(), orc.step(v, dt, 2)
+    sim.close()
+    for i in range(got.shape[0]):
+        bar = (1e-6 if i in (0, 4) else 1e-5) if p.precision else 1e-10
+        assert np.abs(got[i] - want[i]).max() <= bar * np.abs(want[i]).max(), (name, i)
 
 
 @pytest.mark.parametrize("dims,decomp,form,kw", [
