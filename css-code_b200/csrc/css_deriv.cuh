@@ -630,9 +630,6 @@ struct CurlLine {  // r A along r, from the block's first radius
     return (double)__ldg(p + (long long)k * (long long)ps) * __ldg(r + k);
   }
 };
-struct CurlIdx {
-  __device__ __forceinline__ int operator()(int j) const { return j - 1; }
-};
 template <typename TS>
 __global__ void __launch_bounds__(DV_NT) k_curl_rg(CssGeo g, const TS *__restrict__ a, double *__restrict__ out,
                                                    int apply_bc) {
@@ -644,10 +641,9 @@ __global__ void __launch_bounds__(DV_NT) k_curl_rg(CssGeo g, const TS *__restric
   const size_t n = (size_t)g.ncell, ps = (size_t)g.nth * g.nphi, base = (size_t)r0 * ps + line;
   double *t = sm + threadIdx.x;
   const int bdry = g.ibcr[z == 0 ? 10 : 11];
-  line_solve_g<1>(CurlLine<TS>{a + z * n + base, g.r_ind + r0, ps}, CurlIdx{}, m, dtype_of(D, b), bdry, 0.0, 0.0,
+  line_solve_g<1>(CurlLine<TS>{a + z * n + base, g.r_ind + r0, ps}, StridedIn{1}, m, dtype_of(D, b), bdry, 0.0, 0.0,
                   tabp(g, 0, b, 1, bdry), g.tstride, D.dnum[b], D.dnum[b], 0, t, ts, t, StridedOut{ts});
   const int it = line % g.nth;
-  const bool wall = apply_bc && (it == 0 || it == g.nth - 1);
   double *o = out + (z == 0 ? n : 0) + base;  // B_phi, B_theta
   for (int j0 = 0; j0 < m; j0 += 4) {
     double in[4];
@@ -660,12 +656,9 @@ __global__ void __launch_bounds__(DV_NT) k_curl_rg(CssGeo g, const TS *__restric
       double d = t[(j0 + k) * ts];
       if (g.non_uniform) d = d * g.dxdr[ir];
       double v = z == 0 ? in[k] + d * g.r_inv[ir] : in[k] - d * g.r_inv[ir];
-      if (apply_bc) {  // Compute_B's face zeroing (derivatives.f90:1830-1892)
-        if (wall && (z == 0) == !g.theta_perf_conductor) v = 0.0;
-        const bool lo = ir == 0, hi = ir == g.nr - 1;
-        if ((lo && g.bottom_radial_field) || (hi && g.top_radial_field)) v = 0.0;
-        const bool br0 = (wall && !g.theta_perf_conductor) || (lo && !g.bottom_radial_field && g.bottom_perfect_cond) ||
-                         (hi && !g.top_radial_field && g.top_perfect_cond);
+      if (apply_bc) {  // this half's component; the B_phi half zeroes B_r
+        double other = 0.0;
+        const bool br0 = z == 0 ? curl_faces(g, it, ir, other, v) : curl_faces(g, it, ir, v, other);
         if (z == 0 && br0) out[2 * n + base + (size_t)(j0 + k) * ps] = 0.0;
       }
       o[(size_t)(j0 + k) * ps] = v;

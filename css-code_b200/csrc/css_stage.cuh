@@ -40,9 +40,6 @@ struct SLine {
     return x;
   }
 };
-struct RIdx {
-  __device__ __forceinline__ int operator()(int j) const { return j - 1; }
-};
 
 // slab (state fields of storage size ts, then B_theta and B_phi), derivative
 // tiles, a face datum a line, an mbarrier
@@ -152,10 +149,10 @@ __global__ void __launch_bounds__(SG_NT, StageCfg<KIND>::CTAS) k_rstage_g(CssGeo
       if (bot_open) lo = 0.0;  // open faces: data of w, v, u, s zero (rhs_mpi.f90:594-596, :626-628)
       if (top_open) hi = 0.0;
       if (k == 4)
-        line_solve_g<2>(x, RIdx{}, m, dtype, bdry, lo, hi, tabp(g, 0, br, 2, bdry), g.tstride, dn, dn * dn, 0, o, 32, o,
+        line_solve_g<2>(x, StridedIn{1}, m, dtype, bdry, lo, hi, tabp(g, 0, br, 2, bdry), g.tstride, dn, dn * dn, 0, o, 32, o,
                         StridedOut{32});
       else
-        line_solve_g<1>(x, RIdx{}, m, dtype, bdry, lo, hi, tabp(g, 0, br, 1, bdry), g.tstride, dn, dn, 0, o, 32, o,
+        line_solve_g<1>(x, StridedIn{1}, m, dtype, bdry, lo, hi, tabp(g, 0, br, 1, bdry), g.tstride, dn, dn, 0, o, 32, o,
                         StridedOut{32});
     };
     if (!mag || k < 6) {
