@@ -419,8 +419,8 @@ def run_ours(args):
                 "avg_launch_ms": kms / cnt, "peak_source": peak_src,
                 "time_share": kms / sum(v[0] for v in stats.values()),
                 # the FP64 bound beside the HBM one: ncu's FP64-pipe activity
-                # of this kernel (profiles/traffic.json, captured on the
-                # 128x128x256 case of the same kind of run)
+                # of this kernel (profiles/traffic.json, captured on a
+                # smaller case of the same kind of run)
                 "fp64_pipe_frac": (fp64 / 100.0) if fp64 is not None else None}
     step_ach = step_alg_bytes(nv) * cells * args.steps / (ms / 1e3) / 1e9
     out = {

@@ -2737,7 +2737,7 @@ extern "C" int css_closure_features(int nct, int ncp, int ncr, const double *fie
     k_closure_feature_rows<<<148 * 8, 128>>>(fields, nct, ncp, ncr, scale, (__nv_bfloat16 *)x);
   } else {
     // segments of phi: long ones recompute fewer columns at their ends (two a
-    // segment), but every SM should hold its four CTAs
+    // segment), but there should be four CTAs an SM, two waves of the two it holds
     const int ntc = (nct + CF_T - 1) / CF_T;
     int seg = 32;
     while (seg > 4 && (long long)ntc * ncr * ((ncp + seg - 1) / seg) < 4 * 148) seg /= 2;

@@ -87,8 +87,11 @@ __device__ __forceinline__ void cl_quantities(const double *__restrict__ F, int 
 // at the ends, phi periodic; order (dr, dt, dp) with dp fastest) x the five
 // quantities divided by scale[q], then zeros.
 //
-// Bound by the rows it writes (288 bytes a cell; 604 MB, 92 us at 6550 GB/s,
-// on 64x128x256).  A CTA owns CF_T cells along theta of one radius and walks
+// Its floor is the rows it writes (288 bytes a cell; 604 MB, 92 us at 6550
+// GB/s, on 64x128x256); what it takes above that is instructions and the
+// barrier a column at two CTAs an SM (96 registers): issue slots 43 % busy,
+// stalls of 2.3 fixed-latency, 2.0 barrier and 1.2 shared-memory cycles an
+// issue, HBM at 34 %.  A CTA owns CF_T cells along theta of one radius and walks
 // a segment of phi.  The scaled quantities of the CF_T + 2 by 3 (theta, r)
 // neighbours of one phi sit in shared memory as BF16, four phi at a time, so
 // walking on by one phi computes one new column (3.1 cells a row) instead of

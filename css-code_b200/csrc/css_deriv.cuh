@@ -6,12 +6,14 @@
 // the 32 lines are consecutive theta, so a lane reads its line straight from
 // global memory (256 bytes a warp load) into registers, solves it and stores
 // it: nothing is staged.  Along theta a warp transposes its 32 lines through a
-// tile.  On large grids these passes are
-// bound by HBM (a field in, a field out: 268 MB, 41 us at 6550 GB/s on
-// 128x256x512).  Measured there, r / theta / phi: 63 / 88 / 45 us forward and
-// 53 / 76 / 63 us adjoint, against 297 / 235 / 253 us with 16-line tiles
-// staged in shared memory (16 of 128 threads solving) and 1410 us for an
-// adjoint that gathered a dense 32 x 40 block column per point.
+// tile.  The floor of a pass is HBM (a field in, a field out: 268 MB, 41 us at
+// 6550 GB/s on 128x256x512).  Measured there, r / theta / phi: 53 / 81 / 41 us
+// forward and 55 / 78 / 65 us adjoint, against 297 / 235 / 253 us with 16-line
+// tiles staged in shared memory (16 of 128 threads solving) and 1410 us for an
+// adjoint that gathered a dense 32 x 40 block column per point.  What keeps
+// the others off the floor is the latency of their loads at 7 to 14 warps an
+// SM (146 to 254 registers, or the theta tiles' shared memory): 3.8 to 6.4 of
+// the cycles between two issues.
 #pragma once
 #include "css_kernels.cuh"
 

@@ -395,9 +395,10 @@ int css_set_curl_pass(css_ctx *ctx, int mode);
  * css_ensemble_step advances every member by nsteps RK4 steps of its own
  * dt[i]: one step of all members is captured once into a CUDA graph, each
  * member's kernels on a stream of its own so small members share the GPU,
- * and the graph is replayed per step (it is captured again when a dt
- * changes).  The first call, and every call with a new dt, must not be made
- * during another stream capture.  Member contexts stay owned by the caller
+ * and the graph is replayed per step.  It is captured again when a dt
+ * changes, or what a member steps with (css_set_sld_speed2, css_set_fused,
+ * css_set_tiles, css_set_curl_pass, css_autotune); such a call and the first
+ * one must not be made during another stream capture.  Member contexts stay owned by the caller
  * and must outlive the ensemble; a member must not be stepped through
  * css_step_rk4 while an ensemble step is running.  Returns CSS_ERR_NAN
  * (naming the member) when a member's state went non-finite.  The ensemble
