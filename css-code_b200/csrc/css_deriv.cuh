@@ -507,11 +507,12 @@ __global__ void __launch_bounds__(64) k_adj_t(CssGeo g, const double *__restrict
 
 // Adjoint on few lines: W warps a CTA take W blocks in a row of the same 32
 // lines, so that the sweeps of a line's blocks run side by side where the
-// lines alone leave the chip idle (adj_warps has the line and both sides).  What a block adds to its neighbours passes
-// through shared memory (two buffers in turn, one barrier a group of blocks);
-// the last four points of a group wait for the next group's first block.
-// Block lengths at run time; the same sums in the same order as above.
-// tile: 32 lines of a block, theta rows at an odd stride
+// lines alone leave the chip idle (adj_warps has the line and both sides).
+// What a block adds to its neighbours passes through shared memory (two
+// buffers in turn, one barrier a group of blocks); the last four points of a
+// group wait for the next group's first block.  Block lengths at run time; the
+// same sums in the same order as above.  tile: 32 lines of a block, theta rows
+// at an odd stride.
 __host__ __device__ constexpr int adj_w_tile(int dir, int m) { return 32 * (dir == 1 ? m | 1 : m); }
 __host__ __device__ constexpr int adj_w_smem(int dir, int m, int w) {  // doubles
   return w * (adj_w_tile(dir, m) + 2 * 8 * 32) + 2 * 8 * 32 + 8 * 32;
